@@ -61,7 +61,7 @@ struct dampm_batch {
   int *count = nullptr, *start = nullptr, *perm = nullptr;
   int* skey = nullptr;  // the cell key of each sorted position
   int *tile_sum = nullptr, *clist = nullptr, *clist_n = nullptr, *cbig = nullptr;
-  unsigned char* tflag = nullptr;  // the scan tiles of a pass (k_b_tile_flags)
+  unsigned char* tflag = nullptr;  // the scan tiles of a pass (k_b_step_begin)
   int* cmid = nullptr;  // cells with more than 16 particles
   int* ustart = nullptr;
   long long* upex = nullptr;
@@ -237,7 +237,7 @@ int read_scalars(dampm_batch* b) {
 }
 
 // One pass of every live scenario: kPassLaunches kernel launches.
-constexpr int kPassLaunches = 14;
+constexpr int kPassLaunches = 9;
 int enqueue_pass(dampm_batch* b) {
   cudaStream_t st = b->stream;
   const int nscn = int(b->scns.size());
@@ -247,30 +247,28 @@ int enqueue_pass(dampm_batch* b) {
   const int* key = b->precision == DAMPM_FP32 ? b->p32[b->cur].key : b->p64[b->cur].key;
   const int* slot = b->precision == DAMPM_FP32 ? b->p32[b->cur].slot : b->p64[b->cur].slot;
   const int* idx = b->precision == DAMPM_FP32 ? b->p32[b->cur].idx : b->p64[b->cur].idx;
-  k_b_step_begin<<<1, 1024, 0, st>>>(b->scn, b->S, nscn, b->Sg);
   const int gp = grid_blocks(b->P_tot, 256);
-  // the counting sort of every scenario at once (G2P counted the keys), over
-  // the tiles the scenarios' key ranges meet
-  k_b_tile_flags<<<grid_blocks(ntiles, 256), 256, 0, st>>>(b->scn, b->S, nscn, b->Sg,
-                                                            b->tflag, ntiles);
+  // the step's begin, and the scan tiles of the sort: the counting sort of
+  // every scenario at once (G2P counted the keys), over the tiles the
+  // scenarios' key ranges meet
+  k_b_step_begin<<<1 + grid_blocks(ntiles, 256), 256, 0, st>>>(b->scn, b->S, nscn, b->Sg,
+                                                                b->tflag, ntiles);
+  const Gate gate = kGateBegun;
   k_scan_sums<<<ntiles, kScanThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->clist_n,
-                                               b->Sg, 0, b->tflag);
+                                               b->Sg, gate, 0, b->tflag);
   k_scan_apply<<<ntiles, kScanThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->start,
-                                                b->clist, b->clist_n, b->Sg, 0, b->tflag);
+                                                b->clist, b->clist_n, b->Sg, gate, 0,
+                                                b->tflag);
   k_scatter<<<gp, 256, 0, st>>>(key, slot, idx, b->start, b->perm, b->skey, b->sortbuf,
-                                b->Sg);
+                                b->Sg, gate);
   k_segment_order<<<148 * 4, 256, 0, st>>>(b->start, b->clist, b->clist_n, b->perm,
-                                            b->sortbuf, b->cmid, b->Sg);
-  k_segment_order_mid<<<148 * 8, 256, 0, st>>>(b->start, b->cmid, b->clist_n, b->perm,
-                                                b->sortbuf, b->cbig, b->Sg);
-  k_segment_order_big<<<148, 1024, sort_big_smem_bytes(), st>>>(b->start, b->cbig, b->clist_n, b->perm,
-                                            b->sortbuf, b->P_cap, b->Sg);
-  k_b_units_plan<<<b->strips_tot, kPlanThreads, 0, st>>>(
-      b->start, b->scn, b->S, b->strip_scn, b->Sg, b->units_per_cta * b->p2g_grid,
-      b->col_weight, b->ustart, b->upex, b->uplan, b->strip_n, b->ucount + 3);
-  k_b_units_flat<<<1, kPlanThreads, sizeof(int) * (b->strips_tot + 1), st>>>(
-      b->strip_n, b->strips_tot, b->strip_scn, b->scn, nscn, b->uplan, b->ulist, b->uorder,
-      b->ucount, b->scn_units, b->S, b->Sg);
+                                            b->sortbuf, b->cmid, b->cbig, b->Sg, gate);
+  k_segment_order_large<<<148, 1024, sort_big_smem_bytes(), st>>>(
+      b->start, b->cmid, b->cbig, b->clist_n, b->perm, b->sortbuf, b->P_cap, b->Sg, gate);
+  k_b_units<<<b->strips_tot, kPlanThreads, sizeof(int) * (b->strips_tot + 1), st>>>(
+      b->start, b->scn, b->S, nscn, b->strip_scn, b->Sg, b->units_per_cta * b->p2g_grid,
+      b->col_weight, b->ustart, b->upex, b->uplan, b->strip_n, b->ulist, b->uorder, b->ucount,
+      b->scn_units);
   if (b->precision == DAMPM_FP32)
     launch_b_p2g<float>(b->p2g_grid, st, b->p32[b->cur], b->perm, b->start,
                         static_cast<float2*>(b->vvL),
@@ -279,20 +277,26 @@ int enqueue_pass(dampm_batch* b) {
     launch_b_p2g<double>(b->p2g_grid, st, b->p64[b->cur], b->perm, b->start,
                          static_cast<double2*>(b->vvL),
                          b->led_part, b->scn, b->S, b->ulist, b->uorder, b->ucount, b->Sg);
-  k_b_ledger<<<nscn, 256, 0, st>>>(b->led_part, b->scn_units, b->scn, b->S, nscn,
-                                   b->Sg);
   if (b->precision == DAMPM_FP32)
     launch_b_g2p<float>(b->nblk, st, b->p32[b->cur], b->p32[nxt], b->perm, b->skey,
                         static_cast<const float2*>(b->vvL), b->Z[b->zcur], b->scn, b->S,
-                        b->gblk, b->Sg, b->count);
+                        b->gblk, b->Sg, b->count, b->led_part, b->scn_units, nscn);
   else
     launch_b_g2p<double>(b->nblk, st, b->p64[b->cur], b->p64[nxt], b->perm, b->skey,
                          static_cast<const double2*>(b->vvL), b->Z[b->zcur], b->scn, b->S,
-                         b->gblk, b->Sg, b->count);
-  k_b_step_end<<<1, 1024, 0, st>>>(b->scn, b->S, nscn);
+                         b->gblk, b->Sg, b->count, b->led_part, b->scn_units, nscn);
   b->cur = nxt;
   b->launches += kPassLaunches;
   cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return bfail(b, DAMPM_ERR_CUDA, cudaGetErrorString(e));
+  return DAMPM_OK;
+}
+
+// Ends the last pass of a call (a pass ends with the begin of the next one).
+int enqueue_end(dampm_batch* b) {
+  k_b_step_end<<<1, 1024, 0, b->stream>>>(b->scn, b->S, int(b->scns.size()));
+  b->launches += 1;
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return bfail(b, DAMPM_ERR_CUDA, cudaGetErrorString(e));
   return DAMPM_OK;
 }
@@ -441,8 +445,8 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   rc = rc ? rc : balloc(b, &b->led_part, us * 6);
   rc = rc ? rc : balloc(b, &b->strip_n, size_t(b->STRIP_cap));
   rc = rc ? rc : balloc(b, &b->strip_scn, size_t(b->STRIP_cap));
-  rc = rc ? rc : balloc(b, &b->ucount, 4);
-  if (rc == DAMPM_OK && cudaMemsetAsync(b->ucount, 0, sizeof(int) * 4, b->stream) != cudaSuccess)
+  rc = rc ? rc : balloc(b, &b->ucount, 8);
+  if (rc == DAMPM_OK && cudaMemsetAsync(b->ucount, 0, sizeof(int) * 8, b->stream) != cudaSuccess)
     rc = bfail(b, DAMPM_ERR_CUDA, "cudaMemsetAsync failed");
   rc = rc ? rc : balloc(b, &b->scn_units, size_t(scenario_cap));
   rc = rc ? rc : balloc(b, &b->gblk, size_t(b->B_cap));
@@ -671,6 +675,7 @@ int ensure_batch_graph(dampm_batch* b, int h) {
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   int rc = DAMPM_OK;
   for (int k = 0; k < kBatchGraphPasses && rc == DAMPM_OK; ++k) rc = enqueue_pass(b);
+  if (rc == DAMPM_OK) rc = enqueue_end(b);
   b->launches = l0;
   b->cur = cur0;  // nothing ran
   cudaGraph_t g = nullptr;
@@ -705,11 +710,16 @@ int dampm_batch_step(dampm_batch* b, int nsteps) {
     if (rc) return rc;
     for (; left >= kBatchGraphPasses; left -= kBatchGraphPasses) {
       BCK(cudaGraphLaunch(b->graph[h], b->stream));
-      b->launches += (long long)kPassLaunches * kBatchGraphPasses;
+      b->launches += (long long)kPassLaunches * kBatchGraphPasses + 1;
     }
   }
+  const bool plain = left > 0;
   for (; left > 0; --left) {
     int rc = enqueue_pass(b);
+    if (rc) return rc;
+  }
+  if (plain) {  // (a graph ends its last pass itself)
+    int rc = enqueue_end(b);
     if (rc) return rc;
   }
   // the graph the next call starts from, captured now rather than inside it

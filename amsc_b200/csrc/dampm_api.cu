@@ -253,41 +253,41 @@ int alloc_particles(dampm_ctx* ctx, long long cap) {
 
 // Enqueues the binning of the current particles (SORT), whose slots and
 // counts are in hand (from G2P, or from k_count after an upload, a state
-// upload or a merge/split).
-void enqueue_sort(dampm_ctx* ctx) {
+// upload or a merge/split).  begun: the step has begun (or the call is no
+// step: a standalone merge/split).
+void enqueue_sort(dampm_ctx* ctx, int begun) {
+  const Gate gate = make_gate(ctx->P, begun);
   const int gp = grid_for(ctx->cap, 256);
   k_scan_sums<<<ctx->ntiles, kScanThreads, 0, ctx->stream>>>(ctx->count, ctx->nc,
                                                              ctx->tile_sum, ctx->clist_n,
-                                                             ctx->S, 1, nullptr);
+                                                             ctx->S, gate, 1, nullptr);
   k_scan_apply<<<ctx->ntiles, kScanThreads, 0, ctx->stream>>>(
-      ctx->count, ctx->nc, ctx->tile_sum, ctx->start, ctx->clist, ctx->clist_n, ctx->S, 1,
+      ctx->count, ctx->nc, ctx->tile_sum, ctx->start, ctx->clist, ctx->clist_n, ctx->S, gate, 1,
       nullptr);
   k_scatter<<<gp, 256, 0, ctx->stream>>>(ctx->p.key, ctx->p.slot, ctx->p.idx, ctx->start,
-                                         ctx->perm, ctx->skey, ctx->sortbuf, ctx->S);
-  k_segment_order<<<148 * 4, 256, 0, ctx->stream>>>(ctx->start, ctx->clist,
-                                                   ctx->clist_n, ctx->perm, ctx->sortbuf,
-                                                   ctx->cmid, ctx->S);
-  k_segment_order_mid<<<148 * 8, 256, 0, ctx->stream>>>(ctx->start, ctx->cmid,
-                                                       ctx->clist_n, ctx->perm, ctx->sortbuf,
-                                                       ctx->cbig, ctx->S);
-  k_segment_order_big<<<148, 1024, sort_big_smem_bytes(), ctx->stream>>>(ctx->start, ctx->cbig, ctx->clist_n,
-                                                     ctx->perm, ctx->sortbuf, ctx->cap,
-                                                     ctx->S);
-  ctx->launches += 6;
+                                         ctx->perm, ctx->skey, ctx->sortbuf, ctx->S, gate);
+  k_segment_order<<<148 * 4, 256, 0, ctx->stream>>>(ctx->start, ctx->clist, ctx->clist_n,
+                                                   ctx->perm, ctx->sortbuf, ctx->cmid,
+                                                   ctx->cbig, ctx->S, gate);
+  k_segment_order_large<<<148, 1024, sort_big_smem_bytes(), ctx->stream>>>(
+      ctx->start, ctx->cmid, ctx->cbig, ctx->clist_n, ctx->perm, ctx->sortbuf, ctx->cap,
+      ctx->S, gate);
+  ctx->launches += 5;
 }
 
-// One pass of the loop body in two halves: step start, sort and P2G; then
-// G2P and step end (slab mode exchanges node columns between them).
+// One pass of the loop body in two halves: sort, units (which end the step
+// before and begin this one) and P2G; then G2P (slab mode exchanges node
+// columns between them).  enqueue_end ends the last pass of a call.
 int enqueue_front(dampm_ctx* ctx) {
   const long long it_next = ctx->it_host + 1;
   const bool ms_due = ctx->ms_enabled && ctx->params.MERGE_SPLIT_ON != 0 &&
                       ctx->ms.call_interval > 0 &&
                       (it_next % ctx->ms.call_interval) == 0;
   ev_mark(ctx, 3);
-  k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->S, ctx->G, ctx->P);
-  ctx->launches += 1;
   if (ms_due) {  // on the binning of the particles as they lie in storage
-    enqueue_sort(ctx);
+    k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->S, ctx->G, ctx->P);
+    ctx->launches += 1;
+    enqueue_sort(ctx, 1);
     ctx->launches += ms_enqueue(ctx->msb, ctx->p, ctx->q, ctx->start, ctx->perm, ctx->nc,
                                 ctx->G, ctx->P, ctx->Z, ctx->ms, ctx->S, ctx->cap,
                                 ctx->stream, /*use_step_dt=*/1, 0.0, ctx->ms_variant,
@@ -299,14 +299,12 @@ int enqueue_front(dampm_ctx* ctx) {
     ctx->launches += 2;
   }
   ev_mark(ctx, 0);
-  enqueue_sort(ctx);
+  enqueue_sort(ctx, ms_due);
   ev_mark(ctx, 1);
-  k_units_plan<<<ctx->strips, kPlanThreads, 0, ctx->stream>>>(
-      ctx->start, ctx->G, ctx->S, kUnitsPerCta * ctx->p2g_grid, ctx->useg, ctx->ustart,
-      ctx->upex, ctx->uplan, ctx->strip_n, ctx->ucount + 3);
-  k_units_flat<<<1, kPlanThreads, sizeof(int) * (ctx->strips + 1), ctx->stream>>>(
-      ctx->strip_n, ctx->strips, ctx->useg, ctx->uplan, ctx->ulist, ctx->uorder, ctx->ucount,
-      ctx->S);
+  k_units<<<ctx->strips, kPlanThreads, sizeof(int) * (ctx->strips + 1), ctx->stream>>>(
+      ctx->start, ctx->G, ctx->P, ctx->S, kUnitsPerCta * ctx->p2g_grid, ctx->useg,
+      ctx->ustart, ctx->upex, ctx->uplan, ctx->strip_n, ctx->ulist, ctx->uorder, ctx->ucount,
+      make_gate(ctx->P, ms_due));
   if (ctx->record) {
     Nodes& n = ctx->nodes;
     double* nf[] = {n.Mv,  n.mvx,  n.mvy,   n.avx,   n.avy,  n.vvx, n.vvy,
@@ -319,9 +317,6 @@ int enqueue_front(dampm_ctx* ctx) {
              ctx->led_part, ctx->G, ctx->P, ctx->S, ctx->record ? 1 : 0, ctx->ulist, ctx->uorder,
              ctx->ucount);
   ctx->launches += 2;
-  ev_mark(ctx, 3);
-  k_ledger_final<<<1, 1024, 0, ctx->stream>>>(ctx->led_part, ctx->ucount, ctx->S,
-                                               ctx->ledger_log);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(ctx, DAMPM_ERR_CUDA, cudaGetErrorString(e));
   return DAMPM_OK;
@@ -336,19 +331,26 @@ int enqueue_back(dampm_ctx* ctx) {
   ev_mark(ctx, 2);
   launch_g2p(grid_for(ctx->cap, kG2PThreads), ctx->stream, ctx->p, ctx->q, ctx->perm,
              ctx->skey, ctx->nodes, ctx->Z, ctx->G, ctx->P, ctx->S, ctx->count, ctx->leave,
-             ctx->record ? 1 : 0,
+             ctx->led_part, ctx->ucount, ctx->ledger_log, ctx->record ? 1 : 0,
              (grad_next || ctx->record) ? 1 : 0);
   if (ctx->record) {
     k_hv<<<grid_for(ctx->nn, 256), 256, 0, ctx->stream>>>(ctx->q, ctx->start,
                                                            ctx->nodes.HV, ctx->G, ctx->S);
     ctx->launches += 1;
   }
-  ev_mark(ctx, 3);
-  k_step_end<<<1, 1, 0, ctx->stream>>>(ctx->S);
-  ctx->launches += 4;
+  ctx->launches += 1;
   swap_moving(ctx->p, ctx->q);
   ctx->it_host = it_next;
   cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(ctx, DAMPM_ERR_CUDA, cudaGetErrorString(e));
+  return DAMPM_OK;
+}
+
+int enqueue_end(dampm_ctx* ctx) {
+  ev_mark(ctx, 3);
+  k_step_end<<<1, 1, 0, ctx->stream>>>(ctx->S);
+  ctx->launches += 1;
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(ctx, DAMPM_ERR_CUDA, cudaGetErrorString(e));
   return DAMPM_OK;
 }
@@ -448,6 +450,7 @@ int ensure_graph(dampm_ctx* ctx, int passes, int phase, dampm_ctx::GraphSlot** o
     return graphs_off(ctx);
   int rc = DAMPM_OK;
   for (int k = 0; k < passes && rc == DAMPM_OK; ++k) rc = enqueue_pass(ctx);
+  if (rc == DAMPM_OK) rc = enqueue_end(ctx);
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   const long long captured = ctx->launches - l0;
@@ -702,7 +705,7 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   rc = rc ? rc : dalloc(ctx, &ctx->ulist, size_t(ctx->n_led));
   rc = rc ? rc : dalloc(ctx, &ctx->uorder, size_t(ctx->n_led));
   rc = rc ? rc : dalloc(ctx, &ctx->strip_n, size_t(ctx->strips));
-  rc = rc ? rc : dalloc(ctx, &ctx->ucount, 4);
+  rc = rc ? rc : dalloc(ctx, &ctx->ucount, 8);
   rc = rc ? rc : dalloc(ctx, &ctx->ledger_log, size_t(kLedgerLog) * 3);
   rc = rc ? rc : dalloc(ctx, &ctx->S, 1);
   if (rc == DAMPM_OK) {
@@ -710,7 +713,7 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   }
   if (rc == DAMPM_OK) {
     cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream);
-    cudaMemsetAsync(ctx->ucount, 0, sizeof(int) * 4, ctx->stream);
+    cudaMemsetAsync(ctx->ucount, 0, sizeof(int) * 8, ctx->stream);
     cudaMemsetAsync(ctx->nodes.vvL, 0, sizeof(double2) * nn, ctx->stream);
     cudaMemsetAsync(ctx->S, 0, sizeof(Scalars), ctx->stream);
     int per_sm = setup_p2g(), nsm = 0, dev = 0;
@@ -852,6 +855,7 @@ int dampm_step(dampm_ctx* ctx, int nsteps) {
   ctx->evused = 0;
   int s = 0;
   int phase = 0;
+  bool plain = false;  // the last pass was launched plainly
   const int len = graph_eligible(ctx) ? graph_shape(ctx, &phase) : 0;
   if (len > 0) {
     bool aligned = true;
@@ -862,6 +866,7 @@ int dampm_step(dampm_ctx* ctx, int nsteps) {
       for (; s < nsteps && int(ctx->it_host % len) != phase; ++s) {
         int rc = enqueue_pass(ctx);
         if (rc) return rc;
+        plain = true;
       }
       aligned = int(ctx->it_host % len) == phase;
     }
@@ -875,6 +880,7 @@ int dampm_step(dampm_ctx* ctx, int nsteps) {
       if (rc) return rc;
       if (!g || s + len > nsteps) break;
       CK(cudaGraphLaunch(g->exec, ctx->stream));
+      plain = false;
       advance_buffers(ctx, len);
       ctx->it_host += len;
       ctx->launches += g->launches;
@@ -883,6 +889,11 @@ int dampm_step(dampm_ctx* ctx, int nsteps) {
   }
   for (; s < nsteps; ++s) {
     int rc = enqueue_pass(ctx);
+    if (rc) return rc;
+    plain = true;
+  }
+  if (plain) {  // (a graph ends its last step itself)
+    int rc = enqueue_end(ctx);
     if (rc) return rc;
   }
   // without merge/split, the graph the next call starts from (the buffers of
@@ -957,7 +968,7 @@ int dampm_merge_split(dampm_ctx* ctx, double dt, long long counts[4]) {
   CK(cudaMemcpyAsync(&S->active, &ctx->Sh->active, sizeof(int),
                      cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  enqueue_sort(ctx);
+  enqueue_sort(ctx, 1);
   ms_enqueue(ctx->msb, ctx->p, ctx->q, ctx->start, ctx->perm, ctx->nc, ctx->G, ctx->P,
              ctx->Z, ctx->ms, ctx->S, ctx->cap, ctx->stream, /*use_step_dt=*/0, dt,
              ctx->ms_variant, ctx->ms_stretch);
@@ -1213,7 +1224,10 @@ int dampm_slab_pass(dampm_ctx* ctx, int phase) {
   if (rc) return rc;
   ctx->launches = 0;
   if (phase == 0) return enqueue_front(ctx);
-  if (phase == 1) return enqueue_back(ctx);
+  if (phase == 1) {
+    rc = enqueue_back(ctx);
+    return rc ? rc : enqueue_end(ctx);
+  }
   return DAMPM_ERR_ARG;
 }
 

@@ -39,6 +39,7 @@ struct Scalars {
   double dt;
   int it;
   int active;   // this pass of the loop body executes
+  int pending;  // G2P has run, its step has not been ended yet
   int fresh;    // next P2G reads Ap/mom/Fb from the stored arrays
   int status;   // error bits (kStatus*)
   int np;       // current particle count
@@ -54,6 +55,20 @@ struct Scalars {
   double ledger[9];
   long long ms_counts[4];
 };
+
+// Whether a sort runs: with the step begun, when it is active; before it
+// begins, when the loop condition holds after the pass before it
+// (main/optim_par.cpp:281; a flagged run does no further passes).
+struct Gate {
+  int begun, fixed, NSTEPS;
+  double T;
+};
+constexpr Gate kGateBegun{1, 0, 0, 0.0};
+__device__ __forceinline__ bool gate_open(const Scalars* S, const Gate& g) {
+  if (g.begun) return S->active;
+  if (S->status != 0) return false;
+  return g.fixed ? S->it < g.NSTEPS : (S->pending ? S->t + S->dt : S->t) < g.T;
+}
 
 constexpr int kStatusCapacity = 1;
 constexpr int kStatusNonFinite = 2;

@@ -154,37 +154,33 @@ void launch_prep(int grid, int block, cudaStream_t st, ParticlesT<R> p, const do
 __global__ void k_count(const int* key, int* count, int* slot,
                         const Scalars* S);
 __global__ void k_count_n(const int* key, int* count, int* slot, int n);
-// tflag (may be null): scan only the flagged tiles (k_b_tile_flags)
+// tflag (may be null): scan only the flagged tiles (k_b_step_begin)
 __global__ void k_scan_sums(const int* count, int n, int* tile_sum, int* list_n,
-                            const Scalars* S, int ranged, const unsigned char* tflag);
+                            const Scalars* S, Gate gate, int ranged,
+                            const unsigned char* tflag);
 __global__ void k_scan_apply(int* count, int n, const int* tile_sum,
                              int* start, int* list, int* list_n,
-                             const Scalars* S, int ranged, const unsigned char* tflag);
+                             const Scalars* S, Gate gate, int ranged,
+                            const unsigned char* tflag);
 // pk: 2 x capacity entries; the scatter writes the first half, which the
 // per-cell ordering sorts (the crowded cells use both halves)
 __global__ void k_scatter(const int* key, const int* slot, const int* idx, const int* start,
-                          int* perm, int* skey, unsigned long long* pk, Scalars* S);
+                          int* perm, int* skey, unsigned long long* pk, Scalars* S, Gate gate);
 __global__ void k_segment_order(const int* start, const int* list, int* list_n,
                                 int* perm, const unsigned long long* pk, int* mid,
-                                const Scalars* S);
-__global__ void k_segment_order_mid(const int* start, const int* mid, int* list_n,
-                                    int* perm, const unsigned long long* pk, int* big,
-                                    const Scalars* S);
-__global__ void k_segment_order_big(const int* start, const int* big,
-                                    const int* list_n, int* perm, unsigned long long* pk,
-                                    long long cap, const Scalars* S);
-// dynamic shared memory of k_segment_order_big; setup_sort sets its limit
+                                int* big, const Scalars* S, Gate gate);
+__global__ void k_segment_order_large(const int* start, const int* mid, const int* big,
+                                      const int* list_n, int* perm, unsigned long long* pk,
+                                      long long cap, const Scalars* S, Gate gate);
+// dynamic shared memory of k_segment_order_large; setup_sort sets its limit
 // (0 on failure)
 size_t sort_big_smem_bytes();
 int setup_sort();
-__global__ void k_units_plan(const int* cstart, Geom G, const Scalars* S,
-                             int target_units, int seg, int* ustart,
-                             long long* upex, int4* plan, int* strip_n, int* heavy_n);
-// the flat unit list and uorder, the order P2G hands the units out in
-// (heavy units first)
-__global__ void k_units_flat(const int* strip_n, int strips, int seg,
-                             const int4* plan, int4* ulist, int* uorder, int* ucount,
-                             const Scalars* S);
+// the unit list and uorder, the order P2G hands the units out in (heavy units
+// first); ends the step before and begins this one unless it has begun
+__global__ void k_units(const int* cstart, Geom G, Phys P, Scalars* S, int target_units,
+                        int seg, int* ustart, long long* upex, int4* plan, int* strip_n,
+                        int4* ulist, int* uorder, int* ucount, Gate gate);
 // P2G of the single-scenario step (k_p2g specialised for recorded outputs);
 // setup_p2g sets its shared-memory attributes and returns the resident CTAs
 // per SM (0 on failure)
@@ -193,14 +189,13 @@ void launch_p2g(int grid, cudaStream_t st, Particles p, const int* perm, const i
                 const int4* ulist, const int* uorder, const int* ucount);
 int setup_p2g();
 constexpr int kLedgerLog = 1024;  // rows of the per-step ledger log
-__global__ void k_ledger_final(const double* led_part, const int* ucount,
-                               Scalars* S, double* log);
 // G2P of the single-scenario step (k_g2p_t specialised for the two flags):
-// reads `cur` through perm, writes `nxt` in this step's sorted order and
-// counts the next binning's keys
+// reads `cur` through perm, writes `nxt` in this step's sorted order, counts
+// the next binning's keys and sums the ledger; the step's end is left pending
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
-                int* count, int* leave, int record, int want_grad);
+                int* count, int* leave, const double* led_part, const int* ucount, double* log,
+                int record, int want_grad);
 
 // ---- batches of independent scenarios --------------------------------------
 // One scenario of a batch: its geometry, physics and place in the packed
@@ -216,18 +211,14 @@ struct Scn {
   int live;                // 0 once removed
 };
 
-__global__ void k_b_step_begin(const Scn* scn, Scalars* S, int nscn, Scalars* Sg);
-__global__ void k_b_step_end(const Scn* scn, Scalars* S, int nscn);
-__global__ void k_b_units_plan(const int* cstart, const Scn* scn, const Scalars* S,
-                               const int* strip_scn, const Scalars* Sg,
-                               int target_units, int col_weight, int* ustart,
-                               long long* upex, int4* plan, int* strip_n, int* heavy_n);
-__global__ void k_b_units_flat(const int* strip_n, int strips, const int* strip_scn,
-                               const Scn* scn, int nscn, const int4* plan,
-                               int4* ulist, int* uorder, int* ucount, int2* scn_units,
-                               Scalars* S, const Scalars* Sg);
-__global__ void k_b_tile_flags(const Scn* scn, const Scalars* S, int nscn, const Scalars* Sg,
+__global__ void k_b_units(const int* cstart, const Scn* scn, Scalars* S, int nscn,
+                          const int* strip_scn, const Scalars* Sg, int target_units,
+                          int col_weight, int* ustart, long long* upex, int4* plan,
+                          int* strip_n, int4* ulist, int* uorder, int* ucount,
+                          int2* scn_units);
+__global__ void k_b_step_begin(const Scn* scn, Scalars* S, int nscn, Scalars* Sg,
                                unsigned char* tflag, int ntiles);
+__global__ void k_b_step_end(const Scn* scn, Scalars* S, int nscn);
 template <class R>
 void launch_b_p2g(int grid, cudaStream_t st, ParticlesT<R> p, const int* perm,
                   const int* cstart, V2<R>* vvL, double* led_part, const Scn* scn,
@@ -237,13 +228,11 @@ void launch_b_p2g(int grid, cudaStream_t st, ParticlesT<R> p, const int* perm,
 // resident CTAs per SM (0 on failure)
 template <class R>
 int setup_b_p2g();
-__global__ void k_b_ledger(const double* led_part, const int2* scn_units,
-                           const Scn* scn, Scalars* S, int nscn,
-                           const Scalars* Sg);
 template <class R>
-void launch_b_g2p(int grid, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nxt,
+void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nxt,
                   const int* perm, const int* skey, const V2<R>* vvL, const double* Z,
-                  const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count);
+                  const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count,
+                  const double* led_part, const int2* scn_units, int nscn);
 template <class R>
 void launch_b_move(int grid, cudaStream_t st, ParticlesT<R> dst, ParticlesT<R> src,
                    const int4* mblk);

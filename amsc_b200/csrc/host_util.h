@@ -50,6 +50,12 @@ inline Phys make_phys(const dampm_params& d) {
   return P;
 }
 
+// The condition a pass's sort runs on (Gate): begun != 0 where the step has
+// begun before it.
+inline Gate make_gate(const Phys& P, int begun) {
+  return Gate{begun, P.fixed, P.NSTEPS, P.T};
+}
+
 // Host halves (a, b) of n pairs into a pair array: two strided copies.
 template <class T, class V>
 cudaError_t upload_pair(V* dst, const T* a, const T* b, long long n, cudaStream_t st) {

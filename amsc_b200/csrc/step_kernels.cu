@@ -1,14 +1,16 @@
 // step_kernels.cu -- the FP64 MPM time step on sm_100a.
 //
 // One pass of the loop body of main/optim_par.cpp:281-668 is
-//   step_begin  : dt (fixed or CFL from the previous G2P's max-reductions),
-//                 it++, loop condition -- one thread, no host sync
 //   SORT        : count -> scan -> scatter -> per-cell order  (a1)
+//   UNITS       : P2G's work list; its last block ends the step before (t += dt)
+//                 and begins this one -- dt (fixed or CFL from the previous
+//                 G2P's max-reductions), it++
 //   P2G+NODAL   : per-node sequential chains over the sorted particles of the
 //                 node's 4 cells, nodal momentum/velocity/BC  (a2-a7, a10, a14)
 //   G2P         : velocity, advection, gradients, height, Bingham stress,
-//                 next cell key, CFL max-reductions  (a8, a9, a11, a13)
-//   step_end    : t += dt
+//                 next cell key, CFL max-reductions  (a8, a9, a11, a13); one
+//                 block of its own sums the ledger
+// The loop state lives on the device: no host synchronisation in a pass.
 #include <cstdio>
 
 #include "dampm_device.cuh"
@@ -19,9 +21,22 @@ namespace dampm {
 // ---------------------------------------------------------------------------
 // loop control
 // ---------------------------------------------------------------------------
-// One scenario's pass start: the loop condition, dt, it++ (device side).
+// The end of the step that G2P left pending.
+__device__ __forceinline__ void step_end_one(Scalars* S) {
+  if (!S->pending) return;
+  S->pending = 0;
+  S->t += S->dt;
+  S->fresh = 0;
+  S->red_cur[0] = S->red_next[0];
+  S->red_cur[1] = S->red_next[1];
+  S->red_cur[2] = S->red_next[2];
+}
+
+// One scenario's pass start, after the end of the one before: the loop
+// condition, dt, it++ (device side).
 __device__ __forceinline__ void step_begin_one(Scalars* S, const Geom& G,
                                                const Phys& P) {
+  step_end_one(S);
   const bool cond = P.fixed ? (S->it < P.NSTEPS) : (S->t < P.T);
   if (!cond || S->status != 0) {
     S->active = 0;
@@ -51,27 +66,37 @@ __device__ __forceinline__ void step_begin_one(Scalars* S, const Geom& G,
   S->red_next[0] = S->red_next[1] = S->red_next[2] = 0ull;
 }
 
-__device__ __forceinline__ void step_end_one(Scalars* S) {
-  // slab mode: the neighbour's column copies were read by P2G only; G2P
-  // wrote the slab's own particles
-  S->np -= S->nghost;
-  S->nghost = 0;
-  if (!S->active) return;
-  S->t += S->dt;
-  S->fresh = 0;
-  S->red_cur[0] = S->red_next[0];
-  S->red_cur[1] = S->red_next[1];
-  S->red_cur[2] = S->red_next[2];
+// The last of n blocks to call it (counted in *arrived, which it resets): all
+// its threads get true.  What thread 0 of a block did before (its stores, its
+// atomics) is visible to the last block past L1.
+__device__ __forceinline__ bool last_block(int* arrived, int n) {
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(arrived, 1) == n - 1;
+    if (last) *arrived = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
 }
 
+// The pass start as a launch of its own: a merge/split at the cadence comes
+// between it and the sort.
 __global__ void k_step_begin(Scalars* S, Geom G, Phys P) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   step_begin_one(S, G, P);
 }
 
+// The step end as a launch of its own, after the last pass of a call: the
+// state is complete when the host reads it.
 __global__ void k_step_end(Scalars* S) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   step_end_one(S);
+  // slab mode: the neighbour's column copies were read by P2G only; G2P
+  // wrote the slab's own particles
+  S->np -= S->nghost;
+  S->nghost = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -347,9 +372,9 @@ __device__ __forceinline__ void scan_tiles_of(const Scalars* S, int n, int range
 
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_sums(const int* __restrict__ count, int n, int* __restrict__ tile_sum,
-                int* __restrict__ list_n, const Scalars* S, int ranged,
+                int* __restrict__ list_n, const Scalars* S, Gate gate, int ranged,
                 const unsigned char* __restrict__ tflag) {
-  if (!S->active) return;
+  if (!gate_open(S, gate)) return;
   if (list_n && blockIdx.x == 0 && threadIdx.x < 3) list_n[threadIdx.x] = 0;
   int t0, t1;
   scan_tiles_of(S, n, ranged, t0, t1);
@@ -368,14 +393,14 @@ __global__ void __launch_bounds__(kScanThreads)
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_apply(int* __restrict__ count, int n, const int* __restrict__ tile_sum,
                  int* __restrict__ start, int* __restrict__ list,
-                 int* __restrict__ list_n, const Scalars* S, int ranged,
+                 int* __restrict__ list_n, const Scalars* S, Gate gate, int ranged,
                  const unsigned char* __restrict__ tflag) {
-  if (!S->active) return;
+  if (!gate_open(S, gate)) return;
   int t0, t1;
   scan_tiles_of(S, n, ranged, t0, t1);
   const int t = blockIdx.x;
   if (t < t0 || t > t1) return;  // block-uniform
-  if (tflag && !tflag[t]) return;  // its starts stand (see k_b_tile_flags)
+  if (tflag && !tflag[t]) return;  // its starts stand (see k_b_step_begin)
   __shared__ int wsum[32];
   // particles in the range's tiles before this one
   int pre = 0;
@@ -438,8 +463,8 @@ __global__ void k_scatter(const int* __restrict__ key,
                           const int* __restrict__ slot, const int* __restrict__ idx,
                           const int* __restrict__ start, int* __restrict__ perm,
                           int* __restrict__ skey, unsigned long long* __restrict__ pk,
-                          Scalars* S) {
-  if (!S->active) return;
+                          Scalars* S, Gate gate) {
+  if (!gate_open(S, gate)) return;
   const int np = S->np;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np;
        i += gridDim.x * blockDim.x) {
@@ -462,15 +487,15 @@ __global__ void k_scatter(const int* __restrict__ key,
 // slots in arbitrary order).  A segment entry is the 64-bit value
 // idx << 32 | slot that the scatter wrote to pk at the same position, so
 // sorting those values orders by reference index (unique) and carries the
-// slot along; a cell whose entries are already in order is left as it is.  k_segment_order: each lane sorts a
-// cell of up to kThreadSort particles in registers (a bitonic network over
-// static indices) and hands larger cells on to `mid`.  k_segment_order_mid,
-// one warp per cell: a register bitonic sort across the lanes for up to 32
-// particles, a rank sort for up to 32 * kRankPer (each lane holds kRankPer
-// values and counts, over all the cell's values broadcast lane by lane,
-// those below each of its own; the values are unique, so the ranks are a
-// permutation of [0, m)); larger cells go on to `big` for
-// k_segment_order_big.
+// slot along; a cell whose entries are already in order is left as it is.
+// k_segment_order: each lane sorts a cell of up to kThreadSort particles in
+// registers (a bitonic network over static indices) and hands larger cells on
+// to `mid`, crowded ones (above 32 * kRankPer) to `big`.
+// k_segment_order_large, one warp per cell of `mid`: a register bitonic sort
+// across the lanes for up to 32 particles, else a rank sort (each lane holds
+// kRankPer values and counts, over all the cell's values broadcast lane by
+// lane, those below each of its own; the values are unique, so the ranks are
+// a permutation of [0, m)); then one block per cell of `big`.
 constexpr int kThreadSort = 16;
 constexpr int kRankPer = 8;
 constexpr int kBigRun = 8192;  // entries of a sorted run (two buffers: 128 KB of shared memory)
@@ -555,14 +580,12 @@ __device__ __forceinline__ void merge_level(const unsigned long long* src,
 }
 
 __device__ __forceinline__ void warp_sort_segment(int* __restrict__ perm, int b, int m,
-                                                  int c, int lane,
-                                                  const unsigned long long* __restrict__ pk,
-                                                  int* __restrict__ big,
-                                                  int* __restrict__ list_n) {
+                                                  int lane,
+                                                  const unsigned long long* __restrict__ pk) {
   if (m <= 32) {
     const unsigned long long v = warp_bitonic32((lane < m) ? pk[b + lane] : kNoEntry, lane);
     if (lane < m) perm[b + lane] = int(unsigned(v));
-  } else if (m <= 32 * kRankPer) {
+  } else {
     unsigned long long v[kRankPer];
     int rank[kRankPer];
 #pragma unroll
@@ -584,8 +607,6 @@ __device__ __forceinline__ void warp_sort_segment(int* __restrict__ perm, int b,
 #pragma unroll
     for (int t = 0; t < kRankPer; ++t)
       if (lane + 32 * t < m) perm[b + rank[t]] = int(unsigned(v[t]));
-  } else if (lane == 0) {
-    big[atomicAdd(&list_n[1], 1)] = c;
   }
 }
 
@@ -595,8 +616,9 @@ __global__ void __launch_bounds__(256, 4) k_segment_order(const int* __restrict_
                                 int* __restrict__ list_n,
                                 int* __restrict__ perm,
                                 const unsigned long long* __restrict__ pk,
-                                int* __restrict__ mid, const Scalars* S) {
-  if (!S->active) return;
+                                int* __restrict__ mid, int* __restrict__ big,
+                                const Scalars* S, Gate gate) {
+  if (!gate_open(S, gate)) return;
   const int lane = threadIdx.x & 31;
   const int nl = list_n[0];
   for (int w0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; w0 < nl;
@@ -614,33 +636,20 @@ __global__ void __launch_bounds__(256, 4) k_segment_order(const int* __restrict_
     // larger cells: one atomic per warp
     const unsigned larger = __ballot_sync(0xffffffffu, m > kThreadSort);
     if (larger) {
+      const bool crowded = m > 32 * kRankPer;
+      const unsigned most = __ballot_sync(0xffffffffu, crowded);
+      const unsigned some = larger & ~most;
       int base = 0;
-      if (lane == 0) base = atomicAdd(&list_n[2], __popc(larger));
+      if (lane == 0 && some) base = atomicAdd(&list_n[2], __popc(some));
       base = __shfl_sync(0xffffffffu, base, 0);
-      if (m > kThreadSort) mid[base + __popc(larger & ((1u << lane) - 1u))] = c;
+      if (m > kThreadSort && !crowded) mid[base + __popc(some & ((1u << lane) - 1u))] = c;
+      if (crowded) big[atomicAdd(&list_n[1], 1)] = c;
     }
   }
 }
 
-__global__ void __launch_bounds__(256, 4) k_segment_order_mid(const int* __restrict__ start,
-                                    const int* __restrict__ mid,
-                                    int* __restrict__ list_n,
-                                    int* __restrict__ perm,
-                                    const unsigned long long* __restrict__ pk,
-                                    int* __restrict__ big, const Scalars* S) {
-  if (!S->active) return;
-  const int lane = threadIdx.x & 31;
-  const int nm = list_n[2];
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nm;
-       w += (gridDim.x * blockDim.x) >> 5) {
-    const int c = mid[w];
-    const int b = start[c];
-    warp_sort_segment(perm, b, start[c + 1] - b, c, lane, pk, big, list_n);
-  }
-}
-
-// Crowded cells (more than 32 * kRankPer particles), one block of 1024
-// threads each: runs of up to kBigRun entries of tmp[b, b+m) (the pk the
+// The larger cells.  Those of the mid list: one warp each.  Crowded cells
+// (more than 32 * kRankPer particles), one block of 1024 threads each: runs of up to kBigRun entries of tmp[b, b+m) (the pk the
 // scatter wrote) are sorted in shared memory -- groups of 32 by a bitonic
 // network in each warp's registers, then merged level by level along the
 // merge path between two buffers -- and written back; longer cells then
@@ -649,12 +658,19 @@ __global__ void __launch_bounds__(256, 4) k_segment_order_mid(const int* __restr
 // starts by a binary search along the merge path, then merges the piece
 // sequentially.  The slots go back to perm.
 __global__ void __launch_bounds__(1024)
-    k_segment_order_big(const int* __restrict__ start, const int* __restrict__ big,
-                        const int* __restrict__ list_n, int* __restrict__ perm,
-                        unsigned long long* __restrict__ tmp, long long cap,
-                        const Scalars* S) {
-  if (!S->active) return;
+    k_segment_order_large(const int* __restrict__ start, const int* __restrict__ mid,
+                          const int* __restrict__ big, const int* __restrict__ list_n,
+                          int* __restrict__ perm, unsigned long long* __restrict__ tmp,
+                          long long cap, const Scalars* S, Gate gate) {
+  if (!gate_open(S, gate)) return;
   extern __shared__ unsigned long long sv[];  // two buffers of kBigRun entries
+  const int nm = list_n[2];
+  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nm;
+       w += (gridDim.x * blockDim.x) >> 5) {
+    const int c = mid[w];
+    const int b = start[c];
+    warp_sort_segment(perm, b, start[c + 1] - b, threadIdx.x & 31, tmp);
+  }
   const int nb = list_n[1];
   for (int q = blockIdx.x; q < nb; q += gridDim.x) {
     const int c = big[q];
@@ -1293,27 +1309,6 @@ __device__ __forceinline__ long long unit_weight(const Scalars* S,
   return T < kUnitMinWeight ? kUnitMinWeight : T;
 }
 
-__global__ void __launch_bounds__(kPlanThreads)
-    k_units_plan(const int* __restrict__ cstart, Geom G, const Scalars* S,
-                 int target_units, int seg, int* __restrict__ ustart,
-                 long long* __restrict__ upex, int4* __restrict__ plan,
-                 int* __restrict__ strip_n, int* __restrict__ heavy_n) {
-  if (!S->active) return;
-  const int strip = blockIdx.x;
-  const size_t b = (size_t)strip * seg;
-  // node columns of the cells the particles are binned to (the key range the
-  // scatter just rolled over), plus the column right of them
-  const int L = S->krange[0], H = S->krange[1];
-  if (L > H) {  // no particle
-    if (threadIdx.x == 0) strip_n[strip] = 0;
-    return;
-  }
-  const int c_lo = L / G.nrows, c_hi = min(H / G.nrows + 1, G.ncols);
-  const int J = plan_strip(cstart, G, unit_weight(S, target_units), strip,
-                           ustart + b, upex + b, plan + b, kColWeight, c_lo, c_hi, heavy_n);
-  if (threadIdx.x == 0) strip_n[strip] = J;
-}
-
 // The order P2G hands the units out in: the heavy ones first, then the
 // others, each group in list order (a stable partition; heavy(f) is 0 or 1).
 // A unit's ledger slot stays its list position, so the order changes no sum.
@@ -1336,39 +1331,78 @@ __device__ __forceinline__ void heavy_first(int total, F heavy, int* __restrict_
   }
 }
 
-// One block: strip offsets by a scan of strip_n, then the flat unit list
-// {strip, cA, cB} in (strip, column) order.  ucount[0] = units,
-// ucount[1] = P2G's work cursor, ucount[2] = heavy units (P2G reads uorder
-// when there are any, else takes the list in order), ucount[3] = the heavy
-// units the plan counts for the next list.
-__global__ void __launch_bounds__(kPlanThreads)
-    k_units_flat(const int* __restrict__ strip_n, int strips, int seg,
-                 const int4* __restrict__ plan, int4* __restrict__ ulist,
-                 int* __restrict__ uorder, int* __restrict__ ucount, const Scalars* S) {
-  if (!S->active) return;
-  const int H = ucount[3];  // heavy units, counted by the plan
-  extern __shared__ int uoff[];  // strips + 1
-  __shared__ int wt_i[32];
+// Strip offsets uoff (strips + 1) by a scan of strip_n, by all threads of the
+// block; returns the number of units.
+__device__ __forceinline__ int strip_offsets(const int* strip_n, int strips, int* uoff,
+                                             int* wt) {
   int carry = 0;
   for (int base = 0; base < strips; base += blockDim.x) {
     const int s = base + threadIdx.x;
-    const int n = s < strips ? strip_n[s] : 0;
+    const int n = s < strips ? __ldcg(strip_n + s) : 0;
     int tot;
-    const int incl = block_incl_scan<int>(n, wt_i, tot);
+    const int incl = block_incl_scan<int>(n, wt, tot);
     if (s < strips) uoff[s] = carry + incl - n;
     carry += tot;
   }
   if (threadIdx.x == 0) uoff[strips] = carry;
   __syncthreads();
-  const int total = carry;
+  return carry;
+}
+
+__device__ __forceinline__ int strip_of_unit(const int* uoff, int strips, int f) {
+  int lo = 0, hi = strips;  // uoff[lo] <= f < uoff[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (uoff[mid] <= f) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// One block per strip cuts its units; the last block to finish writes the
+// flat list {strip, cA, cB} in (strip, column) order and, unless the pass has
+// begun (a merge/split came before the sort), ends the step before and begins
+// this one.
+// A small scenario's step is bound by its chain of launches (2-3 us each with
+// the gap before it): the list, the step's begin and end, the ledger (a block
+// of G2P) and the sort of the larger cells were launches of their own, 13 in
+// all; with 8 the step of a 4096-particle dam break takes 42 us instead of
+// 49, that of a 0.25M-particle mudflow 97 instead of 104.  The begin sits here
+// and not at the end of G2P, where every block would have to wait for its
+// stores before it counts itself done (7 us at 0.25M and 4M particles).
+// ucount[0] = units, ucount[1] = P2G's work cursor, ucount[2] = heavy units
+// (P2G reads uorder when there are any, else takes the list in order),
+// ucount[3] = the heavy units the strips count, ucount[4] = the blocks done.
+__global__ void __launch_bounds__(kPlanThreads)
+    k_units(const int* __restrict__ cstart, Geom G, Phys P, Scalars* S, int target_units,
+            int seg, int* __restrict__ ustart, long long* __restrict__ upex, int4* plan,
+            int* strip_n, int4* ulist, int* __restrict__ uorder, int* ucount, Gate gate) {
+  if (!gate_open(S, gate)) {
+    if (!gate.begun && blockIdx.x == 0 && threadIdx.x == 0) S->active = 0;
+    return;
+  }
+  extern __shared__ int uoff[];  // strips + 1
+  __shared__ int wt_i[32];
+  const int strip = blockIdx.x, strips = gridDim.x;
+  const size_t b = (size_t)strip * seg;
+  // node columns of the cells the particles are binned to (the key range the
+  // scatter just rolled over), plus the column right of them
+  const int L = S->krange[0], K = S->krange[1];
+  int J = 0;
+  if (L <= K) {
+    const int c_lo = L / G.nrows, c_hi = min(K / G.nrows + 1, G.ncols);
+    J = plan_strip(cstart, G, unit_weight(S, target_units), strip, ustart + b, upex + b,
+                   plan + b, kColWeight, c_lo, c_hi, ucount + 3);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) strip_n[strip] = J;
+  if (!last_block(ucount + 4, strips)) return;
+  const int H = __ldcg(ucount + 3);
+  const int total = strip_offsets(strip_n, strips, uoff, wt_i);
   for (int f = threadIdx.x; f < total; f += blockDim.x) {
-    int lo = 0, hi = strips;  // uoff[lo] <= f < uoff[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (uoff[mid] <= f) lo = mid; else hi = mid;
-    }
-    const int4 u = plan[(size_t)lo * seg + (f - uoff[lo])];
-    ulist[f] = make_int4(lo, u.x, u.y, u.z);  // w: heavy
+    const int s = strip_of_unit(uoff, strips, f);
+    const int4 u = __ldcg(plan + (size_t)s * seg + (f - uoff[s]));
+    ulist[f] = make_int4(s, u.x, u.y, u.z);  // w: heavy
   }
   if (H > 0) {
     __syncthreads();
@@ -1379,6 +1413,7 @@ __global__ void __launch_bounds__(kPlanThreads)
     ucount[1] = 0;
     ucount[2] = H;  // P2G: list order when 0
     ucount[3] = 0;
+    if (!gate.begun) step_begin_one(S, G, P);
   }
 }
 
@@ -1562,7 +1597,7 @@ __global__ void __launch_bounds__(kP2GThreads, kP2GMinBlocks)
 size_t sort_big_smem_bytes() { return 2 * sizeof(unsigned long long) * kBigRun; }
 
 int setup_sort() {
-  return cudaFuncSetAttribute(k_segment_order_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(k_segment_order_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               int(sort_big_smem_bytes())) == cudaSuccess;
 }
 
@@ -1628,10 +1663,9 @@ __device__ __forceinline__ void ledger_reduce(const double* __restrict__ led_par
 }
 
 // log: a ring of kLedgerLog rows {t, err_mass, err_mom}, row (it-1) % kLedgerLog
-__global__ void k_ledger_final(const double* __restrict__ led_part,
-                               const int* __restrict__ ucount, Scalars* S,
-                               double* __restrict__ log) {
-  if (!S->active) return;
+__device__ __forceinline__ void ledger_final(const double* __restrict__ led_part,
+                                             const int* __restrict__ ucount, Scalars* S,
+                                             double* __restrict__ log) {
   ledger_reduce(led_part, 0, ucount[0], S);
   if (threadIdx.x == 0 && log) {
     double* row = log + 3 * ((S->it - 1) % kLedgerLog);
@@ -1912,13 +1946,22 @@ template <bool kRecord, bool kGrad>
 __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     k_g2p_t(Particles cur, Particles nxt, const int* __restrict__ perm,
             const int* __restrict__ skey, Nodes nodes, const double* __restrict__ Z, Geom G,
-            Phys P, Scalars* S, int* __restrict__ count, int* __restrict__ leave) {
+            Phys P, Scalars* S, int* __restrict__ count, int* __restrict__ leave,
+            const double* __restrict__ led_part, const int* __restrict__ ucount,
+            double* __restrict__ log) {
   const int ng = S->nghost;
   const int n = S->np - ng;  // the slab's own particles
-  const int stride = gridDim.x * blockDim.x;
+  const int blk = blockIdx.x - 1;  // the first block sums the ledger
+  const int stride = (gridDim.x - 1) * blockDim.x;
   if (!S->active) {  // (ghosts, imported last, sit in the slots after n)
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride)
-      copy_moving(cur, j, nxt, j);
+    if (blk >= 0)
+      for (int j = blk * blockDim.x + threadIdx.x; j < n; j += stride)
+        copy_moving(cur, j, nxt, j);
+    return;
+  }
+  if (blk < 0) {
+    ledger_final(led_part, ucount, S, log);
+    if (threadIdx.x == 0) S->pending = 1;
     return;
   }
   __shared__ unsigned long long red[3];
@@ -1934,7 +1977,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
   unsigned long long m0 = 0, m1 = 0, m2 = 0;
   int bad = 0, kmin = 0x7fffffff, kmax = -1;
   const int lane = threadIdx.x & 31;
-  for (int t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); t0 < n; t0 += stride) {
+  for (int t0 = blk * blockDim.x + (threadIdx.x & ~31); t0 < n; t0 += stride) {
     const int t = t0 + lane;
     const bool ok = t < n;
     int nkey = -1;
@@ -1963,16 +2006,12 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
 
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
-                int* count, int* leave, int record, int want_grad) {
-  if (record)
-    k_g2p_t<true, true><<<grid, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G, P,
-                                                       S, count, leave);
-  else if (want_grad)
-    k_g2p_t<false, true><<<grid, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G, P,
-                                                        S, count, leave);
-  else
-    k_g2p_t<false, false><<<grid, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G,
-                                                         P, S, count, leave);
+                int* count, int* leave, const double* led_part, const int* ucount, double* log,
+                int record, int want_grad) {
+  auto* kernel = record ? k_g2p_t<true, true>
+                        : want_grad ? k_g2p_t<false, true> : k_g2p_t<false, false>;
+  kernel<<<grid + 1, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G, P, S, count,
+                                           leave, led_part, ucount, log);
 }
 
 size_t p2g_smem_bytes() { return sizeof(P2GSmemT<double>); }
@@ -2000,64 +2039,6 @@ __global__ void k_to_f64(const float* __restrict__ a, double* __restrict__ b,
 // numbers are the same alone and in a batch: its sums run in the same
 // per-node order whatever the unit cuts.
 // ---------------------------------------------------------------------------
-__global__ void k_b_step_begin(const Scn* __restrict__ scn, Scalars* S, int nscn,
-                               Scalars* Sg) {
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
-  for (int s = threadIdx.x; s < nscn; s += blockDim.x) {
-    if (scn[s].live) {
-      step_begin_one(&S[s], scn[s].G, scn[s].P);
-      if (S[s].active) atomicOr(&any, 1);
-    } else {
-      S[s].active = 0;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) Sg->active = any;
-}
-
-__global__ void k_b_step_end(const Scn* __restrict__ scn, Scalars* S, int nscn) {
-  for (int s = threadIdx.x; s < nscn; s += blockDim.x)
-    if (scn[s].live) step_end_one(&S[s]);
-}
-
-// one block per strip of the batch
-__global__ void __launch_bounds__(kPlanThreads)
-    k_b_units_plan(const int* __restrict__ cstart, const Scn* __restrict__ scn,
-                   const Scalars* S, const int* __restrict__ strip_scn,
-                   const Scalars* Sg, int target_units, int col_weight,
-                   int* __restrict__ ustart,
-                   long long* __restrict__ upex, int4* __restrict__ plan,
-                   int* __restrict__ strip_n, int* __restrict__ heavy_n) {
-  const int b = blockIdx.x;
-  const int s = strip_scn[b];
-  if (!Sg->active || !S[s].active) {
-    if (threadIdx.x == 0) strip_n[b] = 0;
-    return;
-  }
-  const Geom G = scn[s].G;
-  const int local = b - scn[s].strip_off;
-  const size_t base = (size_t)scn[s].useg_off + (size_t)local * (G.ncols + 1);
-  // node columns of the cells the scenario's particles are binned to (the
-  // keys its last G2P made), plus the column right of them; every column
-  // after a layout change
-  int c_lo = 0, c_hi = G.ncols;
-  if (!(Sg->krange[0] <= Sg->krange[1])) {
-    const int L = S[s].knext[0], H = S[s].knext[1];
-    if (L > H) {  // no particle
-      if (threadIdx.x == 0) strip_n[b] = 0;
-      return;
-    }
-    c_lo = (L - scn[s].c_off) / G.nrows;
-    c_hi = min((H - scn[s].c_off) / G.nrows + 1, G.ncols);
-  }
-  const int J = plan_strip(cstart + scn[s].c_off, G, unit_weight(Sg, target_units),
-                           local, ustart + base, upex + base, plan + base, col_weight,
-                           c_lo, c_hi, heavy_n);
-  if (threadIdx.x == 0) strip_n[b] = J;
-}
-
 // The scan tiles of a batch pass: those that meet the batch-wide range
 // (every cell after a layout change) or a scenario's keys -- the keys its
 // cell starts describe (krange) or the keys its last G2P made (knext).  A
@@ -2065,13 +2046,27 @@ __global__ void __launch_bounds__(kPlanThreads)
 // its cells' starts (the particles of the scenarios before them) stand
 // while the layout does.  One thread per tile; the scenarios' cells are
 // consecutive, so a binary search finds the first that meets the tile.
-__global__ void k_b_tile_flags(const Scn* __restrict__ scn, const Scalars* S, int nscn,
-                               const Scalars* Sg, unsigned char* __restrict__ tflag,
-                               int ntiles) {
-  if (!Sg->active) return;
+// One more block, the first, ends every scenario's step before and begins
+// this one (the tile blocks read neither).
+__global__ void k_b_step_begin(const Scn* __restrict__ scn, Scalars* S, int nscn, Scalars* Sg,
+                               unsigned char* __restrict__ tflag, int ntiles) {
+  if (blockIdx.x == 0) {
+    int any = 0;
+    for (int s = threadIdx.x; s < nscn; s += blockDim.x) {
+      if (scn[s].live) {
+        step_begin_one(&S[s], scn[s].G, scn[s].P);
+        any |= S[s].active;
+      } else {
+        S[s].active = 0;
+      }
+    }
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) Sg->active = any;
+    return;
+  }
   const int gL = min(Sg->krange[0], Sg->knext[0]), gH = max(Sg->krange[1], Sg->knext[1]);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles;
-       t += gridDim.x * blockDim.x) {
+  for (int t = (blockIdx.x - 1) * blockDim.x + threadIdx.x; t < ntiles;
+       t += (gridDim.x - 1) * blockDim.x) {
     const int c0 = t * kScanTile, c1 = c0 + kScanTile - 1;
     bool f = gL <= gH && gL <= c1 && gH >= c0;
     int lo = 0, hi = nscn;  // the first scenario whose cells end after c0
@@ -2089,42 +2084,62 @@ __global__ void k_b_tile_flags(const Scn* __restrict__ scn, const Scalars* S, in
   }
 }
 
-// one block: the flat list {scenario, strip, cA, cB} in strip order, and each
-// scenario's range of list positions (its ledger slots)
+// The last pass of a call: every scenario's step ends.
+__global__ void k_b_step_end(const Scn* __restrict__ scn, Scalars* S, int nscn) {
+  for (int s = threadIdx.x; s < nscn; s += blockDim.x)
+    if (scn[s].live) step_end_one(&S[s]);
+}
+
+// One block per strip of the batch cuts its units; the last block to finish
+// writes the flat list {scenario, strip, cA, cB} in strip order and each
+// scenario's range of list positions (its ledger slots) and rolls the key
+// ranges over.  ucount as in k_units.
 __global__ void __launch_bounds__(kPlanThreads)
-    k_b_units_flat(const int* __restrict__ strip_n, int strips,
-                   const int* __restrict__ strip_scn, const Scn* __restrict__ scn,
-                   int nscn, const int4* __restrict__ plan, int4* __restrict__ ulist,
-                   int* __restrict__ uorder, int* __restrict__ ucount,
-                   int2* __restrict__ scn_units,
-                   Scalars* S, const Scalars* Sg) {
+    k_b_units(const int* __restrict__ cstart, const Scn* __restrict__ scn, Scalars* S,
+              int nscn, const int* __restrict__ strip_scn, const Scalars* Sg,
+              int target_units,
+              int col_weight, int* __restrict__ ustart, long long* __restrict__ upex,
+              int4* plan, int* strip_n, int4* ulist, int* __restrict__ uorder, int* ucount,
+              int2* __restrict__ scn_units) {
   if (!Sg->active) return;
-  const int H = ucount[3];  // heavy units, counted by the plan
   extern __shared__ int uoff[];  // strips + 1
   __shared__ int wt_i[32];
-  int carry = 0;
-  for (int base = 0; base < strips; base += blockDim.x) {
-    const int b = base + threadIdx.x;
-    const int n = b < strips ? strip_n[b] : 0;
-    int tot;
-    const int incl = block_incl_scan<int>(n, wt_i, tot);
-    if (b < strips) uoff[b] = carry + incl - n;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) uoff[strips] = carry;
-  __syncthreads();
-  const int total = carry;
-  for (int f = threadIdx.x; f < total; f += blockDim.x) {
-    int lo = 0, hi = strips;  // uoff[lo] <= f < uoff[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (uoff[mid] <= f) lo = mid; else hi = mid;
+  const int b = blockIdx.x, strips = gridDim.x;
+  {
+    const int s = strip_scn[b];
+    int J = 0;
+    if (S[s].active) {
+      const Geom G = scn[s].G;
+      const int local = b - scn[s].strip_off;
+      const size_t base = (size_t)scn[s].useg_off + (size_t)local * (G.ncols + 1);
+      // node columns of the cells the scenario's particles are binned to (the
+      // keys its last G2P made), plus the column right of them; every column
+      // after a layout change
+      int c_lo = 0, c_hi = G.ncols;
+      if (!(Sg->krange[0] <= Sg->krange[1])) {
+        const int L = S[s].knext[0], H = S[s].knext[1];
+        c_lo = (L - scn[s].c_off) / G.nrows;
+        c_hi = L > H ? -1 : min((H - scn[s].c_off) / G.nrows + 1, G.ncols);
+      }
+      if (c_hi >= 0)  // (else no particle)
+        J = plan_strip(cstart + scn[s].c_off, G, unit_weight(Sg, target_units), local,
+                       ustart + base, upex + base, plan + base, col_weight, c_lo, c_hi,
+                       ucount + 3);
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) strip_n[b] = J;
+  }
+  if (!last_block(ucount + 4, strips)) return;
+  const int H = __ldcg(ucount + 3);
+  const int total = strip_offsets(strip_n, strips, uoff, wt_i);
+  for (int f = threadIdx.x; f < total; f += blockDim.x) {
+    const int lo = strip_of_unit(uoff, strips, f);
     const int s = strip_scn[lo];
     const int local = lo - scn[s].strip_off;
     const size_t base =
         (size_t)scn[s].useg_off + (size_t)local * (scn[s].G.ncols + 1);
-    const int4 u = plan[base + (f - uoff[lo])];
+    const int4 u = __ldcg(plan + base + (f - uoff[lo]));
     ulist[f] = make_int4(s, local, u.x, u.y);
   }
   if (H > 0) {
@@ -2135,7 +2150,7 @@ __global__ void __launch_bounds__(kPlanThreads)
         const int4 L = ulist[f];
         const int st = scn[L.x].strip_off + L.y;
         const size_t base = (size_t)scn[L.x].useg_off + (size_t)L.y * (scn[L.x].G.ncols + 1);
-        return plan[base + (f - uoff[st])].z;
+        return __ldcg(plan + base + (f - uoff[st])).z;
       },
       uorder, wt_i);
   }
@@ -2187,31 +2202,32 @@ __global__ void __launch_bounds__(kP2GThreads, kP2GMinBlocks)
   }
 }
 
-// one block per scenario
-__global__ void k_b_ledger(const double* __restrict__ led_part,
-                           const int2* __restrict__ scn_units,
-                           const Scn* __restrict__ scn, Scalars* S, int nscn,
-                           const Scalars* Sg) {
-  const int s = blockIdx.x;
-  if (!Sg->active || s >= nscn || !scn[s].live || !S[s].active) return;
-  ledger_reduce(led_part, scn_units[s].x, scn_units[s].y, &S[s]);
-}
-
 // gblk[b] = {scenario, its first particle handled by block b}.  A
 // scenario's particles are positions [p_off, p_off + np) of the sorted order
 // (its cell keys lie between those of the scenarios before and after it).
 // Thread j takes position j: slot perm[j] of `cur`, written to slot j of
 // `nxt`; a scenario that does not step in this pass (finished, stopped or
 // removed) is copied through in sorted order and counted for the next sort;
-// a pass in which no scenario steps copies `cur` to `nxt` unchanged.
+// a pass in which no scenario steps copies `cur` to `nxt` unchanged.  The
+// first nscn blocks sum one scenario's ledger each.
 template <class R>
 __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     k_b_g2p(ParticlesT<R> cur, ParticlesT<R> nxt, const int* __restrict__ perm,
             const int* __restrict__ skey, const V2<R>* __restrict__ vvL,
             const double* __restrict__ Z,
             const Scn* __restrict__ scn, Scalars* S, const int2* __restrict__ gblk,
-            Scalars* Sg, int* __restrict__ count) {
-  const int2 e = gblk[blockIdx.x];
+            const Scalars* Sg, int* __restrict__ count, const double* __restrict__ led_part,
+            const int2* __restrict__ scn_units, int nscn) {
+  if (blockIdx.x < nscn) {
+    const int q = blockIdx.x;
+    if (!Sg->active) return;
+    if (scn[q].live && S[q].active) {
+      ledger_reduce(led_part, scn_units[q].x, scn_units[q].y, &S[q]);
+      if (threadIdx.x == 0) S[q].pending = 1;
+    }
+    return;
+  }
+  const int2 e = gblk[blockIdx.x - nscn];
   const int s = e.x;
   const int p_off = scn[s].p_off, np = scn[s].np;
   const int li = e.y + threadIdx.x;
@@ -2365,11 +2381,12 @@ int setup_b_p2g() {
 }
 
 template <class R>
-void launch_b_g2p(int grid, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nxt,
+void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nxt,
                   const int* perm, const int* skey, const V2<R>* vvL, const double* Z,
-                  const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count) {
-  k_b_g2p<R><<<grid, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, vvL, Z, scn, S, gblk, Sg,
-                                           count);
+                  const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count,
+                  const double* led_part, const int2* scn_units, int nscn) {
+  k_b_g2p<R><<<nblk + nscn, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, vvL, Z, scn, S, gblk,
+                                                  Sg, count, led_part, scn_units, nscn);
 }
 
 template <class R>
@@ -2390,7 +2407,8 @@ void launch_b_move(int grid, cudaStream_t st, ParticlesT<R> dst, ParticlesT<R> s
   template int setup_b_p2g<R>();                                                      \
   template void launch_b_g2p<R>(int, cudaStream_t, ParticlesT<R>, ParticlesT<R>,      \
                                 const int*, const int*, const V2<R>*, const double*,  \
-                                const Scn*, Scalars*, const int2*, Scalars*, int*);   \
+                                const Scn*, Scalars*, const int2*, Scalars*, int*,    \
+                                const double*, const int2*, int);                     \
   template void launch_b_move<R>(int, cudaStream_t, ParticlesT<R>, ParticlesT<R>,     \
                                  const int4*);
 DAMPM_INSTANTIATE(double)
