@@ -24,6 +24,10 @@ using namespace dampm;
 
 namespace {
 
+// A piece of an addition's arrays (1 MB: a larger one costs more to set up
+// than it saves)
+constexpr size_t kRawDoubles = size_t(1) << 17;
+
 struct HostScn {
   int handle = -1;
   Scn d{};  // the device table entry
@@ -75,6 +79,18 @@ struct dampm_batch {
   Scn* scn = nullptr;
   Scalars *S = nullptr, *Sg = nullptr;
   Scalars* Sh = nullptr;  // pinned mirror of S
+  void* pinned = nullptr;  // the host memory of Sh, the mirrors and raw_h
+  // pinned mirrors of the tables: an addition appends its entries and copies
+  // them without waiting (only a compaction, which waits, rewrites them)
+  Scn* scn_h = nullptr;
+  int* strip_scn_h = nullptr;
+  int2* gblk_h = nullptr;
+  // staging of an addition's arrays, pinned and on the device, two of each:
+  // one is filled while the other travels
+  double* raw_h[2] = {nullptr, nullptr};
+  double* raw_d[2] = {nullptr, nullptr};
+  cudaEvent_t raw_ev[2] = {nullptr, nullptr};
+  int raw_turn = 0;
   int p2g_grid = 1;
   long long launches = 0;
   // tuning: P2G units per CTA and the weight of a column in the unit plan
@@ -186,38 +202,34 @@ ParticlesT<R> shifted(const ParticlesT<R>& p, long long off) {
 
 int strips_of(const dampm_grid& g) { return (g.Ney + 1 + kTR - 1) / kTR; }
 
-// Rebuilds the strip and G2P block tables from the host scenario list and
-// uploads them with the scenario table and the batch totals.
-int upload_tables(dampm_batch* b) {
-  std::vector<int> strip_scn(std::max(b->strips_tot, 1));
-  std::vector<int2> gblk;
-  gblk.reserve(b->nblk);
-  std::vector<Scn> tab(b->scns.size());
-  for (size_t s = 0; s < b->scns.size(); ++s) {
-    const Scn& d = b->scns[s].d;
-    tab[s] = d;
-    for (int k = 0; k < d.nstrips; ++k) strip_scn[d.strip_off + k] = int(s);
-    for (int f = 0; f < d.np; f += kG2PThreads) gblk.push_back(make_int2(int(s), f));
-  }
-  b->nblk = int(gblk.size());
-  if (!tab.empty())
-    BCK(cudaMemcpyAsync(b->scn, tab.data(), sizeof(Scn) * tab.size(),
+// Appends scenario `pos` to the table mirrors; the entries' ranges in *strip
+// and *blk.
+void append_tables(dampm_batch* b, size_t pos, int2* strip, int2* blk) {
+  const Scn& d = b->scns[pos].d;
+  b->scn_h[pos] = d;
+  *strip = make_int2(d.strip_off, d.nstrips);
+  for (int k = 0; k < d.nstrips; ++k) b->strip_scn_h[d.strip_off + k] = int(pos);
+  blk->x = b->nblk;
+  for (int f = 0; f < d.np; f += kG2PThreads) b->gblk_h[b->nblk++] = make_int2(int(pos), f);
+  blk->y = b->nblk - blk->x;
+}
+
+// Uploads entries of the tables (scenarios, strips, G2P blocks) with the
+// batch totals, without waiting.
+int upload_tables(dampm_batch* b, int2 scn, int2 strip, int2 blk) {
+  if (scn.y > 0)
+    BCK(cudaMemcpyAsync(b->scn + scn.x, b->scn_h + scn.x, sizeof(Scn) * size_t(scn.y),
                         cudaMemcpyHostToDevice, b->stream));
-  BCK(cudaMemcpyAsync(b->strip_scn, strip_scn.data(), sizeof(int) * strip_scn.size(),
-                      cudaMemcpyHostToDevice, b->stream));
-  if (!gblk.empty())
-    BCK(cudaMemcpyAsync(b->gblk, gblk.data(), sizeof(int2) * gblk.size(),
+  if (strip.y > 0)
+    BCK(cudaMemcpyAsync(b->strip_scn + strip.x, b->strip_scn_h + strip.x,
+                        sizeof(int) * size_t(strip.y), cudaMemcpyHostToDevice, b->stream));
+  if (blk.y > 0)
+    BCK(cudaMemcpyAsync(b->gblk + blk.x, b->gblk_h + blk.x, sizeof(int2) * size_t(blk.y),
                         cudaMemcpyHostToDevice, b->stream));
-  Scalars g{};
-  g.np = int(b->P_tot);
-  g.active = 1;
   // the next sort scans every cell of the new layout
-  g.krange[0] = 0x7fffffff;
-  g.krange[1] = -1;
-  g.knext[0] = 0;
-  g.knext[1] = int(std::max<long long>(b->C_tot, 1)) - 1;
-  BCK(cudaMemcpyAsync(b->Sg, &g, sizeof(Scalars), cudaMemcpyHostToDevice, b->stream));
-  BCK(cudaStreamSynchronize(b->stream));  // host vectors die here
+  k_b_layout<<<1, 1, 0, b->stream>>>(b->Sg, int(b->P_tot),
+                                     int(std::max<long long>(b->C_tot, 1)));
+  BCK(cudaGetLastError());
   b->graph_dirty[0] = b->graph_dirty[1] = true;  // launch sizes or buffers changed
   return DAMPM_OK;
 }
@@ -301,29 +313,62 @@ int enqueue_end(dampm_batch* b) {
   return DAMPM_OK;
 }
 
-// Particles of one scenario into the current half (converted to R on the
-// host), then the initial state of main/optim_par.cpp:239-264 on the device.
+// A piece of an addition's host arrays in flight: `fill` writes it into a
+// pinned buffer, which is copied to its device twin (*dev).  Two buffers
+// alternate, so the host fills one while the other travels; raw_sent marks
+// the end of what reads the device twin.
+template <class F>
+int stage_raw(dampm_batch* b, size_t n, F fill, double** dev) {
+  const int t = b->raw_turn;
+  BCK(cudaEventSynchronize(b->raw_ev[t]));
+  fill(b->raw_h[t]);
+  BCK(cudaMemcpyAsync(b->raw_d[t], b->raw_h[t], sizeof(double) * n, cudaMemcpyHostToDevice,
+                      b->stream));
+  *dev = b->raw_d[t];
+  return DAMPM_OK;
+}
+int raw_sent(dampm_batch* b) {
+  BCK(cudaEventRecord(b->raw_ev[b->raw_turn], b->stream));
+  b->raw_turn ^= 1;
+  return DAMPM_OK;
+}
+
+// Terrain and particles of one scenario into the current half, then the
+// initial state of main/optim_par.cpp:239-264 on the device.  The arrays go
+// through the staging in pieces and are converted on the device, so the call
+// waits for nothing but a free piece (96 scenarios of 12000 particles: 31 ms
+// in FP64 and 42 in FP32 with one copy, one wait and a conversion on the host
+// per array).
 template <class R>
-int upload_scenario(dampm_batch* b, const Scn& d, int pos, long long np,
-                    const double* const* in, double* Zs) {
+int upload_scenario(dampm_batch* b, const Scn& d, int pos, long long np, long long nn,
+                    const double* Z, const double* const* in, double* Zs) {
   ParticlesT<R> p = shifted(halves<R>(b)[b->cur], d.p_off);
-  // in: x, y, Mp, Ap, vpx, vpy, hp, mom_px, mom_py, Vp
-  R* dst[10] = {p.x, p.y, p.Mp, p.Ap, p.vpx, p.vpy, p.hp, nullptr, nullptr, p.Vp};
   cudaStream_t st = b->stream;
-  std::vector<R> tmp, tmp2;
-  auto host_r = [&](int k, std::vector<R>& t) -> const R* {
-    if (sizeof(R) == sizeof(double)) return reinterpret_cast<const R*>(in[k]);
-    t.assign(in[k], in[k] + np);
-    return t.data();
-  };
-  for (int k = 0; k < 10; ++k) {
-    if (!dst[k]) continue;
-    BCK(cudaMemcpyAsync(dst[k], host_r(k, tmp), sizeof(R) * size_t(np),
-                        cudaMemcpyHostToDevice, st));
-    if (sizeof(R) != sizeof(double)) BCK(cudaStreamSynchronize(st));  // tmp is reused
+  for (long long o = 0; o < nn; o += (long long)kRawDoubles) {
+    const size_t n = size_t(std::min<long long>((long long)kRawDoubles, nn - o));
+    double* dev = nullptr;
+    int rc = stage_raw(b, n, [&](double* h) { std::memcpy(h, Z + o, sizeof(double) * n); }, &dev);
+    if (rc) return rc;
+    BCK(cudaMemcpyAsync(Zs + o, dev, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+    rc = raw_sent(b);
+    if (rc) return rc;
   }
-  BCK(upload_pair(p.mp, host_r(7, tmp), host_r(8, tmp2), np, st));
-  BCK(cudaStreamSynchronize(st));
+  const long long per = (long long)(kRawDoubles / 10);
+  for (long long o = 0; o < np; o += per) {
+    const size_t n = size_t(std::min(per, np - o));
+    double* dev = nullptr;
+    int rc = stage_raw(
+        b, 10 * n,
+        [&](double* h) {
+          for (int k = 0; k < 10; ++k) std::memcpy(h + k * n, in[k] + o, sizeof(double) * n);
+        },
+        &dev);
+    if (rc) return rc;
+    launch_b_unpack<R>(grid_blocks((long long)n, 256), st, shifted(p, o), dev, int(n));
+    b->launches += 1;
+    rc = raw_sent(b);
+    if (rc) return rc;
+  }
   // (the terrain gradients only feed recorded outputs, which a batch does
   // not keep, so Z stands in for them)
   launch_init_particles<R>(grid_blocks(np, 256), 256, st, p, Zs, Zs, Zs, d.G, d.P,
@@ -455,9 +500,36 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   rc = rc ? rc : balloc(b, &b->scn, size_t(scenario_cap));
   rc = rc ? rc : balloc(b, &b->S, size_t(scenario_cap));
   rc = rc ? rc : balloc(b, &b->Sg, 1);
-  if (rc == DAMPM_OK &&
-      cudaMallocHost(&b->Sh, sizeof(Scalars) * size_t(scenario_cap)) != cudaSuccess)
-    rc = bfail(b, DAMPM_ERR_CUDA, "cudaMallocHost failed");
+  for (int k = 0; k < 2; ++k) {
+    rc = rc ? rc : balloc(b, &b->raw_d[k], kRawDoubles);
+    if (rc == DAMPM_OK &&
+        cudaEventCreateWithFlags(&b->raw_ev[k], cudaEventDisableTiming) != cudaSuccess)
+      rc = bfail(b, DAMPM_ERR_CUDA, "cudaEventCreate failed");
+  }
+  if (rc == DAMPM_OK) {  // one pinned allocation, cut up
+    size_t bytes = 0;
+    auto place = [&](size_t n) {
+      const size_t at = bytes;
+      bytes += (n + 255) / 256 * 256;
+      return at;
+    };
+    const size_t at_S = place(sizeof(Scalars) * size_t(scenario_cap));
+    const size_t at_scn = place(sizeof(Scn) * size_t(scenario_cap));
+    const size_t at_strip = place(sizeof(int) * size_t(b->STRIP_cap));
+    const size_t at_blk = place(sizeof(int2) * size_t(b->B_cap));
+    const size_t at_raw[2] = {place(sizeof(double) * kRawDoubles),
+                              place(sizeof(double) * kRawDoubles)};
+    if (cudaMallocHost(&b->pinned, bytes) != cudaSuccess) {
+      rc = bfail(b, DAMPM_ERR_CUDA, "cudaMallocHost failed");
+    } else {
+      char* p = static_cast<char*>(b->pinned);
+      b->Sh = reinterpret_cast<Scalars*>(p + at_S);
+      b->scn_h = reinterpret_cast<Scn*>(p + at_scn);
+      b->strip_scn_h = reinterpret_cast<int*>(p + at_strip);
+      b->gblk_h = reinterpret_cast<int2*>(p + at_blk);
+      for (int k = 0; k < 2; ++k) b->raw_h[k] = reinterpret_cast<double*>(p + at_raw[k]);
+    }
+  }
   if (rc == DAMPM_OK) {
     cudaMemsetAsync(b->count, 0, sizeof(int) * (nn + 4), b->stream);
     cudaMemsetAsync(b->vvL, 0, 2 * rsz * nn, b->stream);
@@ -486,7 +558,9 @@ int dampm_batch_destroy(dampm_batch* b) {
   for (cudaGraphExec_t g : b->graph)
     if (g) cudaGraphExecDestroy(g);
   for (void* q : b->allocs) cudaFree(q);
-  if (b->Sh) cudaFreeHost(b->Sh);
+  if (b->pinned) cudaFreeHost(b->pinned);
+  for (cudaEvent_t e : b->raw_ev)
+    if (e) cudaEventDestroy(e);
   if (b->own_stream) cudaStreamDestroy(b->stream);
   delete b;
   return DAMPM_OK;
@@ -535,7 +609,6 @@ int dampm_batch_add(dampm_batch* b, const dampm_grid* grid, const dampm_params* 
   // particles and terrain into the current half
   cudaStream_t st = b->stream;
   double* Zs = b->Z[b->zcur] + d.n_off;
-  BCK(cudaMemcpyAsync(Zs, Z, sizeof(double) * size_t(h.nn), cudaMemcpyHostToDevice, st));
   Scalars s0{};
   s0.fresh = 1;
   s0.np = int(np);
@@ -548,8 +621,9 @@ int dampm_batch_add(dampm_batch* b, const dampm_grid* grid, const dampm_params* 
   BCK(cudaMemcpyAsync(b->S + pos, b->Sh + pos, sizeof(Scalars), cudaMemcpyHostToDevice,
                       st));
   const double* in[10] = {x, y, Mp, Ap, vpx, vpy, hp, mom_px, mom_py, Vp};
-  int urc = b->precision == DAMPM_FP32 ? upload_scenario<float>(b, d, pos, np, in, Zs)
-                                       : upload_scenario<double>(b, d, pos, np, in, Zs);
+  int urc = b->precision == DAMPM_FP32
+                ? upload_scenario<float>(b, d, pos, np, h.nn, Z, in, Zs)
+                : upload_scenario<double>(b, d, pos, np, h.nn, Z, in, Zs);
   if (urc) return urc;
   BCK(cudaGetLastError());
   b->scns.push_back(h);
@@ -558,7 +632,9 @@ int dampm_batch_add(dampm_batch* b, const dampm_grid* grid, const dampm_params* 
   b->C_tot += h.nc;
   b->strips_tot += nstrips;
   b->useg_tot += useg;
-  int rc = upload_tables(b);
+  int2 strip, blk;
+  append_tables(b, size_t(pos), &strip, &blk);
+  int rc = upload_tables(b, make_int2(pos, 1), strip, blk);
   if (rc) return rc;
   *handle = h.handle;
   return DAMPM_OK;
@@ -653,7 +729,13 @@ int dampm_batch_compact(dampm_batch* b) {
   b->C_tot = C;
   b->strips_tot = strips;
   b->useg_tot = U;
-  return upload_tables(b);
+  // every table entry anew, once the copies of the old ones have been made
+  BCK(cudaStreamSynchronize(b->stream));
+  b->nblk = 0;
+  int2 strip, blk;
+  for (size_t s = 0; s < keep.size(); ++s) append_tables(b, s, &strip, &blk);
+  return upload_tables(b, make_int2(0, int(keep.size())), make_int2(0, strips),
+                       make_int2(0, b->nblk));
 }
 
 // Passes per graph: even, so that a replay ends on the half it began.

@@ -97,6 +97,7 @@ struct dampm_ctx {
   int outbuf_fields = 0;
   long long outbuf_cap = 0;
   bool side_pending = false;
+  double* node_tmp = nullptr;  // one nodal field, for downloads
   // timing
   bool timing = false;
   std::vector<cudaEvent_t> evpool;
@@ -784,14 +785,14 @@ int dampm_upload_particles(dampm_ctx* ctx, long long np, const double* x,
   if (np > 0) {
     CK(cudaMemcpyAsync(p.x, x, b, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(p.y, y, b, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(p.xp, x, b, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(p.yp, y, b, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(p.xp, p.x, b, cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(p.yp, p.y, b, cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaMemcpyAsync(p.Mp, Mp, b, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(p.Ap, Ap, b, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(p.vpx, vpx, b, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(p.vpy, vpy, b, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(p.hp, hp, b, cudaMemcpyHostToDevice, ctx->stream));
-    CK(upload_pair(p.mp, mom_px, mom_py, np, ctx->stream));
+    CK(upload_pair(p.mp, mom_px, mom_py, np, ctx->msb.mx, ctx->msb.my, ctx->stream));
     CK(cudaMemcpyAsync(p.Vp, Vp, b, cudaMemcpyHostToDevice, ctx->stream));
   }
   Scalars s0{};
@@ -802,7 +803,6 @@ int dampm_upload_particles(dampm_ctx* ctx, long long np, const double* x,
   CK(cudaMemcpyAsync(ctx->S, ctx->Sh, sizeof(Scalars), cudaMemcpyHostToDevice,
                      ctx->stream));
   CK(cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));  // Sh is reused below
   if (np > 0) {
     // the slots hold the particles in DATA order (idx = slot)
     launch_init_particles<double>(grid_for(np, 256), 256, ctx->stream, p, ctx->Z,
@@ -1013,7 +1013,12 @@ int dampm_download_nodal(dampm_ctx* ctx, const char* field, double* out) {
   const double* src = nullptr;
   Nodes& n = ctx->nodes;
   if (f == "vvxL" || f == "vvyL") {
-    CK(download_pair_half(out, n.vvL, f == "vvxL" ? 0 : 1, ctx->nn, ctx->stream));
+    if (!ctx->node_tmp) {  // (first use; outputs only)
+      const int rc = dalloc(ctx, &ctx->node_tmp, size_t(ctx->nn));
+      if (rc) return rc;
+    }
+    CK(download_pair_half(out, n.vvL, f == "vvxL" ? 0 : 1, ctx->nn, ctx->node_tmp,
+                          ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return DAMPM_OK;
   }
@@ -1087,7 +1092,7 @@ int dampm_set_state(dampm_ctx* ctx, long long np, const double* const* fields,
   const bool fresh = Ap && mom_px && mom_py && Fb_x && Fb_y;
   if (fresh) {
     CK(cudaMemcpyAsync(p.Ap, Ap, b, cudaMemcpyHostToDevice, ctx->stream));
-    CK(upload_pair(p.mp, mom_px, mom_py, np, ctx->stream));
+    CK(upload_pair(p.mp, mom_px, mom_py, np, ctx->msb.mx, ctx->msb.my, ctx->stream));
     CK(cudaMemcpyAsync(p.Fbx, Fb_x, b, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(p.Fby, Fb_y, b, cudaMemcpyHostToDevice, ctx->stream));
   }

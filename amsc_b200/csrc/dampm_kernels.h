@@ -236,9 +236,15 @@ void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nx
 template <class R>
 void launch_b_move(int grid, cudaStream_t st, ParticlesT<R> dst, ParticlesT<R> src,
                    const int4* mblk);
-// float <-> double copies of one particle field (FP32 batch upload/download)
-__global__ void k_to_f32(const double* a, float* b, long long n);
-__global__ void k_to_f64(const float* a, double* b, long long n);
+// n particles of a new scenario from raw[10][n] (x, y, Mp, Ap, vpx, vpy, hp,
+// mom_px, mom_py, Vp), converted to R
+template <class R>
+void launch_b_unpack(int grid, cudaStream_t st, ParticlesT<R> p, const double* raw, int n);
+// the totals of a batch's layout; the next sort scans every cell of it
+__global__ void k_b_layout(Scalars* Sg, int np, int ncells);
+// pairs from their halves, and one half of them
+__global__ void k_pair_join(const double* a, const double* b, double2* out, long long n);
+__global__ void k_pair_half(const double2* a, int half, double* out, long long n);
 __global__ void k_b_move_nodes(double* dst, const double* src, const int4* nblk);
 
 __global__ void k_hv(const Particles p, const int* cstart, double* HV, Geom G,

@@ -2016,18 +2016,20 @@ void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const i
 
 size_t p2g_smem_bytes() { return sizeof(P2GSmemT<double>); }
 
-__global__ void k_to_f32(const double* __restrict__ a, float* __restrict__ b,
-                         long long n) {
+__global__ void k_pair_join(const double* __restrict__ a, const double* __restrict__ b,
+                            double2* __restrict__ out, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
-    b[i] = float(a[i]);
+    out[i] = double2{a[i], b[i]};
 }
 
-__global__ void k_to_f64(const float* __restrict__ a, double* __restrict__ b,
-                         long long n) {
+__global__ void k_pair_half(const double2* __restrict__ a, int half, double* __restrict__ out,
+                            long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    b[i] = double(a[i]);
+       i += (long long)gridDim.x * blockDim.x) {
+    const double2 v = a[i];
+    out[i] = half ? v.y : v.x;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2273,6 +2275,28 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
   flag_non_finite(bad, &S[s]);
 }
 
+template <class R>
+__global__ void k_b_unpack(ParticlesT<R> p, const double* __restrict__ raw, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    R* const dst[8] = {p.x, p.y, p.Mp, p.Ap, p.vpx, p.vpy, p.hp, p.Vp};
+    constexpr int at[8] = {0, 1, 2, 3, 4, 5, 6, 9};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) dst[k][i] = R(raw[(size_t)at[k] * n + i]);
+    p.mp[i] = V2<R>{R(raw[(size_t)7 * n + i]), R(raw[(size_t)8 * n + i])};
+  }
+}
+
+__global__ void k_b_layout(Scalars* Sg, int np, int ncells) {
+  Scalars s{};
+  s.np = np;
+  s.active = 1;
+  s.krange[0] = 0x7fffffff;
+  s.krange[1] = -1;
+  s.knext[0] = 0;
+  s.knext[1] = ncells - 1;
+  *Sg = s;
+}
+
 // Compaction of a batch into the other half of its double buffer:
 // mblk[b] = {destination first particle, source first particle, count <= 256,
 // cell-key shift}.
@@ -2390,6 +2414,11 @@ void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nx
 }
 
 template <class R>
+void launch_b_unpack(int grid, cudaStream_t st, ParticlesT<R> p, const double* raw, int n) {
+  k_b_unpack<R><<<grid, 256, 0, st>>>(p, raw, n);
+}
+
+template <class R>
 void launch_b_move(int grid, cudaStream_t st, ParticlesT<R> dst, ParticlesT<R> src,
                    const int4* mblk) {
   k_b_move<R><<<grid, kG2PThreads, 0, st>>>(dst, src, mblk);
@@ -2409,6 +2438,7 @@ void launch_b_move(int grid, cudaStream_t st, ParticlesT<R> dst, ParticlesT<R> s
                                 const int*, const int*, const V2<R>*, const double*,  \
                                 const Scn*, Scalars*, const int2*, Scalars*, int*,    \
                                 const double*, const int2*, int);                     \
+  template void launch_b_unpack<R>(int, cudaStream_t, ParticlesT<R>, const double*, int); \
   template void launch_b_move<R>(int, cudaStream_t, ParticlesT<R>, ParticlesT<R>,     \
                                  const int4*);
 DAMPM_INSTANTIATE(double)

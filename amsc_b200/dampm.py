@@ -306,9 +306,10 @@ class Solver:
         when the arrays are page-locked (pinned_array).  Call staged_wait()
         before reading them.  Returns the count of values each receives."""
         names = list(out)
+        count = self.num_particles
         for k in names:
             a = out[k]
-            if a.dtype != np.float64 or not a.flags.c_contiguous or a.size < self.num_particles:
+            if a.dtype != np.float64 or not a.flags.c_contiguous or a.size < count:
                 raise ValueError(f"{k}: needs a contiguous float64 array of >= np values")
         self._staged = [out[k] for k in names]  # kept alive until the copies end
         fields = (C.c_char_p * len(names))(*[k.encode() for k in names])
