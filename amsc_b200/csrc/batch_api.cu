@@ -63,18 +63,16 @@ struct dampm_batch {
   double* stage = nullptr;  // one field in reference order, for downloads
   unsigned long long* sortbuf = nullptr;  // 2 x capacity: crowded cells' order
   int *count = nullptr, *start = nullptr, *perm = nullptr;
-  int* skey = nullptr;  // the cell key of each sorted position
-  int *tile_sum = nullptr, *clist = nullptr, *clist_n = nullptr, *cbig = nullptr;
+  // of each sorted position: cell, storage slot and reference index before the
+  // order inside the cells
+  int *skey = nullptr, *sslot = nullptr, *sidx = nullptr;
+  int *tile_sum = nullptr, *cbig = nullptr;
   unsigned char* tflag = nullptr;  // the scan tiles of a pass (k_b_step_begin)
-  int* cmid = nullptr;  // cells with more than 16 particles
-  int* ustart = nullptr;
-  long long* upex = nullptr;
-  int4* uplan = nullptr;  // {cA, cB, heavy, 0}
-  int4* ulist = nullptr;
-  int* uorder = nullptr;  // the order P2G takes the units in
+  int4* ulist = nullptr;  // plain units, then heavy ones (USEG_cap each)
+  int* uslot = nullptr;   // their ledger slots
   int *strip_n = nullptr, *ucount = nullptr, *strip_scn = nullptr;
   double* led_part = nullptr;
-  int2 *scn_units = nullptr, *gblk = nullptr;
+  int2* gblk = nullptr;
   int4 *mblk = nullptr, *nmove = nullptr;
   Scn* scn = nullptr;
   Scalars *S = nullptr, *Sg = nullptr;
@@ -249,7 +247,7 @@ int read_scalars(dampm_batch* b) {
 }
 
 // One pass of every live scenario: kPassLaunches kernel launches.
-constexpr int kPassLaunches = 9;
+constexpr int kPassLaunches = 6;
 int enqueue_pass(dampm_batch* b) {
   cudaStream_t st = b->stream;
   const int nscn = int(b->scns.size());
@@ -266,37 +264,31 @@ int enqueue_pass(dampm_batch* b) {
   k_b_step_begin<<<1 + grid_blocks(ntiles, 256), 256, 0, st>>>(b->scn, b->S, nscn, b->Sg,
                                                                 b->tflag, ntiles);
   const Gate gate = kGateBegun;
-  k_scan_sums<<<ntiles, kScanThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->clist_n,
-                                               b->Sg, gate, 0, b->tflag);
-  k_scan_apply<<<ntiles, kScanThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->start,
-                                                b->clist, b->clist_n, b->Sg, gate, 0,
-                                                b->tflag);
-  k_scatter<<<gp, 256, 0, st>>>(key, slot, idx, b->start, b->perm, b->skey, b->sortbuf,
-                                b->Sg, gate);
-  k_segment_order<<<148 * 4, 256, 0, st>>>(b->start, b->clist, b->clist_n, b->perm,
-                                            b->sortbuf, b->cmid, b->cbig, b->Sg, gate);
-  k_segment_order_large<<<148, 1024, sort_big_smem_bytes(), st>>>(
-      b->start, b->cmid, b->cbig, b->clist_n, b->perm, b->sortbuf, b->P_cap, b->Sg, gate);
-  k_b_units<<<b->strips_tot, kPlanThreads, sizeof(int) * (b->strips_tot + 1), st>>>(
-      b->start, b->scn, b->S, nscn, b->strip_scn, b->Sg, b->units_per_cta * b->p2g_grid,
-      b->col_weight, b->ustart, b->upex, b->uplan, b->strip_n, b->ulist, b->uorder, b->ucount,
-      b->scn_units);
+  k_scan_apply<<<ntiles, kScanThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->start, b->cbig,
+                                                b->ucount, b->Sg, gate, 0, b->tflag);
+  const Binning n{key, slot, idx, b->sslot, b->sidx, b->skey};
+  k_scatter<<<gp, 256, 0, st>>>(n, b->start, b->tile_sum, ntiles, b->Sg, gate);
+  const UnitPlan u{b->units_per_cta * b->p2g_grid, int(b->USEG_cap), b->ulist, b->uslot,
+                   b->strip_n, b->ucount};
+  k_b_order_units<<<order_blocks(b->P_tot), kOrderThreads, order_smem_bytes(), st>>>(
+      CellOrder{n, b->start, b->cbig, b->ucount, b->perm, b->sortbuf, b->P_cap, b->count, 0},
+      u, b->scn, b->S, nscn, b->strip_scn, b->strips_tot, b->Sg, b->col_weight);
   if (b->precision == DAMPM_FP32)
     launch_b_p2g<float>(b->p2g_grid, st, b->p32[b->cur], b->perm, b->start,
                         static_cast<float2*>(b->vvL),
-                        b->led_part, b->scn, b->S, b->ulist, b->uorder, b->ucount, b->Sg);
+                        b->led_part, b->scn, b->S, u, b->Sg);
   else
     launch_b_p2g<double>(b->p2g_grid, st, b->p64[b->cur], b->perm, b->start,
                          static_cast<double2*>(b->vvL),
-                         b->led_part, b->scn, b->S, b->ulist, b->uorder, b->ucount, b->Sg);
+                         b->led_part, b->scn, b->S, u, b->Sg);
   if (b->precision == DAMPM_FP32)
     launch_b_g2p<float>(b->nblk, st, b->p32[b->cur], b->p32[nxt], b->perm, b->skey,
                         static_cast<const float2*>(b->vvL), b->Z[b->zcur], b->scn, b->S,
-                        b->gblk, b->Sg, b->count, b->led_part, b->scn_units, nscn);
+                        b->gblk, b->Sg, b->count, b->tile_sum, b->led_part, u, nscn);
   else
     launch_b_g2p<double>(b->nblk, st, b->p64[b->cur], b->p64[nxt], b->perm, b->skey,
                          static_cast<const double2*>(b->vvL), b->Z[b->zcur], b->scn, b->S,
-                         b->gblk, b->Sg, b->count, b->led_part, b->scn_units, nscn);
+                         b->gblk, b->Sg, b->count, b->tile_sum, b->led_part, u, nscn);
   b->cur = nxt;
   b->launches += kPassLaunches;
   cudaError_t e = cudaGetLastError();
@@ -374,7 +366,7 @@ int upload_scenario(dampm_batch* b, const Scn& d, int pos, long long np, long lo
   launch_init_particles<R>(grid_blocks(np, 256), 256, st, p, Zs, Zs, Zs, d.G, d.P,
                            b->S + pos, int(np), d.c_off);
   // the new keys join the counts the last pass left for the next sort
-  k_count_n<<<grid_blocks(np, 256), 256, 0, st>>>(p.key, b->count, p.slot, int(np));
+  k_count_n<<<grid_blocks(np, 256), 256, 0, st>>>(p.key, b->count, b->tile_sum, p.slot, int(np));
   launch_prep<R>(grid_blocks(np, 256), 256, st, p, Zs, d.G, d.P, b->S + pos, 0);
   b->launches += 3;
   BCK(cudaGetLastError());
@@ -473,27 +465,22 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   // cells of all scenarios: fewer than their nodes
   rc = rc ? rc : balloc(b, &b->count, nn + 4);
   rc = rc ? rc : balloc(b, &b->start, nn + 1);
-  rc = rc ? rc : balloc(b, &b->clist, nn + 4);
-  rc = rc ? rc : balloc(b, &b->clist_n, 4);
   rc = rc ? rc : balloc(b, &b->tile_sum, nn / kScanTile + 2);
   rc = rc ? rc : balloc(b, &b->tflag, nn / kScanTile + 2);
   rc = rc ? rc : balloc(b, &b->perm, pc);
   rc = rc ? rc : balloc(b, &b->skey, pc);
+  rc = rc ? rc : balloc(b, &b->sslot, pc);
+  rc = rc ? rc : balloc(b, &b->sidx, pc);
   rc = rc ? rc : balloc(b, &b->cbig, pc / 256 + 4);
-  rc = rc ? rc : balloc(b, &b->cmid, pc / 17 + 4);
   const size_t us = size_t(b->USEG_cap);
-  rc = rc ? rc : balloc(b, &b->ustart, us);
-  rc = rc ? rc : balloc(b, &b->upex, us);
-  rc = rc ? rc : balloc(b, &b->uplan, us);
-  rc = rc ? rc : balloc(b, &b->ulist, us);
-  rc = rc ? rc : balloc(b, &b->uorder, us);
+  rc = rc ? rc : balloc(b, &b->ulist, 2 * us);
+  rc = rc ? rc : balloc(b, &b->uslot, 2 * us);
   rc = rc ? rc : balloc(b, &b->led_part, us * 6);
   rc = rc ? rc : balloc(b, &b->strip_n, size_t(b->STRIP_cap));
   rc = rc ? rc : balloc(b, &b->strip_scn, size_t(b->STRIP_cap));
   rc = rc ? rc : balloc(b, &b->ucount, 8);
   if (rc == DAMPM_OK && cudaMemsetAsync(b->ucount, 0, sizeof(int) * 8, b->stream) != cudaSuccess)
     rc = bfail(b, DAMPM_ERR_CUDA, "cudaMemsetAsync failed");
-  rc = rc ? rc : balloc(b, &b->scn_units, size_t(scenario_cap));
   rc = rc ? rc : balloc(b, &b->gblk, size_t(b->B_cap));
   rc = rc ? rc : balloc(b, &b->mblk, size_t(b->B_cap));
   rc = rc ? rc : balloc(b, &b->nmove, nn / kG2PThreads + size_t(scenario_cap) + 1);
@@ -532,6 +519,7 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   }
   if (rc == DAMPM_OK) {
     cudaMemsetAsync(b->count, 0, sizeof(int) * (nn + 4), b->stream);
+    cudaMemsetAsync(b->tile_sum, 0, sizeof(int) * (nn / kScanTile + 2), b->stream);
     cudaMemsetAsync(b->vvL, 0, 2 * rsz * nn, b->stream);
     cudaMemsetAsync(b->S, 0, sizeof(Scalars) * size_t(scenario_cap), b->stream);
     cudaMemsetAsync(b->Sg, 0, sizeof(Scalars), b->stream);
@@ -698,6 +686,7 @@ int dampm_batch_compact(dampm_batch* b) {
   // beyond the new total may hold counts of removed scenarios, which a later
   // scenario's cells would otherwise inherit)
   BCK(cudaMemsetAsync(b->count, 0, sizeof(int) * size_t(b->N_cap + 4), b->stream));
+  BCK(cudaMemsetAsync(b->tile_sum, 0, sizeof(int) * size_t(b->N_cap / kScanTile + 2), b->stream));
   if (!mv.empty()) {
     BCK(cudaMemcpyAsync(b->mblk, mv.data(), sizeof(int4) * mv.size(),
                         cudaMemcpyHostToDevice, b->stream));
@@ -708,7 +697,7 @@ int dampm_batch_compact(dampm_batch* b) {
                             b->mblk);
     const int* key = b->precision == DAMPM_FP32 ? b->p32[nxt].key : b->p64[nxt].key;
     int* slot = b->precision == DAMPM_FP32 ? b->p32[nxt].slot : b->p64[nxt].slot;
-    k_count_n<<<grid_blocks(P, 256), 256, 0, b->stream>>>(key, b->count, slot, int(P));
+    k_count_n<<<grid_blocks(P, 256), 256, 0, b->stream>>>(key, b->count, b->tile_sum, slot, int(P));
   }
   if (!nm.empty()) {
     BCK(cudaMemcpyAsync(b->nmove, nm.data(), sizeof(int4) * nm.size(),

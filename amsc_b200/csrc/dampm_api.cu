@@ -35,20 +35,18 @@ struct dampm_ctx {
   Nodes nodes{};
   double *Z = nullptr, *dZdx = nullptr, *dZdy = nullptr;
   int *count = nullptr, *start = nullptr, *perm = nullptr, *tile_sum = nullptr;
-  int* skey = nullptr;  // the cell of each sorted position
+  // of each sorted position: cell, storage slot and reference index before the
+  // order inside the cells
+  int *skey = nullptr, *sslot = nullptr, *sidx = nullptr;
   unsigned long long* sortbuf = nullptr;  // 2 x capacity: crowded cells' order
   int ntiles = 0;
   double* led_part = nullptr;
   int n_led = 0;
   int strips = 0, useg = 0;  // strips; unit slots per strip (ncols + 1)
-  int *ustart = nullptr, *strip_n = nullptr, *ucount = nullptr;
-  long long* upex = nullptr;
-  int4* uplan = nullptr;  // {cA, cB, heavy, 0}
-  int4* ulist = nullptr;
-  int* uorder = nullptr;  // the order P2G takes the units in
-  int *clist = nullptr, *clist_n = nullptr;  // cells with >= 2 particles
+  int *strip_n = nullptr, *ucount = nullptr;
+  int4* ulist = nullptr;  // plain units, then heavy ones (n_led each)
+  int* uslot = nullptr;   // their ledger slots
   int* cbig = nullptr;  // cells with more than 256 particles (capacity / 256)
-  int* cmid = nullptr;  // cells with more than 16 particles (capacity / 17)
   double* ledger_log = nullptr;  // kLedgerLog rows {t, err_mass, err_mom}
   int p2g_grid = 0;
   Scalars* S = nullptr;
@@ -230,7 +228,7 @@ int alloc_particles(dampm_ctx* ctx, long long cap) {
     if (rc) return rc;
     CK(cudaMemsetAsync(*q, 0, cap * sizeof(double), ctx->stream));
   }
-  int** fi[] = {&p.label, &p.level, &ctx->perm, &ctx->skey};
+  int** fi[] = {&p.label, &p.level, &ctx->perm, &ctx->skey, &ctx->sslot, &ctx->sidx};
   for (int** q : fi) {
     int rc = dalloc(ctx, q, cap);
     if (rc) return rc;
@@ -239,8 +237,6 @@ int alloc_particles(dampm_ctx* ctx, long long cap) {
     int rc = dalloc(ctx, &ctx->sortbuf, size_t(2 * cap));
     if (rc) return rc;
     rc = dalloc(ctx, &ctx->cbig, size_t(cap / 256 + 4));
-    if (rc) return rc;
-    rc = dalloc(ctx, &ctx->cmid, size_t(cap / 17 + 4));
     if (rc) return rc;
   }
   share_fixed(ctx);
@@ -252,28 +248,42 @@ int alloc_particles(dampm_ctx* ctx, long long cap) {
   return DAMPM_OK;
 }
 
+// A grid that one launch scans and scatters (k_scan_scatter); the others' tile
+// totals are counted with the keys.
+bool small_grid(const dampm_ctx* ctx) { return ctx->nc <= kSmallCells; }
+int* tile_totals(const dampm_ctx* ctx) { return small_grid(ctx) ? nullptr : ctx->tile_sum; }
+
+UnitPlan unit_plan(const dampm_ctx* ctx) {
+  return UnitPlan{kUnitsPerCta * ctx->p2g_grid, ctx->n_led, ctx->ulist, ctx->uslot,
+                  ctx->strip_n, ctx->ucount};
+}
+
 // Enqueues the binning of the current particles (SORT), whose slots and
 // counts are in hand (from G2P, or from k_count after an upload, a state
 // upload or a merge/split).  begun: the step has begun (or the call is no
-// step: a standalone merge/split).
-void enqueue_sort(dampm_ctx* ctx, int begun) {
+// step: a standalone merge/split).  units: and P2G's work list, with the end of
+// the step before and the begin of this one.
+void enqueue_sort(dampm_ctx* ctx, int begun, bool units) {
   const Gate gate = make_gate(ctx->P, begun);
-  const int gp = grid_for(ctx->cap, 256);
-  k_scan_sums<<<ctx->ntiles, kScanThreads, 0, ctx->stream>>>(ctx->count, ctx->nc,
-                                                             ctx->tile_sum, ctx->clist_n,
-                                                             ctx->S, gate, 1, nullptr);
-  k_scan_apply<<<ctx->ntiles, kScanThreads, 0, ctx->stream>>>(
-      ctx->count, ctx->nc, ctx->tile_sum, ctx->start, ctx->clist, ctx->clist_n, ctx->S, gate, 1,
-      nullptr);
-  k_scatter<<<gp, 256, 0, ctx->stream>>>(ctx->p.key, ctx->p.slot, ctx->p.idx, ctx->start,
-                                         ctx->perm, ctx->skey, ctx->sortbuf, ctx->S, gate);
-  k_segment_order<<<148 * 4, 256, 0, ctx->stream>>>(ctx->start, ctx->clist, ctx->clist_n,
-                                                   ctx->perm, ctx->sortbuf, ctx->cmid,
-                                                   ctx->cbig, ctx->S, gate);
-  k_segment_order_large<<<148, 1024, sort_big_smem_bytes(), ctx->stream>>>(
-      ctx->start, ctx->cmid, ctx->cbig, ctx->clist_n, ctx->perm, ctx->sortbuf, ctx->cap,
-      ctx->S, gate);
-  ctx->launches += 5;
+  const int strips = units ? ctx->strips : 0;
+  const bool small = small_grid(ctx);
+  const Binning n{ctx->p.key, ctx->p.slot, ctx->p.idx, ctx->sslot, ctx->sidx, ctx->skey};
+  if (small) {
+    k_scan_scatter<<<order_blocks(ctx->cap), kScanThreads, sizeof(int) * size_t(ctx->nc),
+                     ctx->stream>>>(ctx->count, ctx->nc, ctx->start, ctx->cbig, ctx->ucount, n,
+                                    ctx->S, gate);
+  } else {
+    k_scan_apply<<<ctx->ntiles, kScanThreads, 0, ctx->stream>>>(
+        ctx->count, ctx->nc, ctx->tile_sum, ctx->start, ctx->cbig, ctx->ucount, ctx->S, gate, 1,
+        nullptr);
+    k_scatter<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(n, ctx->start, ctx->tile_sum,
+                                                                ctx->ntiles, ctx->S, gate);
+  }
+  k_order_units<<<order_blocks(ctx->cap), kOrderThreads, order_smem_bytes(), ctx->stream>>>(
+      CellOrder{n, ctx->start, ctx->cbig, ctx->ucount, ctx->perm, ctx->sortbuf, ctx->cap,
+                ctx->count, small ? ctx->nc : 0},
+      unit_plan(ctx), ctx->G, ctx->P, ctx->S, strips, ctx->useg, gate);
+  ctx->launches += small ? 2 : 3;
 }
 
 // One pass of the loop body in two halves: sort, units (which end the step
@@ -288,24 +298,20 @@ int enqueue_front(dampm_ctx* ctx) {
   if (ms_due) {  // on the binning of the particles as they lie in storage
     k_step_begin<<<1, 1, 0, ctx->stream>>>(ctx->S, ctx->G, ctx->P);
     ctx->launches += 1;
-    enqueue_sort(ctx, 1);
+    enqueue_sort(ctx, 1, false);
     ctx->launches += ms_enqueue(ctx->msb, ctx->p, ctx->q, ctx->start, ctx->perm, ctx->nc,
                                 ctx->G, ctx->P, ctx->Z, ctx->ms, ctx->S, ctx->cap,
                                 ctx->stream, /*use_step_dt=*/1, 0.0, ctx->ms_variant,
                                 ctx->ms_stretch);
     swap_moving(ctx->p, ctx->q);
     k_keys<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(ctx->p, ctx->G, ctx->S, 0);
-    k_count<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(ctx->p.key, ctx->count,
-                                                             ctx->p.slot, ctx->S);
+    k_count<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(
+        ctx->p.key, ctx->count, tile_totals(ctx), ctx->p.slot, ctx->S);
     ctx->launches += 2;
   }
   ev_mark(ctx, 0);
-  enqueue_sort(ctx, ms_due);
+  enqueue_sort(ctx, ms_due, true);
   ev_mark(ctx, 1);
-  k_units<<<ctx->strips, kPlanThreads, sizeof(int) * (ctx->strips + 1), ctx->stream>>>(
-      ctx->start, ctx->G, ctx->P, ctx->S, kUnitsPerCta * ctx->p2g_grid, ctx->useg,
-      ctx->ustart, ctx->upex, ctx->uplan, ctx->strip_n, ctx->ulist, ctx->uorder, ctx->ucount,
-      make_gate(ctx->P, ms_due));
   if (ctx->record) {
     Nodes& n = ctx->nodes;
     double* nf[] = {n.Mv,  n.mvx,  n.mvy,   n.avx,   n.avy,  n.vvx, n.vvy,
@@ -315,9 +321,8 @@ int enqueue_front(dampm_ctx* ctx) {
     cudaMemsetAsync(n.vvL, 0, sizeof(double2) * ctx->nn, ctx->stream);
   }
   launch_p2g(ctx->p2g_grid, ctx->stream, ctx->p, ctx->perm, ctx->start, ctx->nodes,
-             ctx->led_part, ctx->G, ctx->P, ctx->S, ctx->record ? 1 : 0, ctx->ulist, ctx->uorder,
-             ctx->ucount);
-  ctx->launches += 2;
+             ctx->led_part, ctx->G, ctx->P, ctx->S, ctx->record ? 1 : 0, unit_plan(ctx));
+  ctx->launches += 1;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(ctx, DAMPM_ERR_CUDA, cudaGetErrorString(e));
   return DAMPM_OK;
@@ -331,8 +336,10 @@ int enqueue_back(dampm_ctx* ctx) {
                          ((it_next + 1) % ctx->ms.call_interval) == 0;
   ev_mark(ctx, 2);
   launch_g2p(grid_for(ctx->cap, kG2PThreads), ctx->stream, ctx->p, ctx->q, ctx->perm,
-             ctx->skey, ctx->nodes, ctx->Z, ctx->G, ctx->P, ctx->S, ctx->count, ctx->leave,
-             ctx->led_part, ctx->ucount, ctx->ledger_log, ctx->record ? 1 : 0,
+             ctx->skey, ctx->nodes, ctx->Z, ctx->G, ctx->P, ctx->S, ctx->count,
+             tile_totals(ctx), ctx->leave, ctx->led_part, unit_plan(ctx), ctx->strips, ctx->useg,
+             ctx->ledger_log,
+             ctx->record ? 1 : 0,
              (grad_next || ctx->record) ? 1 : 0);
   if (ctx->record) {
     k_hv<<<grid_for(ctx->nn, 256), 256, 0, ctx->stream>>>(ctx->q, ctx->start,
@@ -690,8 +697,6 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   rc = rc ? rc : dalloc(ctx, &ctx->nodes.vvL, nn);
   ctx->ntiles = (ctx->nc + kScanTile - 1) / kScanTile;
   rc = rc ? rc : dalloc(ctx, &ctx->count, size_t(ctx->nc) + 4);
-  rc = rc ? rc : dalloc(ctx, &ctx->clist, size_t(ctx->nc) + 4);
-  rc = rc ? rc : dalloc(ctx, &ctx->clist_n, 4);
   rc = rc ? rc : dalloc(ctx, &ctx->start, size_t(ctx->nc) + 1);
   rc = rc ? rc : dalloc(ctx, &ctx->tile_sum, size_t(ctx->ntiles) + 1);
   ctx->strips = (grid->Ney + 1 + kTR - 1) / kTR;
@@ -700,11 +705,8 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   if (ctx->strips > kMaxStrips)
     rc = fail(ctx, DAMPM_ERR_ARG, "grid has too many rows for the P2G unit planner");
   rc = rc ? rc : dalloc(ctx, &ctx->led_part, size_t(ctx->n_led) * 6);
-  rc = rc ? rc : dalloc(ctx, &ctx->ustart, size_t(ctx->n_led));
-  rc = rc ? rc : dalloc(ctx, &ctx->upex, size_t(ctx->n_led));
-  rc = rc ? rc : dalloc(ctx, &ctx->uplan, size_t(ctx->n_led));
-  rc = rc ? rc : dalloc(ctx, &ctx->ulist, size_t(ctx->n_led));
-  rc = rc ? rc : dalloc(ctx, &ctx->uorder, size_t(ctx->n_led));
+  rc = rc ? rc : dalloc(ctx, &ctx->ulist, size_t(ctx->n_led) * 2);
+  rc = rc ? rc : dalloc(ctx, &ctx->uslot, size_t(ctx->n_led) * 2);
   rc = rc ? rc : dalloc(ctx, &ctx->strip_n, size_t(ctx->strips));
   rc = rc ? rc : dalloc(ctx, &ctx->ucount, 8);
   rc = rc ? rc : dalloc(ctx, &ctx->ledger_log, size_t(kLedgerLog) * 3);
@@ -714,6 +716,7 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   }
   if (rc == DAMPM_OK) {
     cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream);
+    cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * size_t(ctx->ntiles), ctx->stream);
     cudaMemsetAsync(ctx->ucount, 0, sizeof(int) * 8, ctx->stream);
     cudaMemsetAsync(ctx->nodes.vvL, 0, sizeof(double2) * nn, ctx->stream);
     cudaMemsetAsync(ctx->S, 0, sizeof(Scalars), ctx->stream);
@@ -803,12 +806,13 @@ int dampm_upload_particles(dampm_ctx* ctx, long long np, const double* x,
   CK(cudaMemcpyAsync(ctx->S, ctx->Sh, sizeof(Scalars), cudaMemcpyHostToDevice,
                      ctx->stream));
   CK(cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream));
+  CK(cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * size_t(ctx->ntiles), ctx->stream));
   if (np > 0) {
     // the slots hold the particles in DATA order (idx = slot)
     launch_init_particles<double>(grid_for(np, 256), 256, ctx->stream, p, ctx->Z,
                                   ctx->dZdx, ctx->dZdy, ctx->G, ctx->P, ctx->S, int(np), 0);
-    k_count_n<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p.key, ctx->count, p.slot,
-                                                           int(np));
+    k_count_n<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p.key, ctx->count, tile_totals(ctx),
+                                                           p.slot, int(np));
     launch_prep<double>(grid_for(np, 256), 256, ctx->stream, p, ctx->Z, ctx->G, ctx->P,
                         ctx->S, 0);
     CK(cudaGetLastError());
@@ -968,14 +972,14 @@ int dampm_merge_split(dampm_ctx* ctx, double dt, long long counts[4]) {
   CK(cudaMemcpyAsync(&S->active, &ctx->Sh->active, sizeof(int),
                      cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  enqueue_sort(ctx, 1);
+  enqueue_sort(ctx, 1, false);
   ms_enqueue(ctx->msb, ctx->p, ctx->q, ctx->start, ctx->perm, ctx->nc, ctx->G, ctx->P,
              ctx->Z, ctx->ms, ctx->S, ctx->cap, ctx->stream, /*use_step_dt=*/0, dt,
              ctx->ms_variant, ctx->ms_stretch);
   swap_moving(ctx->p, ctx->q);
   k_keys<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(ctx->p, ctx->G, ctx->S, 0);
-  k_count<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(ctx->p.key, ctx->count,
-                                                           ctx->p.slot, ctx->S);
+  k_count<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(
+        ctx->p.key, ctx->count, tile_totals(ctx), ctx->p.slot, ctx->S);
   CK(cudaGetLastError());
   rc = sync_status(ctx);
   if (rc) return rc;
@@ -1107,8 +1111,10 @@ int dampm_set_state(dampm_ctx* ctx, long long np, const double* const* fields,
                      ctx->stream));
   // the slots now hold the particles in reference order
   CK(cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream));
+  CK(cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * size_t(ctx->ntiles), ctx->stream));
   k_keys<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p, ctx->G, ctx->S, 1);
-  k_count_n<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p.key, ctx->count, p.slot, int(np));
+  k_count_n<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p.key, ctx->count, tile_totals(ctx),
+                                                           p.slot, int(np));
   k_reduce_state<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p, ctx->S);
   launch_prep<double>(grid_for(np, 256), 256, ctx->stream, p, ctx->Z, ctx->G, ctx->P,
                       ctx->S, fresh ? 0 : 1);
@@ -1372,6 +1378,7 @@ int dampm_slab_import(dampm_ctx* ctx, const double* buf, long long n, int ghosts
     k_slab_check<<<grid_for(n, 256), 256, 0, ctx->stream>>>(ctx->p.key + base, int(n), lo, hi,
                                                             ctx->grid.Ney, ctx->S);
     k_count_n<<<grid_for(n, 256), 256, 0, ctx->stream>>>(ctx->p.key + base, ctx->count,
+                                                         tile_totals(ctx),
                                                          ctx->p.slot + base, int(n));
   }
   k_slab_scalars<<<1, 1, 0, ctx->stream>>>(ctx->S, int(base + n), ghosts ? int(n) : 0,

@@ -22,7 +22,7 @@ constexpr int kTR = 30;
 constexpr int kUnitsPerCta = DAMPM_UNITS_PER_CTA;
 constexpr int kUnitMinWeight = 1024;
 constexpr int kColWeight = DAMPM_COL_WEIGHT;
-constexpr int kPlanThreads = 1024;
+constexpr int kOrderThreads = 1024;
 constexpr int kMaxStrips = 8192;  // strip offsets of the unit list in shared memory
 constexpr int kP2GThreads = 128;
 #ifndef DAMPM_P2G_CAP
@@ -44,6 +44,7 @@ constexpr int kG2PThreads = 256;
 constexpr int kG2PMinBlocks = DAMPM_G2P_MIN_BLOCKS;
 constexpr int kScanTile = 4096;
 constexpr int kScanThreads = 1024;
+constexpr int kSmallCells = 4 * kScanTile;  // grids that k_scan_scatter takes
 
 // Two values of R side by side (one 16-byte load in FP64, 8 in FP32).
 template <class R>
@@ -151,42 +152,69 @@ void launch_prep(int grid, int block, cudaStream_t st, ParticlesT<R> p, const do
 // merge/split; a step's G2P counts the keys it makes), the scan of the
 // counts over the key range (ranged != 0; else over all n), the scatter into
 // perm, and the order by reference index inside each cell
-__global__ void k_count(const int* key, int* count, int* slot,
-                        const Scalars* S);
-__global__ void k_count_n(const int* key, int* count, int* slot, int n);
-// tflag (may be null): scan only the flagged tiles (k_b_step_begin)
-__global__ void k_scan_sums(const int* count, int n, int* tile_sum, int* list_n,
-                            const Scalars* S, Gate gate, int ranged,
-                            const unsigned char* tflag);
-__global__ void k_scan_apply(int* count, int n, const int* tile_sum,
-                             int* start, int* list, int* list_n,
-                             const Scalars* S, Gate gate, int ranged,
-                            const unsigned char* tflag);
-// pk: 2 x capacity entries; the scatter writes the first half, which the
-// per-cell ordering sorts (the crowded cells use both halves)
-__global__ void k_scatter(const int* key, const int* slot, const int* idx, const int* start,
-                          int* perm, int* skey, unsigned long long* pk, Scalars* S, Gate gate);
-__global__ void k_segment_order(const int* start, const int* list, int* list_n,
-                                int* perm, const unsigned long long* pk, int* mid,
-                                int* big, const Scalars* S, Gate gate);
-__global__ void k_segment_order_large(const int* start, const int* mid, const int* big,
-                                      const int* list_n, int* perm, unsigned long long* pk,
-                                      long long cap, const Scalars* S, Gate gate);
-// dynamic shared memory of k_segment_order_large; setup_sort sets its limit
-// (0 on failure)
-size_t sort_big_smem_bytes();
+__global__ void k_count(const int* key, int* count, int* tile_sum, int* slot, const Scalars* S);
+__global__ void k_count_n(const int* key, int* count, int* tile_sum, int* slot, int n);
+// the tile totals of counts that count_key did not make
+__global__ void k_scan_sums(const int* count, int n, int* tile_sum, const Scalars* S);
+// tflag (may be null): scan only the flagged tiles (k_b_step_begin); big (its size
+// in list_n[0]; may be null: a scan alone): the crowded cells
+__global__ void k_scan_apply(int* count, int n, const int* tile_sum, int* start, int* big,
+                             int* list_n, const Scalars* S, Gate gate, int ranged,
+                             const unsigned char* tflag);
+// The binning of the particles as they lie in storage, and at each sorted
+// position the storage slot, the reference index and the cell key.
+struct Binning {
+  const int *key, *slot, *idx;
+  int *sslot, *sidx, *skey;
+};
+__global__ void k_scatter(Binning n, const int* start, int* tile_sum, int ntiles, Scalars* S,
+                          Gate gate);
+// scan and scatter in one, for up to kSmallCells cells (dynamic shared memory:
+// ncell ints); leaves the counts to be zeroed by the ordering
+__global__ void k_scan_scatter(const int* count, int ncell, int* start, int* big, int* list_n,
+                               Binning n, Scalars* S, Gate gate);
+// What it takes to order the particles inside the cells.
+struct CellOrder {
+  Binning n;
+  const int *start, *big;
+  int *list_n, *perm;
+  unsigned long long* pk;  // 2 x cap entries, for the crowded cells
+  long long cap;
+  int* count;  // counts to be zeroed (n_count of them; 0: they are zero)
+  int n_count;
+};
+// The counters of a pass: the crowded cells (k_order_units, which uses them,
+// empties the list), P2G's units (plain, heavy) and its work cursor (set to zero
+// by G2P), the blocks of k_order_units that are done.
+constexpr int kUnitsPlain = 1, kUnitsHeavy = 2, kUnitCursor = 3, kUnitCounts = 3, kOrderDone = 4;
+// P2G's unit list -- the plain units from 0, the heavy ones (which P2G takes
+// first) from cap -- with each unit's ledger slot.
+struct UnitPlan {
+  int target_units, cap;
+  int4* ulist;
+  int* uslot;
+  int* strip_n;  // units of each strip
+  int* ucount;   // the counters
+};
+// orders the particles inside the cells and, with strips > 0, makes the unit
+// list (seg: unit slots per strip) and ends the step before and begins this
+// one unless it has begun.  order_smem_bytes(): its dynamic shared memory;
+// setup_sort sets the sort kernels' limits (0 on failure)
+__global__ void k_order_units(CellOrder o, UnitPlan u, Geom G, Phys P, Scalars* S, int strips,
+                              int seg, Gate gate);
+size_t order_smem_bytes();
 int setup_sort();
-// the unit list and uorder, the order P2G hands the units out in (heavy units
-// first); ends the step before and begins this one unless it has begun
-__global__ void k_units(const int* cstart, Geom G, Phys P, Scalars* S, int target_units,
-                        int seg, int* ustart, long long* upex, int4* plan, int* strip_n,
-                        int4* ulist, int* uorder, int* ucount, Gate gate);
+// blocks of 1024 threads for np particles, one per SM at most
+inline int order_blocks(long long np) {
+  const long long b = (np + kOrderThreads - 1) / kOrderThreads;
+  return int(b < 1 ? 1 : b > 148 ? 148 : b);
+}
 // P2G of the single-scenario step (k_p2g specialised for recorded outputs);
 // setup_p2g sets its shared-memory attributes and returns the resident CTAs
 // per SM (0 on failure)
 void launch_p2g(int grid, cudaStream_t st, Particles p, const int* perm, const int* cstart,
                 Nodes nodes, double* led_part, Geom G, Phys P, const Scalars* S, int record,
-                const int4* ulist, const int* uorder, const int* ucount);
+                const UnitPlan& u);
 int setup_p2g();
 constexpr int kLedgerLog = 1024;  // rows of the per-step ledger log
 // G2P of the single-scenario step (k_g2p_t specialised for the two flags):
@@ -194,8 +222,8 @@ constexpr int kLedgerLog = 1024;  // rows of the per-step ledger log
 // the next binning's keys and sums the ledger; the step's end is left pending
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
-                int* count, int* leave, const double* led_part, const int* ucount, double* log,
-                int record, int want_grad);
+                int* count, int* tile_sum, int* leave, const double* led_part, const UnitPlan& u,
+                int strips, int seg, double* log, int record, int want_grad);
 
 // ---- batches of independent scenarios --------------------------------------
 // One scenario of a batch: its geometry, physics and place in the packed
@@ -211,19 +239,16 @@ struct Scn {
   int live;                // 0 once removed
 };
 
-__global__ void k_b_units(const int* cstart, const Scn* scn, Scalars* S, int nscn,
-                          const int* strip_scn, const Scalars* Sg, int target_units,
-                          int col_weight, int* ustart, long long* upex, int4* plan,
-                          int* strip_n, int4* ulist, int* uorder, int* ucount,
-                          int2* scn_units);
+__global__ void k_b_order_units(CellOrder o, UnitPlan u, const Scn* scn, Scalars* S, int nscn,
+                                const int* strip_scn, int strips, const Scalars* Sg,
+                                int col_weight);
 __global__ void k_b_step_begin(const Scn* scn, Scalars* S, int nscn, Scalars* Sg,
                                unsigned char* tflag, int ntiles);
 __global__ void k_b_step_end(const Scn* scn, Scalars* S, int nscn);
 template <class R>
 void launch_b_p2g(int grid, cudaStream_t st, ParticlesT<R> p, const int* perm,
                   const int* cstart, V2<R>* vvL, double* led_part, const Scn* scn,
-                  Scalars* S, const int4* ulist, const int* uorder, const int* ucount,
-                  const Scalars* Sg);
+                  Scalars* S, const UnitPlan& u, const Scalars* Sg);
 // sets the batched P2G kernel's shared-memory attributes; returns the
 // resident CTAs per SM (0 on failure)
 template <class R>
@@ -232,7 +257,7 @@ template <class R>
 void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nxt,
                   const int* perm, const int* skey, const V2<R>* vvL, const double* Z,
                   const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count,
-                  const double* led_part, const int2* scn_units, int nscn);
+                  int* tile_sum, const double* led_part, const UnitPlan& u, int nscn);
 template <class R>
 void launch_b_move(int grid, cudaStream_t st, ParticlesT<R> dst, ParticlesT<R> src,
                    const int4* mblk);

@@ -1,10 +1,10 @@
 // step_kernels.cu -- the FP64 MPM time step on sm_100a.
 //
 // One pass of the loop body of main/optim_par.cpp:281-668 is
-//   SORT        : count -> scan -> scatter -> per-cell order  (a1)
-//   UNITS       : P2G's work list; its last block ends the step before (t += dt)
-//                 and begins this one -- dt (fixed or CFL from the previous
-//                 G2P's max-reductions), it++
+//   SORT        : scan -> scatter -> per-cell order (G2P counted the keys; a1);
+//                 the last kernel also cuts P2G's work list, ends the step before
+//                 (t += dt) and begins this one -- dt (fixed or CFL from the
+//                 previous G2P's max-reductions), it++
 //   P2G+NODAL   : per-node sequential chains over the sorted particles of the
 //                 node's 4 cells, nodal momentum/velocity/BC  (a2-a7, a10, a14)
 //   G2P         : velocity, advection, gradients, height, Bingham stress,
@@ -71,6 +71,7 @@ __device__ __forceinline__ void step_begin_one(Scalars* S, const Geom& G,
 // atomics) is visible to the last block past L1.
 __device__ __forceinline__ bool last_block(int* arrived, int n) {
   __shared__ int last;
+  __syncthreads();  // every thread has done its part (and left a call before)
   if (threadIdx.x == 0) {
     __threadfence();
     last = atomicAdd(arrived, 1) == n - 1;
@@ -269,41 +270,76 @@ __global__ void k_prep(ParticlesT<R> p, const double* __restrict__ Z, Geom G,
 // SORT: stable counting sort by cell, (cell, particle index) order
 // (init_particle_mesh + cell_start/cell_ptcls, main/gpu_offload.cpp:243-249)
 // ---------------------------------------------------------------------------
-// Particle i takes slot[i] among its cell's particles: one atomic per cell
-// and warp (the lanes of a warp that share a cell take consecutive slots in
-// index order).
-__global__ void k_count(const int* __restrict__ key, int* __restrict__ count,
-                        int* __restrict__ slot, const Scalars* S) {
-  if (!S->active) return;
-  const int np = S->np;
+// The counting sort's first step, done where the keys are made (G2P; k_count
+// after an upload or a merge/split): a particle of cell k takes a slot among its
+// cell's particles, one atomic per cell and warp (the lanes that share a cell
+// take consecutive slots), and its tile of kScanTile cells counts it, mostly
+// with one more atomic per warp, whose result nobody waits for: the scan needs
+// no pass of its own over the counts for the tile totals (a launch of 7 us at 4M
+// particles, 3 at 0.25M, 8 for 96 scenarios).
+// tile_sum may be null (a grid that k_scan_scatter takes).  All 32 lanes call
+// it; ok == false lanes take part without a particle.
+__device__ __forceinline__ void count_key(int k, bool ok, int* __restrict__ count,
+                                          int* __restrict__ tile_sum,
+                                          int* __restrict__ slot_out) {
+  const int lane = threadIdx.x & 31;
+  const int kk = ok ? k : -1;
+  const unsigned peers = __match_any_sync(0xffffffffu, kk);
+  const int leader = __ffs(peers) - 1;
+  int base = 0;
+  if (ok && lane == leader) base = atomicAdd(&count[kk], __popc(peers));
+  if (tile_sum) {
+    const unsigned who = __ballot_sync(0xffffffffu, ok);
+    const int first = __ffs(who) - 1, t = kk / kScanTile;
+    const int t0 = __shfl_sync(0xffffffffu, t, first & 31);
+    if (__all_sync(0xffffffffu, !ok || t == t0)) {
+      if (lane == first) atomicAdd(&tile_sum[t], __popc(who));
+    } else if (ok && lane == leader) {
+      atomicAdd(&tile_sum[t], __popc(peers));
+    }
+  }
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (ok) *slot_out = base + __popc(peers & ((1u << lane) - 1u));
+}
+
+// Slots and counts of the keys [0, n).
+__device__ __forceinline__ void count_keys(const int* __restrict__ key, int* __restrict__ count,
+                                           int* __restrict__ tile_sum, int* __restrict__ slot,
+                                           int n) {
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * blockDim.x;
-  for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < np; i0 += stride) {
+  for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
     const int i = i0 + lane;
-    const bool ok = i < np;
-    const int k = ok ? key[i] : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, k);
-    const int leader = __ffs(peers) - 1;
-    int base = 0;
-    if (ok && lane == leader) base = atomicAdd(&count[k], __popc(peers));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (ok) slot[i] = base + __popc(peers & ((1u << lane) - 1u));
+    const bool ok = i < n;
+    count_key(ok ? key[i] : -1, ok, count, tile_sum, slot + (ok ? i : 0));
   }
 }
+__global__ void k_count(const int* __restrict__ key, int* __restrict__ count,
+                        int* __restrict__ tile_sum, int* __restrict__ slot, const Scalars* S) {
+  if (S->active) count_keys(key, count, tile_sum, slot, S->np);
+}
+__global__ void k_count_n(const int* __restrict__ key, int* __restrict__ count,
+                          int* __restrict__ tile_sum, int* __restrict__ slot, int n) {
+  count_keys(key, count, tile_sum, slot, n);
+}
+
+// Cells of more than kCrowded particles are ordered by a block each (see
+// order_crowded).
+constexpr int kCrowded = 256;
+constexpr int kBigRun = 8192;  // entries of a sorted run (two buffers: 128 KB of shared memory)
+constexpr unsigned long long kNoEntry = ~0ull;
 
 // Exclusive scan of count[0..n) into start[0..n], restricted to the tiles of
 // kScanTile = 4 x kScanThreads cells (each thread one int4) that meet the key
 // range [L, H] = krange U knext: the keys the starts describe and the keys
 // G2P produced since.  Outside that range no cell's count changed and every
 // start is either 0 (below every key) or np (above), as before, so the old
-// values stand.  k_scan_sums writes the tile totals; k_scan_apply adds, per
-// tile, the totals of the preceding tiles in the range to a block scan.
+// values stand.  k_scan_apply adds, per tile, the totals of the preceding
+// tiles in the range (count_key's, or k_scan_sums') to a block scan.
 // count is zeroed on the way (ready for the next step's atomics).  With
 // tile flags (batches) only the flagged tiles are scanned: the others hold
 // no particle of any scenario, now or at the last sort, so their totals are
-// zero and their starts stand.  When
-// `list` is given, cells holding two or more particles are appended to it
-// (the cells whose order k_segment_order has to establish).
+// zero and their starts stand.  The crowded cells are listed.
 __device__ __forceinline__ int block_incl_scan(int v, int* wsum) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int incl = v;
@@ -372,28 +408,27 @@ __device__ __forceinline__ void scan_tiles_of(const Scalars* S, int n, int range
 
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_sums(const int* __restrict__ count, int n, int* __restrict__ tile_sum,
-                int* __restrict__ list_n, const Scalars* S, Gate gate, int ranged,
-                const unsigned char* __restrict__ tflag) {
-  if (!gate_open(S, gate)) return;
-  if (list_n && blockIdx.x == 0 && threadIdx.x < 3) list_n[threadIdx.x] = 0;
-  int t0, t1;
-  scan_tiles_of(S, n, ranged, t0, t1);
+                const Scalars* S) {
+  if (!S->active) return;
   const int t = blockIdx.x;
-  if (t < t0 || t > t1) return;  // block-uniform
-  if (tflag && !tflag[t]) {  // a tile no scenario's keys meet: no particles
-    if (threadIdx.x == 0) tile_sum[t] = 0;
-    return;
-  }
   __shared__ int wsum[32];
   const int4 c = load_count4(count, t * kScanTile + threadIdx.x * 4, n);
   const int tot = block_sum(c.x + c.y + c.z + c.w, wsum);
   if (threadIdx.x == 0) tile_sum[t] = tot;
 }
 
+// Appends a thread's crowded cells among i0 .. i0+3 (of cv particles) to `big`.
+__device__ __forceinline__ void list_crowded(const int (&cv)[4], int i0, int* __restrict__ big,
+                                             int* __restrict__ big_n) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (cv[k] > kCrowded) big[atomicAdd(big_n, 1)] = i0 + k;
+}
+
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_apply(int* __restrict__ count, int n, const int* __restrict__ tile_sum,
-                 int* __restrict__ start, int* __restrict__ list,
-                 int* __restrict__ list_n, const Scalars* S, Gate gate, int ranged,
+                 int* __restrict__ start, int* __restrict__ big, int* __restrict__ list_n,
+                 const Scalars* S, Gate gate, int ranged,
                  const unsigned char* __restrict__ tflag) {
   if (!gate_open(S, gate)) return;
   int t0, t1;
@@ -427,109 +462,163 @@ __global__ void __launch_bounds__(kScanThreads)
         count[i0 + k] = 0;
       }
   }
-  if (list) {
-    // one atomic per warp: the warp's listed cells go to consecutive slots
+  if (big) {
     const int cv[4] = {c.x, c.y, c.z, c.w};
-    int mine = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) mine += cv[k] >= 2 ? 1 : 0;
-    const int lane = threadIdx.x & 31;
-    int incl2 = mine;
-#pragma unroll
-    for (int o2 = 1; o2 < 32; o2 <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, incl2, o2);
-      if (lane >= o2) incl2 += u;
-    }
-    const int wtot = __shfl_sync(0xffffffffu, incl2, 31);
-    int base = 0;
-    if (lane == 31 && wtot > 0) base = atomicAdd(list_n, wtot);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    int q = base + incl2 - mine;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (cv[k] >= 2) list[q++] = i0 + k;
+    list_crowded(cv, i0, big, list_n);
   }
   // start[n]: the total (with a key range: every particle, unchanged by a
   // step; written whenever the range reaches the last tile)
   if (t == (n - 1) / kScanTile && threadIdx.x == blockDim.x - 1) start[n] = pre + incl;
 }
 
-// perm[start[key] + slot] = the storage slot, skey there the key (the
-// cell of each sorted position, which G2P reads without waiting for perm)
-// and pk the entry idx << 32 | slot that the per-cell ordering sorts; block
-// 0 then rolls the key ranges over: the starts now describe knext, and the
-// next G2P starts an empty knext.
-__global__ void k_scatter(const int* __restrict__ key,
-                          const int* __restrict__ slot, const int* __restrict__ idx,
-                          const int* __restrict__ start, int* __restrict__ perm,
-                          int* __restrict__ skey, unsigned long long* __restrict__ pk,
-                          Scalars* S, Gate gate) {
-  if (!gate_open(S, gate)) return;
-  const int np = S->np;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np;
-       i += gridDim.x * blockDim.x) {
-    const int k = key[i];
-    const int pos = start[k] + slot[i];
-    perm[pos] = i;
-    skey[pos] = k;
-    pk[pos] = ((unsigned long long)(unsigned)idx[i] << 32) | (unsigned)i;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    S->krange[0] = S->knext[0];
-    S->krange[1] = S->knext[1];
-    S->knext[0] = 0x7fffffff;
-    S->knext[1] = -1;
+// The starts now describe the keys the last G2P made, and the next G2P starts
+// an empty range.
+__device__ __forceinline__ void roll_keys(Scalars* S) {
+  S->krange[0] = S->knext[0];
+  S->krange[1] = S->knext[1];
+  S->knext[0] = 0x7fffffff;
+  S->knext[1] = -1;
+}
+
+// Sorted position start[key] + slot takes the storage slot, the reference index
+// and the key (the cell of each sorted position, which G2P reads without waiting
+// for perm); inside a cell they lie as the count's atomics came.
+__device__ __forceinline__ void scatter(const Binning& n, const int* start, int np) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
+    const int k = n.key[i];
+    const int pos = start[k] + n.slot[i];
+    n.sslot[pos] = i;
+    n.sidx[pos] = n.idx[i];
+    n.skey[pos] = k;
   }
 }
 
-// Orders each listed cell's segment of perm (storage slots) by the
-// particles' reference index idx[slot] (the atomics of the count hand out
-// slots in arbitrary order).  A segment entry is the 64-bit value
-// idx << 32 | slot that the scatter wrote to pk at the same position, so
-// sorting those values orders by reference index (unique) and carries the
-// slot along; a cell whose entries are already in order is left as it is.
-// k_segment_order: each lane sorts a cell of up to kThreadSort particles in
-// registers (a bitonic network over static indices) and hands larger cells on
-// to `mid`, crowded ones (above 32 * kRankPer) to `big`.
-// k_segment_order_large, one warp per cell of `mid`: a register bitonic sort
-// across the lanes for up to 32 particles, else a rank sort (each lane holds
-// kRankPer values and counts, over all the cell's values broadcast lane by
-// lane, those below each of its own; the values are unique, so the ranks are
-// a permutation of [0, m)); then one block per cell of `big`.
-constexpr int kThreadSort = 16;
-constexpr int kRankPer = 8;
-constexpr int kBigRun = 8192;  // entries of a sorted run (two buffers: 128 KB of shared memory)
-constexpr unsigned long long kNoEntry = ~0ull;
+// Also zeroes the tile totals (the scan has used them); block 0 rolls the key
+// ranges over.
+__global__ void k_scatter(Binning n, const int* __restrict__ start, int* __restrict__ tile_sum,
+                          int ntiles, Scalars* S, Gate gate) {
+  if (!gate_open(S, gate)) return;
+  scatter(n, start, S->np);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
+    tile_sum[t] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) roll_keys(S);
+}
 
-__device__ __forceinline__ void thread_sort_segment(int* __restrict__ seg, int m,
-                                                    const unsigned long long* __restrict__ pk) {
-  unsigned long long v[kThreadSort];
+// The scan and the scatter of a small grid (up to kSmallCells cells) in one
+// launch: every block scans all the counts into its shared memory, then
+// scatters its share of the particles; block 0 writes the starts and the list
+// of crowded cells.  The counts are zeroed by the kernel after (k_order_units):
+// blocks that start later still read them.
+// At 4096 particles on 64 x 64 cells the launches it replaces (tile totals, scan,
+// scatter) took 8.7 us, this one 4.2.  The line lies where a block's share of the
+// work, 64 KB of counts from L2, costs what the launches did.
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_scatter(const int* __restrict__ count, int ncell, int* __restrict__ start,
+                   int* __restrict__ big, int* __restrict__ list_n, Binning n, Scalars* S,
+                   Gate gate) {
+  if (!gate_open(S, gate)) return;
+  extern __shared__ int sstart[];  // ncell
+  __shared__ int wsum[32];
+  const bool writes = blockIdx.x == 0;
+  int carry = 0;
+  for (int t = 0; t * kScanTile < ncell; ++t) {
+    const int i0 = t * kScanTile + threadIdx.x * 4;
+    const int4 c = load_count4(count, i0, ncell);
+    const int v = c.x + c.y + c.z + c.w;
+    const int incl = block_incl_scan(v, wsum);
+    const int total = wsum[(kScanThreads >> 5) - 1];
+    const int cv[4] = {c.x, c.y, c.z, c.w};
+    int e = carry + incl - v;
 #pragma unroll
-  for (int k = 0; k < kThreadSort; ++k) v[k] = k < m ? pk[k] : kNoEntry;
-  bool in_order = true;
+    for (int k = 0; k < 4; ++k) {
+      if (i0 + k < ncell) {
+        sstart[i0 + k] = e;
+        if (writes) start[i0 + k] = e;
+      }
+      e += cv[k];
+    }
+    if (writes) list_crowded(cv, i0, big, list_n);
+    carry += total;
+    __syncthreads();  // wsum is free again; the starts are in place
+  }
+  scatter(n, sstart, S->np);
+  if (writes && threadIdx.x == 0) {
+    start[ncell] = carry;
+    roll_keys(S);
+  }
+}
+
+// The order inside the cells, by the particles' reference index (unique; the
+// atomics of the count hand out a cell's places in arbitrary order): a
+// position's particle goes to the place its index has among those of its cell,
+// counted over the cell's indices.  A warp takes tiles of kOrderPer positions per
+// lane, with the indices of all their cells in its part `win` of the shared
+// memory (no more than kCrowded before and behind the tile): the lanes lie in a
+// few cells and mostly read the same word, and no warp waits for another.
+// Warp w of nw takes every nw-th tile.
+// Before, a lane sorted a cell of up to 16 particles in registers and a warp a
+// larger one, from lists of cells: reads of 32 cells by 32 lanes, and at 16
+// particles per cell half of the cells in the warps' share.  Counting over the
+// indices in global memory is bound by L1's tag lookups, with a block's tile in
+// shared memory by the block's barriers (k_order_units 66 and 60 us at 4M
+// particles, this way 42; 24 B a particle, which take 15 us).
+constexpr int kOrderPer = 4;
+constexpr int kOrderWin = 32 * kOrderPer + 2 * kCrowded;
+__device__ __forceinline__ void order_cells(const CellOrder& o, int np, int w, int nw, int* win) {
+  const int lane = threadIdx.x & 31;
+  const int per = max(1, min(kOrderPer, np / (32 * nw)));
+  const int tile = 32 * per;
+  const int tiles = (np - 1) / tile + 1;
+  int key[kOrderPer];
+  const auto load_keys = [&](int t) {
 #pragma unroll
-  for (int k = 1; k < kThreadSort; ++k) in_order &= (k >= m) || v[k - 1] < v[k];
-  if (in_order) return;  // perm already holds this order
+    for (int u = 0; u < kOrderPer; ++u) {
+      const int p = t * tile + u * 32 + lane;
+      key[u] = t < tiles && u < per && p < np ? o.n.skey[p] : -1;
+    }
+  };
+  if (np <= 0) return;
+  load_keys(w);
+  for (int t = w; t < tiles; t += nw) {
+    const int p0 = t * tile + lane;
+    int b[kOrderPer], e[kOrderPer], slot[kOrderPer];
+    int lo = 0x7fffffff, hi = 0;  // the cells' positions (crowded ones left out)
 #pragma unroll
-  for (int k = 2; k <= kThreadSort; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-#pragma unroll
-      for (int i = 0; i < kThreadSort; ++i) {
-        const int l = i ^ j;
-        if (l > i) {
-          const unsigned long long a = v[i], b = v[l];
-          const bool up = (i & k) == 0;
-          const bool sw = up ? (a > b) : (a < b);
-          v[i] = sw ? b : a;
-          v[l] = sw ? a : b;
-        }
+    for (int u = 0; u < kOrderPer; ++u) {
+      b[u] = e[u] = slot[u] = 0;
+      if (key[u] >= 0) {
+        b[u] = o.start[key[u]];
+        e[u] = o.start[key[u] + 1];
+        slot[u] = o.n.sslot[p0 + u * 32];
       }
     }
-  }
 #pragma unroll
-  for (int k = 0; k < kThreadSort; ++k)
-    if (k < m) seg[k] = int(unsigned(v[k]));
+    for (int u = 0; u < kOrderPer; ++u) {
+      if (e[u] - b[u] > kCrowded) e[u] = b[u];  // order_crowded's
+      if (e[u] > b[u]) {
+        lo = min(lo, b[u]);
+        hi = max(hi, e[u]);
+      }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lo < hi)  // (else crowded cells only: lo + lane would overflow)
+      for (int i = lo + lane; i < hi; i += 32) win[i - lo] = o.n.sidx[i];
+    load_keys(t + nw < tiles ? t + nw : tiles);
+    __syncwarp();  // the window is filled
+#pragma unroll
+    for (int u = 0; u < kOrderPer; ++u) {
+      const int n = e[u] - b[u];
+      if (n == 0) continue;
+      const int mine = win[p0 + u * 32 - lo];
+      const int* v = win + (b[u] - lo);
+      int rank = 0;
+#pragma unroll 4
+      for (int i = 0; i < n; ++i) rank += v[i] < mine ? 1 : 0;
+      o.perm[b[u] + rank] = slot[u];
+    }
+    __syncwarp();  // the window is free
+  }
 }
 
 // the 32 values of a warp (one per lane) in ascending order across the lanes
@@ -579,101 +668,25 @@ __device__ __forceinline__ void merge_level(const unsigned long long* src,
   }
 }
 
-__device__ __forceinline__ void warp_sort_segment(int* __restrict__ perm, int b, int m,
-                                                  int lane,
-                                                  const unsigned long long* __restrict__ pk) {
-  if (m <= 32) {
-    const unsigned long long v = warp_bitonic32((lane < m) ? pk[b + lane] : kNoEntry, lane);
-    if (lane < m) perm[b + lane] = int(unsigned(v));
-  } else {
-    unsigned long long v[kRankPer];
-    int rank[kRankPer];
-#pragma unroll
-    for (int t = 0; t < kRankPer; ++t) {
-      const int q = lane + 32 * t;
-      v[t] = (q < m) ? pk[b + q] : kNoEntry;
-      rank[t] = 0;
-    }
-#pragma unroll
-    for (int t2 = 0; t2 < kRankPer; ++t2) {
-      if (32 * t2 >= m) break;  // warp-uniform
-      for (int src = 0; src < 32; ++src) {
-        const unsigned long long o = __shfl_sync(0xffffffffu, v[t2], src);
-#pragma unroll
-        for (int t = 0; t < kRankPer; ++t) rank[t] += (o < v[t]) ? 1 : 0;
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < kRankPer; ++t)
-      if (lane + 32 * t < m) perm[b + rank[t]] = int(unsigned(v[t]));
-  }
-}
-
-// (four resident blocks per SM: registers for a lane's whole cell)
-__global__ void __launch_bounds__(256, 4) k_segment_order(const int* __restrict__ start,
-                                const int* __restrict__ list,
-                                int* __restrict__ list_n,
-                                int* __restrict__ perm,
-                                const unsigned long long* __restrict__ pk,
-                                int* __restrict__ mid, int* __restrict__ big,
-                                const Scalars* S, Gate gate) {
-  if (!gate_open(S, gate)) return;
+// All blocks of the kernel call it, with `sv` = two buffers of kBigRun entries
+// in shared memory: zeroes the counts and orders the crowded cells by the
+// entries idx << 32 | slot.  Runs of up to kBigRun of them are sorted in
+// shared memory -- groups of 32 by a bitonic network in each warp's registers,
+// then merged level by level along the merge path between two buffers -- and
+// written to pk[b, b+m); longer cells then merge the sorted runs pairwise,
+// ping-ponging between pk[b, b+m) and pk[cap + b, cap + b + m): each thread finds where its
+// piece of the output starts by a binary search along the merge path, then
+// merges the piece sequentially.  The slots go back to perm.
+__device__ __forceinline__ void order_crowded(const CellOrder& o, unsigned long long* sv) {
   const int lane = threadIdx.x & 31;
-  const int nl = list_n[0];
-  for (int w0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; w0 < nl;
-       w0 += ((gridDim.x * blockDim.x) >> 5) * 32) {
-    const int q = w0 + lane;
-    int c = 0, b = 0, m = 0;
-    if (q < nl) {
-      c = list[q];
-      b = start[c];
-      m = start[c + 1] - b;
-    }
-    if (m <= kThreadSort) {
-      if (m >= 2) thread_sort_segment(perm + b, m, pk + b);
-    }
-    // larger cells: one atomic per warp
-    const unsigned larger = __ballot_sync(0xffffffffu, m > kThreadSort);
-    if (larger) {
-      const bool crowded = m > 32 * kRankPer;
-      const unsigned most = __ballot_sync(0xffffffffu, crowded);
-      const unsigned some = larger & ~most;
-      int base = 0;
-      if (lane == 0 && some) base = atomicAdd(&list_n[2], __popc(some));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (m > kThreadSort && !crowded) mid[base + __popc(some & ((1u << lane) - 1u))] = c;
-      if (crowded) big[atomicAdd(&list_n[1], 1)] = c;
-    }
-  }
-}
-
-// The larger cells.  Those of the mid list: one warp each.  Crowded cells
-// (more than 32 * kRankPer particles), one block of 1024 threads each: runs of up to kBigRun entries of tmp[b, b+m) (the pk the
-// scatter wrote) are sorted in shared memory -- groups of 32 by a bitonic
-// network in each warp's registers, then merged level by level along the
-// merge path between two buffers -- and written back; longer cells then
-// merge the sorted runs pairwise, ping-ponging between tmp[b, b+m) and
-// tmp[cap + b, cap + b + m): each thread finds where its piece of the output
-// starts by a binary search along the merge path, then merges the piece
-// sequentially.  The slots go back to perm.
-__global__ void __launch_bounds__(1024)
-    k_segment_order_large(const int* __restrict__ start, const int* __restrict__ mid,
-                          const int* __restrict__ big, const int* __restrict__ list_n,
-                          int* __restrict__ perm, unsigned long long* __restrict__ tmp,
-                          long long cap, const Scalars* S, Gate gate) {
-  if (!gate_open(S, gate)) return;
-  extern __shared__ unsigned long long sv[];  // two buffers of kBigRun entries
-  const int nm = list_n[2];
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nm;
-       w += (gridDim.x * blockDim.x) >> 5) {
-    const int c = mid[w];
-    const int b = start[c];
-    warp_sort_segment(perm, b, start[c + 1] - b, threadIdx.x & 31, tmp);
-  }
-  const int nb = list_n[1];
+  const int* __restrict__ start = o.start;
+  int* __restrict__ perm = o.perm;
+  const int nb = o.list_n[0];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n_count; i += gridDim.x * blockDim.x)
+    o.count[i] = 0;
   for (int q = blockIdx.x; q < nb; q += gridDim.x) {
-    const int c = big[q];
+    unsigned long long* tmp = o.pk;
+    const int c = o.big[q];
     const int b = start[c], m = start[c + 1] - b;
     for (int r0 = 0; r0 < m; r0 += kBigRun) {
       const int len = min(kBigRun, m - r0);
@@ -681,10 +694,14 @@ __global__ void __launch_bounds__(1024)
       unsigned long long* B = sv + kBigRun;
       // groups of 32 sorted in registers, one warp each, then merged level
       // by level between the two buffers
-      const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-      for (int g = threadIdx.x >> 5; g * 32 < len; g += nw) {
+      const int bw = blockDim.x >> 5;
+      for (int g = threadIdx.x >> 5; g * 32 < len; g += bw) {
         const int q = g * 32 + lane;
-        const unsigned long long v = warp_bitonic32(q < len ? tmp[b + r0 + q] : kNoEntry, lane);
+        const int p = b + r0 + q;
+        const unsigned long long v = warp_bitonic32(
+            q < len ? ((unsigned long long)(unsigned)o.n.sidx[p] << 32) | (unsigned)o.n.sslot[p]
+                    : kNoEntry,
+            lane);
         if (q < len) A[q] = v;
       }
       __syncthreads();
@@ -699,7 +716,7 @@ __global__ void __launch_bounds__(1024)
       __syncthreads();
     }
     unsigned long long* src = tmp + b;
-    unsigned long long* dst = tmp + cap + b;
+    unsigned long long* dst = tmp + o.cap + b;
     for (int w = kBigRun; w < m; w <<= 1) {
       for (int lo = 0; lo < m; lo += 2 * w) {  // runs [lo, lo+w) and [lo+w, lo+2w)
         const int la = min(w, m - lo), lb = max(0, min(w, m - lo - la));
@@ -1190,36 +1207,10 @@ __device__ __forceinline__ void solo_batch(Chains<R>& a, P2GSmemT<R>& s, int rc,
 // carries about the same weight -- its particles plus kColWeight per column
 // -- whatever the local particle density: P2G takes them from a shared
 // cursor, so its time is the average load rather than the heaviest fixed
-// block.  The list is in (strip, column) order and the ledger partial of
-// list entry u sits in slot u, so the ledger reduction order is fixed.
+// block.  The list is in no particular order; the ledger partial of a strip's
+// n-th unit sits in the strip's n-th slot, so the ledger reduction order is
+// fixed.
 namespace {
-
-template <typename T>
-__device__ __forceinline__ T block_incl_scan(T v, T* warp_tot, T& total) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const T u = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += u;
-  }
-  if (lane == 31) warp_tot[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    T t = lane < nw ? warp_tot[lane] : T(0);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const T u = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += u;
-    }
-    if (lane < nw) warp_tot[lane] = t;
-  }
-  __syncthreads();
-  if (w > 0) v += warp_tot[w - 1];
-  total = warp_tot[nw - 1];
-  __syncthreads();  // warp_tot is free again
-  return v;
-}
 
 __device__ __forceinline__ int column_count(const int* __restrict__ cstart,
                                             int rlo, int rhi, int cc, int nrows) {
@@ -1228,79 +1219,123 @@ __device__ __forceinline__ int column_count(const int* __restrict__ cstart,
 
 }  // namespace
 
-// One block per strip.  Pass A: node column nc (< ncols) weighs the
-// particles of cell column nc in the strip's cell rows plus kColWeight; nc
-// starts a unit where floor(exclusive prefix / T) changes.  Pass B keeps the
-// units with particles (including those of the leading column cA-1, which
-// feed node column cA).
-// Cuts strip `strip` of one grid (cstart of that grid's cells) into units
-// of weight about T; st/px are the strip's scratch, plan its output.  All
-// threads of the block call it; it returns the number of units kept.
-__device__ __forceinline__ int plan_strip(const int* __restrict__ cstart,
-                                          const Geom& G, long long T, int strip,
-                                          int* __restrict__ st,
-                                          long long* __restrict__ px,
-                                          int4* __restrict__ plan, int col_weight,
-                                          int c_lo, int c_hi, int* __restrict__ heavy_n) {
-  __shared__ long long wt_ll[32];
-  __shared__ int wt_i[32];
-  __shared__ long long last_id;
+// Cuts strip `strip` of one grid (cstart of that grid's cells, node columns
+// [c_lo, c_hi]) into units of weight about T and appends those with particles
+// (including the particles of the leading column cA-1, which feed node column
+// cA) to P2G's list as make(cA, cB), with the ledger slot slot0 + n of the
+// strip's n-th unit; units of more than twice the target weight (a crowded
+// column) go to the half of the list that P2G takes first.  *strip_n: the
+// number of units.  Node column nc (< ncols) weighs the particles of cell column
+// nc in the strip's cell rows plus col_weight; nc starts a unit where
+// floor(exclusive prefix / T) changes.
+// One warp cuts a strip, 32 columns at a time, and needs no barrier: a lane
+// whose column starts a unit emits the one that ends there.  The units wait in
+// `buf` (kUnitBuf entries of shared memory) and are appended together, so that
+// nothing has to wait for all the strips.  With one block per strip, scans over
+// the block and a flat list by the last block, this took 8 us at 4096 particles,
+// 12 at 4M and 30 for the 800 strips of a batch of 96 scenarios, all of it on the
+// way to P2G; by warps it runs beside the ordering (below).
+constexpr int kUnitBuf = int(2 * sizeof(unsigned long long) * kBigRun / sizeof(int4)) /
+                         (kOrderThreads / 32);
+
+template <class Make>
+__device__ __forceinline__ void flush_units(const UnitPlan& u, const int4* buf, int n, int heavies,
+                                            int slot, Make make) {
+  const int lane = threadIdx.x & 31;
+  int at = 0;  // lane 0: the plain units' place, lane 1: the heavy ones'
+  if (lane == 0 && n > heavies) at = atomicAdd(u.ucount + kUnitsPlain, n - heavies);
+  if (lane == 1 && heavies > 0) at = u.cap + atomicAdd(u.ucount + kUnitsHeavy, heavies);
+  __syncwarp();  // the buffer is written
+  int plain = __shfl_sync(0xffffffffu, at, 0), heavy = __shfl_sync(0xffffffffu, at, 1);
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    const int i = i0 + lane;
+    int4 e = make_int4(0, 0, 0, 0);
+    if (i < n) e = buf[i];
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned mh = __ballot_sync(0xffffffffu, i < n && e.z);
+    const unsigned mp = __ballot_sync(0xffffffffu, i < n && !e.z);
+    if (i < n) {
+      const int f = e.z ? heavy + __popc(mh & below) : plain + __popc(mp & below);
+      u.ulist[f] = make(e.x, e.y);
+      u.uslot[f] = slot + i;
+    }
+    plain += __popc(mp);
+    heavy += __popc(mh);
+  }
+  __syncwarp();  // the buffer is free
+}
+
+template <class Make>
+__device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const Geom& G,
+                                           long long T, int strip, int4* buf, const UnitPlan& u,
+                                           int slot0, int* strip_n, int col_weight, int c_lo,
+                                           int c_hi, Make make) {
   const int nrows = G.nrows, ncols = G.ncols;
   const int r0 = strip * kTR;
   const int rlo = max(r0 - 1, 0), rhi = min(r0 + kTR - 1, nrows - 1);
-  long long carry = 0, prev_id = -1;
-  int K = 0;
-  for (int base = c_lo; base <= c_hi; base += blockDim.x) {
-    const int nc = base + threadIdx.x;
-    long long w = 0;
-    if (nc <= c_hi && nc < ncols) w = column_count(cstart, rlo, rhi, nc, nrows) + col_weight;
-    long long tot;
-    const long long incl = block_incl_scan<long long>(w, wt_ll, tot);
+  const int lane = threadIdx.x & 31;
+  const unsigned T32 = unsigned(T);
+  // floor(p / T): in 32 bits where p allows it (T always does)
+  const auto part = [&](long long p) {
+    return (unsigned long long)p >> 32 ? p / T : (long long)(unsigned(p) / T32);
+  };
+  const auto column = [&](int nc) {
+    return nc <= c_hi && nc < ncols ? column_count(cstart, rlo, rhi, nc, nrows) : 0;
+  };
+  int J = 0, n = 0, heavies = 0;  // units flushed, in the buffer, heavy ones among them
+  const auto emit = [&](bool ends, int cA, int cB, long long p0, long long p1, int prev) {
+    const long long np = p1 - p0 - (long long)col_weight * (min(cB, ncols) - cA) + prev;
+    const bool keep = ends && np > 0, heavy = np > 2 * T;
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if (keep) buf[n + __popc(m & ((1u << lane) - 1u))] = make_int4(cA, cB, heavy ? 1 : 0, 0);
+    n += __popc(m);
+    heavies += __popc(__ballot_sync(0xffffffffu, keep && heavy));
+    if (n > kUnitBuf - 32) {
+      flush_units(u, buf, n, heavies, slot0 + J, make);
+      J += n;
+      n = heavies = 0;
+    }
+  };
+  // the open unit: its first column, the prefix there, the column before it
+  int oA = c_lo, oV = c_lo > 0 ? column_count(cstart, rlo, rhi, c_lo - 1, nrows) : 0;
+  long long oP = 0, carry = 0;
+  int last = oV;  // particles of the column before the tile
+  int next = column(c_lo + lane), next2 = column(c_lo + 32 + lane);
+  for (int base = c_lo; base <= c_hi; base += 32) {
+    const int nc = base + lane;
+    const int cnt = next;
+    next = next2;
+    next2 = column(nc + 64);
+    const long long w = nc <= c_hi && nc < ncols ? (long long)cnt + col_weight : 0;
+    long long incl = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
     const long long pex = carry + incl - w;
-    const long long id = pex / T;
-    // id of the column before: the neighbour thread's, or the previous tile's
-    long long idp = __shfl_up_sync(0xffffffffu, id, 1);
-    if ((threadIdx.x & 31) == 31) wt_ll[threadIdx.x >> 5] = id;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0)
-      idp = threadIdx.x == 0 ? prev_id : wt_ll[(threadIdx.x >> 5) - 1];
-    if (threadIdx.x == blockDim.x - 1) last_id = id;
-    __syncthreads();
-    const int flag = (nc == c_lo) || (nc <= c_hi && nc < ncols && id != idp);
-    int ktot;
-    const int kin = block_incl_scan<int>(flag, wt_i, ktot);
-    if (flag) {
-      st[K + kin - 1] = nc;
-      px[K + kin - 1] = pex;
+    int prev = __shfl_up_sync(0xffffffffu, cnt, 1);
+    if (lane == 0) prev = last;
+    const bool starts = nc > c_lo && nc <= c_hi && nc < ncols &&
+                        part(pex) != part(pex - prev - col_weight);
+    const unsigned m = __ballot_sync(0xffffffffu, starts);
+    if (m) {
+      const unsigned below = m & ((1u << lane) - 1u);
+      const int src = below ? 31 - __clz(below) : lane;
+      const long long sp = __shfl_sync(0xffffffffu, pex, src);
+      const int sv = __shfl_sync(0xffffffffu, prev, src);
+      emit(starts, below ? base + src : oA, nc, below ? sp : oP, pex, below ? sv : oV);
+      const int l = 31 - __clz(m);
+      oA = base + l;
+      oP = __shfl_sync(0xffffffffu, pex, l);
+      oV = __shfl_sync(0xffffffffu, prev, l);
     }
-    carry += tot;
-    prev_id = last_id;
-    K += ktot;
-    __syncthreads();
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+    last = __shfl_sync(0xffffffffu, cnt, 31);
   }
-  const long long ptotal = carry;
-  int J = 0;
-  for (int base = 0; base < K; base += blockDim.x) {
-    const int k = base + threadIdx.x;
-    int flag = 0, cA = 0, cB = 0, heavy = 0;
-    if (k < K) {
-      cA = st[k];
-      const bool more = k + 1 < K;
-      cB = more ? st[k + 1] : c_hi + 1;
-      const long long sumw = (more ? px[k + 1] : ptotal) - px[k];
-      const long long n = sumw - (long long)col_weight * (min(cB, ncols) - cA) +
-                          (cA > 0 ? column_count(cstart, rlo, rhi, cA - 1, nrows) : 0);
-      flag = n > 0;
-      // more than twice the target weight (a crowded column): heavy
-      heavy = n > 2 * T ? 1 : 0;
-    }
-    int jtot;
-    const int jin = block_incl_scan<int>(flag, wt_i, jtot);
-    if (flag) plan[J + jin - 1] = make_int4(cA, cB, heavy, 0);  // P2G takes heavy units first
-    if (flag && heavy) atomicAdd(heavy_n, 1);
-    J += jtot;
-  }
-  return J;
+  emit(lane == 0, oA, c_hi + 1, oP, carry, oV);
+  if (n > 0) flush_units(u, buf, n, heavies, slot0 + J, make);
+  if (lane == 0) *strip_n = J + n;
 }
 
 __device__ __forceinline__ long long unit_weight(const Scalars* S,
@@ -1309,110 +1344,61 @@ __device__ __forceinline__ long long unit_weight(const Scalars* S,
   return T < kUnitMinWeight ? kUnitMinWeight : T;
 }
 
-// The order P2G hands the units out in: the heavy ones first, then the
-// others, each group in list order (a stable partition; heavy(f) is 0 or 1).
-// A unit's ledger slot stays its list position, so the order changes no sum.
-// All threads of the block call it.
-template <class F>
-__device__ __forceinline__ void heavy_first(int total, F heavy, int* __restrict__ uorder,
-                                            int* wt) {
-  int hc = 0;
-  for (int f = threadIdx.x; f < total; f += blockDim.x) hc += heavy(f);
-  int H;
-  block_incl_scan<int>(hc, wt, H);
-  int carry = 0;
-  for (int base = 0; base < total; base += blockDim.x) {
-    const int f = base + threadIdx.x;
-    const int h = f < total ? heavy(f) : 0;
-    int tot;
-    const int incl = block_incl_scan<int>(h, wt, tot);
-    if (f < total) uorder[h ? carry + incl - 1 : H + f - (carry + incl)] = f;
-    carry += tot;
-  }
+// The planning warps of the grid, spread over the blocks: warp 0 of each block,
+// then warp 1 ...
+__device__ __forceinline__ int plan_warp() {
+  return int(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+}
+// The order inside the cells is the other warps' (everyone's where that leaves
+// fewer than half).
+__device__ __forceinline__ void order_share(const CellOrder& o, int np, int w, int strips, int nw,
+                                            unsigned long long* sv) {
+  static_assert(kOrderWin * sizeof(int) <= kUnitBuf * sizeof(int4), "");
+  int* win = reinterpret_cast<int*>(reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf);
+  const int planners = 2 * strips <= nw ? strips : 0;
+  if (w >= planners) order_cells(o, np, w - planners, nw - planners, win);
+}
+__device__ __forceinline__ int4* unit_buf(unsigned long long* sv) {
+  return reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf;
 }
 
-// Strip offsets uoff (strips + 1) by a scan of strip_n, by all threads of the
-// block; returns the number of units.
-__device__ __forceinline__ int strip_offsets(const int* strip_n, int strips, int* uoff,
-                                             int* wt) {
-  int carry = 0;
-  for (int base = 0; base < strips; base += blockDim.x) {
-    const int s = base + threadIdx.x;
-    const int n = s < strips ? __ldcg(strip_n + s) : 0;
-    int tot;
-    const int incl = block_incl_scan<int>(n, wt, tot);
-    if (s < strips) uoff[s] = carry + incl - n;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) uoff[strips] = carry;
-  __syncthreads();
-  return carry;
-}
-
-__device__ __forceinline__ int strip_of_unit(const int* uoff, int strips, int f) {
-  int lo = 0, hi = strips;  // uoff[lo] <= f < uoff[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (uoff[mid] <= f) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
-// One block per strip cuts its units; the last block to finish writes the
-// flat list {strip, cA, cB} in (strip, column) order and, unless the pass has
-// begun (a merge/split came before the sort), ends the step before and begins
-// this one.
-// A small scenario's step is bound by its chain of launches (2-3 us each with
-// the gap before it): the list, the step's begin and end, the ledger (a block
-// of G2P) and the sort of the larger cells were launches of their own, 13 in
-// all; with 8 the step of a 4096-particle dam break takes 42 us instead of
-// 49, that of a 0.25M-particle mudflow 97 instead of 104.  The begin sits here
-// and not at the end of G2P, where every block would have to wait for its
-// stores before it counts itself done (7 us at 0.25M and 4M particles).
-// ucount[0] = units, ucount[1] = P2G's work cursor, ucount[2] = heavy units
-// (P2G reads uorder when there are any, else takes the list in order),
-// ucount[3] = the heavy units the strips count, ucount[4] = the blocks done.
-__global__ void __launch_bounds__(kPlanThreads)
-    k_units(const int* __restrict__ cstart, Geom G, Phys P, Scalars* S, int target_units,
-            int seg, int* __restrict__ ustart, long long* __restrict__ upex, int4* plan,
-            int* strip_n, int4* ulist, int* __restrict__ uorder, int* ucount, Gate gate) {
+// The last kernel of a sort: P2G's work list, which needs the cell starts only,
+// and the order inside the cells.  The last block to finish ends the step before
+// and begins this one unless it has begun (a merge/split came before the sort):
+// no block still reads the loop condition then.
+// The planner and the order of the smaller and of the larger cells were launches
+// of their own: 46 us in all at 4M particles, 20 at 0.25M, 13 at 4096 and 53 in a
+// batch of 96 scenarios; together 42, 13, 6 and 13.
+// The begin sits here and not at the end of G2P, where every block would have
+// to wait for its stores before it counts itself done (7 us at 0.25M and 4M
+// particles).
+// strips = 0: the sort alone (before a merge/split); seg: unit slots per strip
+__global__ void __launch_bounds__(kOrderThreads, 1)
+    k_order_units(CellOrder o, UnitPlan u, Geom G, Phys P, Scalars* S, int strips, int seg,
+                  Gate gate) {
   if (!gate_open(S, gate)) {
     if (!gate.begun && blockIdx.x == 0 && threadIdx.x == 0) S->active = 0;
     return;
   }
-  extern __shared__ int uoff[];  // strips + 1
-  __shared__ int wt_i[32];
-  const int strip = blockIdx.x, strips = gridDim.x;
-  const size_t b = (size_t)strip * seg;
+  extern __shared__ unsigned long long sv[];
   // node columns of the cells the particles are binned to (the key range the
   // scatter just rolled over), plus the column right of them
   const int L = S->krange[0], K = S->krange[1];
-  int J = 0;
-  if (L <= K) {
-    const int c_lo = L / G.nrows, c_hi = min(K / G.nrows + 1, G.ncols);
-    J = plan_strip(cstart, G, unit_weight(S, target_units), strip, ustart + b, upex + b,
-                   plan + b, kColWeight, c_lo, c_hi, ucount + 3);
+  const int w = plan_warp(), nw = (gridDim.x * blockDim.x) >> 5;
+  for (int strip = w; strip < strips; strip += nw) {
+    if (L <= K)
+      plan_strip(o.start, G, unit_weight(S, u.target_units), strip, unit_buf(sv), u, strip * seg,
+                 u.strip_n + strip, kColWeight, L / G.nrows, min(K / G.nrows + 1, G.ncols),
+                 [&](int cA, int cB) { return make_int4(strip, cA, cB, 0); });
+    else if ((threadIdx.x & 31) == 0)
+      u.strip_n[strip] = 0;
   }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) strip_n[strip] = J;
-  if (!last_block(ucount + 4, strips)) return;
-  const int H = __ldcg(ucount + 3);
-  const int total = strip_offsets(strip_n, strips, uoff, wt_i);
-  for (int f = threadIdx.x; f < total; f += blockDim.x) {
-    const int s = strip_of_unit(uoff, strips, f);
-    const int4 u = __ldcg(plan + (size_t)s * seg + (f - uoff[s]));
-    ulist[f] = make_int4(s, u.x, u.y, u.z);  // w: heavy
-  }
-  if (H > 0) {
-    __syncthreads();
-    heavy_first(total, [&](int f) { return ulist[f].w; }, uorder, wt_i);
-  }
+  order_share(o, S->np, w, strips, nw, sv);
+  __syncthreads();  // the shared memory is free again
+  order_crowded(o, sv);
+  if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;
   if (threadIdx.x == 0) {
-    ucount[0] = total;
-    ucount[1] = 0;
-    ucount[2] = H;  // P2G: list order when 0
-    ucount[3] = 0;
+    *o.list_n = 0;
     if (!gate.begun) step_begin_one(S, G, P);
   }
 }
@@ -1571,34 +1557,35 @@ template <bool kRecord>
 __global__ void __launch_bounds__(kP2GThreads, kP2GMinBlocks)
     k_p2g(Particles p, const int* __restrict__ perm,
           const int* __restrict__ cstart, Nodes nodes,
-          double* __restrict__ led_part, Geom G, Phys P, const Scalars* S,
-          const int4* __restrict__ ulist, const int* __restrict__ uorder,
-          const int* __restrict__ ucount) {
+          double* __restrict__ led_part, Geom G, Phys P, const Scalars* S, UnitPlan u) {
   constexpr int record = kRecord ? 1 : 0;
   if (!S->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   P2GSmem& s = *reinterpret_cast<P2GSmem*>(smem_raw);
-  const int nunits = ucount[0], nheavy = ucount[2];
+  const int nheavy = u.ucount[kUnitsHeavy], nunits = nheavy + u.ucount[kUnitsPlain];
   __shared__ int next_unit;
   while (true) {
-    // units are taken in the order of uorder (heavy ones first) from a
-    // shared cursor: CTAs that drew light units take more (the per-SM load
-    // stays even)
-    if (threadIdx.x == 0) next_unit = atomicAdd(const_cast<int*>(ucount) + 1, 1);
+    // units are taken from a shared cursor, the heavy ones first: CTAs that
+    // drew light units take more (the per-SM load stays even)
+    if (threadIdx.x == 0) next_unit = atomicAdd(u.ucount + kUnitCursor, 1);
     __syncthreads();
     const int k = next_unit;
     __syncthreads();
     if (k >= nunits) break;
-    const int ui = nheavy ? uorder[k] : k;
-    p2g_unit(p, perm, cstart, nodes, led_part, G, P, S, record, s, ui, ulist[ui]);
+    const int f = k < nheavy ? u.cap + k : k - nheavy;
+    p2g_unit(p, perm, cstart, nodes, led_part, G, P, S, record, s, u.uslot[f], u.ulist[f]);
   }
 }
 
-size_t sort_big_smem_bytes() { return 2 * sizeof(unsigned long long) * kBigRun; }
+size_t order_smem_bytes() { return 2 * sizeof(unsigned long long) * kBigRun; }
 
 int setup_sort() {
-  return cudaFuncSetAttribute(k_segment_order_large, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(sort_big_smem_bytes())) == cudaSuccess;
+  for (const void* f : {(const void*)k_order_units, (const void*)k_b_order_units})
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(order_smem_bytes())) != cudaSuccess)
+      return 0;
+  return cudaFuncSetAttribute(k_scan_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              int(sizeof(int)) * kSmallCells) == cudaSuccess;
 }
 
 int setup_p2g() {
@@ -1617,24 +1604,30 @@ int setup_p2g() {
 
 void launch_p2g(int grid, cudaStream_t st, Particles p, const int* perm, const int* cstart,
                 Nodes nodes, double* led_part, Geom G, Phys P, const Scalars* S, int record,
-                const int4* ulist, const int* uorder, const int* ucount) {
+                const UnitPlan& u) {
   if (record)
     k_p2g<true><<<grid, kP2GThreads, p2g_smem_bytes(), st>>>(p, perm, cstart, nodes, led_part,
-                                                             G, P, S, ulist, uorder, ucount);
+                                                             G, P, S, u);
   else
     k_p2g<false><<<grid, kP2GThreads, p2g_smem_bytes(), st>>>(p, perm, cstart, nodes, led_part,
-                                                              G, P, S, ulist, uorder, ucount);
+                                                              G, P, S, u);
 }
 
-// Block reduction, in a fixed order, of the ledger partials of units
-// [u0, u1) into S->ledger, and the conservation errors.
+// Block reduction, in a fixed order, of the ledger partials of a grid's units
+// -- strip_n[q] of them from slot q * seg on for strip q -- into S->ledger, and
+// the conservation errors.  One warp takes a strip, its lanes the units.
 __device__ __forceinline__ void ledger_reduce(const double* __restrict__ led_part,
-                                              int u0, int u1, Scalars* S) {
+                                              const int* __restrict__ strip_n, int strips,
+                                              int seg, Scalars* S) {
   __shared__ double sm[6][32];
   double v[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = u0 + threadIdx.x; b < u1; b += blockDim.x)
+  for (int b = threadIdx.x >> 5; b < strips; b += blockDim.x >> 5) {
+    const double* part = led_part + (size_t)b * seg * 6;
+    const int n = strip_n[b];
+    for (int f = threadIdx.x & 31; f < n; f += 32)
 #pragma unroll
-    for (int q = 0; q < 6; ++q) v[q] += led_part[(size_t)b * 6 + q];
+      for (int q = 0; q < 6; ++q) v[q] += part[(size_t)f * 6 + q];
+  }
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
     double x = v[q];
@@ -1664,9 +1657,9 @@ __device__ __forceinline__ void ledger_reduce(const double* __restrict__ led_par
 
 // log: a ring of kLedgerLog rows {t, err_mass, err_mom}, row (it-1) % kLedgerLog
 __device__ __forceinline__ void ledger_final(const double* __restrict__ led_part,
-                                             const int* __restrict__ ucount, Scalars* S,
-                                             double* __restrict__ log) {
-  ledger_reduce(led_part, 0, ucount[0], S);
+                                             const int* __restrict__ strip_n, int strips, int seg,
+                                             Scalars* S, double* __restrict__ log) {
+  ledger_reduce(led_part, strip_n, strips, seg, S);
   if (threadIdx.x == 0 && log) {
     double* row = log + 3 * ((S->it - 1) % kLedgerLog);
     row[0] = S->ledger[8];
@@ -1873,23 +1866,6 @@ __device__ __forceinline__ void flag_non_finite(int bad, Scalars* S) {
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&S->status, kStatusNonFinite);
 }
 
-// The counting sort's first step for the next binning, done where the keys
-// are made: particle j of a warp takes slot[j] among its cell's particles,
-// one atomic per cell and warp (the lanes that share a cell take
-// consecutive slots).  All 32 lanes call it; ok == false lanes take part
-// without a particle.
-__device__ __forceinline__ void count_key(int k, bool ok, int* __restrict__ count,
-                                          int* __restrict__ slot_out) {
-  const int lane = threadIdx.x & 31;
-  const int kk = ok ? k : -1;
-  const unsigned peers = __match_any_sync(0xffffffffu, kk);
-  const int leader = __ffs(peers) - 1;
-  int base = 0;
-  if (ok && lane == leader) base = atomicAdd(&count[kk], __popc(peers));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (ok) *slot_out = base + __popc(peers & ((1u << lane) - 1u));
-}
-
 // Block min/max of the new keys into knext (the scan range of the next
 // sort); all threads of the block call it.
 __device__ __forceinline__ void key_range(int kmin, int kmax, int* sred, Scalars* S) {
@@ -1946,9 +1922,10 @@ template <bool kRecord, bool kGrad>
 __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     k_g2p_t(Particles cur, Particles nxt, const int* __restrict__ perm,
             const int* __restrict__ skey, Nodes nodes, const double* __restrict__ Z, Geom G,
-            Phys P, Scalars* S, int* __restrict__ count, int* __restrict__ leave,
-            const double* __restrict__ led_part, const int* __restrict__ ucount,
-            double* __restrict__ log) {
+            Phys P, Scalars* S, int* __restrict__ count, int* __restrict__ tile_sum,
+            int* __restrict__ leave,
+            const double* __restrict__ led_part, const int* __restrict__ strip_n, int strips,
+            int seg, int* __restrict__ ucount, double* __restrict__ log) {
   const int ng = S->nghost;
   const int n = S->np - ng;  // the slab's own particles
   const int blk = blockIdx.x - 1;  // the first block sums the ledger
@@ -1960,7 +1937,8 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     return;
   }
   if (blk < 0) {
-    ledger_final(led_part, ucount, S, log);
+    ledger_final(led_part, strip_n, strips, seg, S, log);
+    if (threadIdx.x < kUnitCounts) ucount[kUnitsPlain + threadIdx.x] = 0;  // P2G is done
     if (threadIdx.x == 0) S->pending = 1;
     return;
   }
@@ -1997,7 +1975,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
         }
       }
     }
-    count_key(nkey, stay, count, nxt.slot + (ok ? t : 0));
+    count_key(nkey, stay, count, tile_sum, nxt.slot + (ok ? t : 0));
   }
   cfl_block_max(m0, m1, m2, red, S);
   key_range(kmin, kmax, kred, S);
@@ -2006,12 +1984,13 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
 
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
-                int* count, int* leave, const double* led_part, const int* ucount, double* log,
-                int record, int want_grad) {
+                int* count, int* tile_sum, int* leave, const double* led_part, const UnitPlan& u,
+                int strips, int seg, double* log, int record, int want_grad) {
   auto* kernel = record ? k_g2p_t<true, true>
                         : want_grad ? k_g2p_t<false, true> : k_g2p_t<false, false>;
   kernel<<<grid + 1, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G, P, S, count,
-                                           leave, led_part, ucount, log);
+                                           tile_sum, leave, led_part, u.strip_n, strips, seg,
+                                           u.ucount, log);
 }
 
 size_t p2g_smem_bytes() { return sizeof(P2GSmemT<double>); }
@@ -2092,86 +2071,42 @@ __global__ void k_b_step_end(const Scn* __restrict__ scn, Scalars* S, int nscn) 
     if (scn[s].live) step_end_one(&S[s]);
 }
 
-// One block per strip of the batch cuts its units; the last block to finish
-// writes the flat list {scenario, strip, cA, cB} in strip order and each
-// scenario's range of list positions (its ledger slots) and rolls the key
-// ranges over.  ucount as in k_units.
-__global__ void __launch_bounds__(kPlanThreads)
-    k_b_units(const int* __restrict__ cstart, const Scn* __restrict__ scn, Scalars* S,
-              int nscn, const int* __restrict__ strip_scn, const Scalars* Sg,
-              int target_units,
-              int col_weight, int* __restrict__ ustart, long long* __restrict__ upex,
-              int4* plan, int* strip_n, int4* ulist, int* __restrict__ uorder, int* ucount,
-              int2* __restrict__ scn_units) {
+// k_order_units of a batch: the list holds {scenario, strip, cA, cB}; the last
+// block to finish rolls the scenarios' key ranges over.
+__global__ void __launch_bounds__(kOrderThreads, 1)
+    k_b_order_units(CellOrder o, UnitPlan u, const Scn* __restrict__ scn, Scalars* S, int nscn,
+                    const int* __restrict__ strip_scn, int strips, const Scalars* Sg,
+                    int col_weight) {
   if (!Sg->active) return;
-  extern __shared__ int uoff[];  // strips + 1
-  __shared__ int wt_i[32];
-  const int b = blockIdx.x, strips = gridDim.x;
-  {
+  extern __shared__ unsigned long long sv[];
+  const int w = plan_warp(), nw = (gridDim.x * blockDim.x) >> 5;
+  for (int b = w; b < strips; b += nw) {
     const int s = strip_scn[b];
-    int J = 0;
-    if (S[s].active) {
-      const Geom G = scn[s].G;
-      const int local = b - scn[s].strip_off;
-      const size_t base = (size_t)scn[s].useg_off + (size_t)local * (G.ncols + 1);
-      // node columns of the cells the scenario's particles are binned to (the
-      // keys its last G2P made), plus the column right of them; every column
-      // after a layout change
-      int c_lo = 0, c_hi = G.ncols;
-      if (!(Sg->krange[0] <= Sg->krange[1])) {
-        const int L = S[s].knext[0], H = S[s].knext[1];
-        c_lo = (L - scn[s].c_off) / G.nrows;
-        c_hi = L > H ? -1 : min((H - scn[s].c_off) / G.nrows + 1, G.ncols);
-      }
-      if (c_hi >= 0)  // (else no particle)
-        J = plan_strip(cstart + scn[s].c_off, G, unit_weight(Sg, target_units), local,
-                       ustart + base, upex + base, plan + base, col_weight, c_lo, c_hi,
-                       ucount + 3);
+    const Geom G = scn[s].G;
+    const int local = b - scn[s].strip_off;
+    const int slot0 = scn[s].useg_off + local * (G.ncols + 1);
+    // node columns of the cells the scenario's particles are binned to (the
+    // keys its last G2P made), plus the column right of them; every column
+    // after a layout change
+    int c_lo = 0, c_hi = G.ncols;
+    if (!(Sg->krange[0] <= Sg->krange[1])) {
+      const int L = S[s].knext[0], H = S[s].knext[1];
+      c_lo = (L - scn[s].c_off) / G.nrows;
+      c_hi = L > H ? -1 : min((H - scn[s].c_off) / G.nrows + 1, G.ncols);
     }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) strip_n[b] = J;
+    if (S[s].active && c_hi >= 0)  // (else no particle)
+      plan_strip(o.start + scn[s].c_off, G, unit_weight(Sg, u.target_units), local, unit_buf(sv),
+                 u, slot0, u.strip_n + b, col_weight, c_lo, c_hi,
+                 [&](int cA, int cB) { return make_int4(s, local, cA, cB); });
+    else if ((threadIdx.x & 31) == 0)
+      u.strip_n[b] = 0;
   }
-  if (!last_block(ucount + 4, strips)) return;
-  const int H = __ldcg(ucount + 3);
-  const int total = strip_offsets(strip_n, strips, uoff, wt_i);
-  for (int f = threadIdx.x; f < total; f += blockDim.x) {
-    const int lo = strip_of_unit(uoff, strips, f);
-    const int s = strip_scn[lo];
-    const int local = lo - scn[s].strip_off;
-    const size_t base =
-        (size_t)scn[s].useg_off + (size_t)local * (scn[s].G.ncols + 1);
-    const int4 u = __ldcg(plan + base + (f - uoff[lo]));
-    ulist[f] = make_int4(s, local, u.x, u.y);
-  }
-  if (H > 0) {
-    __syncthreads();
-    heavy_first(
-      total,
-      [&](int f) {
-        const int4 L = ulist[f];
-        const int st = scn[L.x].strip_off + L.y;
-        const size_t base = (size_t)scn[L.x].useg_off + (size_t)L.y * (scn[L.x].G.ncols + 1);
-        return __ldcg(plan + base + (f - uoff[st])).z;
-      },
-      uorder, wt_i);
-  }
-  for (int s = threadIdx.x; s < nscn; s += blockDim.x) {
-    const int b0 = scn[s].strip_off, b1 = b0 + scn[s].nstrips;
-    scn_units[s] = make_int2(uoff[b0], uoff[b1]);
-    // each scenario's key ranges roll over: the starts now describe the
-    // keys its last G2P made, and the next G2P starts an empty range
-    S[s].krange[0] = S[s].knext[0];
-    S[s].krange[1] = S[s].knext[1];
-    S[s].knext[0] = 0x7fffffff;
-    S[s].knext[1] = -1;
-  }
-  if (threadIdx.x == 0) {
-    ucount[0] = total;
-    ucount[1] = 0;
-    ucount[2] = H;  // P2G: list order when 0
-    ucount[3] = 0;
-  }
+  order_share(o, Sg->np, w, strips, nw, sv);
+  __syncthreads();  // the shared memory is free again
+  order_crowded(o, sv);
+  if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;
+  if (threadIdx.x == 0) *o.list_n = 0;
+  for (int s = threadIdx.x; s < nscn; s += blockDim.x) roll_keys(&S[s]);
 }
 
 template <class R>
@@ -2179,28 +2114,27 @@ __global__ void __launch_bounds__(kP2GThreads, kP2GMinBlocks)
     k_b_p2g(ParticlesT<R> p, const int* __restrict__ perm, const int* __restrict__ cstart,
             V2<R>* __restrict__ vvL,
             double* __restrict__ led_part, const Scn* __restrict__ scn, Scalars* S,
-            const int4* __restrict__ ulist, const int* __restrict__ uorder,
-            const int* __restrict__ ucount, const Scalars* Sg) {
+            UnitPlan up, const Scalars* Sg) {
   if (!Sg->active) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   P2GSmemT<R>& sm = *reinterpret_cast<P2GSmemT<R>*>(smem_raw);
-  const int nunits = ucount[0], nheavy = ucount[2];
+  const int nheavy = up.ucount[kUnitsHeavy], nunits = nheavy + up.ucount[kUnitsPlain];
   __shared__ int next_unit;
   while (true) {
-    if (threadIdx.x == 0) next_unit = atomicAdd(const_cast<int*>(ucount) + 1, 1);
+    if (threadIdx.x == 0) next_unit = atomicAdd(up.ucount + kUnitCursor, 1);
     __syncthreads();
     const int k = next_unit;
     __syncthreads();
     if (k >= nunits) break;
-    const int ui = nheavy ? uorder[k] : k;  // heavy units first
-    const int4 u = ulist[ui];
+    const int f = k < nheavy ? up.cap + k : k - nheavy;  // heavy units first
+    const int4 u = up.ulist[f];
     const Geom G = scn[u.x].G;
     const Phys P = scn[u.x].P;
     const int n_off = scn[u.x].n_off, c_off = scn[u.x].c_off;
     NodesT<R> nd{};
     nd.vvL = vvL + n_off;
-    p2g_unit<R>(p, perm, cstart + c_off, nd, led_part, G, P, &S[u.x], 0, sm, ui,
-             make_int4(u.y, u.z, u.w, 0));
+    p2g_unit<R>(p, perm, cstart + c_off, nd, led_part, G, P, &S[u.x], 0, sm,
+                up.uslot[f], make_int4(u.y, u.z, u.w, 0));
   }
 }
 
@@ -2218,13 +2152,16 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
             const int* __restrict__ skey, const V2<R>* __restrict__ vvL,
             const double* __restrict__ Z,
             const Scn* __restrict__ scn, Scalars* S, const int2* __restrict__ gblk,
-            const Scalars* Sg, int* __restrict__ count, const double* __restrict__ led_part,
-            const int2* __restrict__ scn_units, int nscn) {
+            const Scalars* Sg, int* __restrict__ count, int* __restrict__ tile_sum,
+            const double* __restrict__ led_part, const int* __restrict__ strip_n,
+            int* __restrict__ ucount, int nscn) {
   if (blockIdx.x < nscn) {
     const int q = blockIdx.x;
     if (!Sg->active) return;
+    if (q == 0 && threadIdx.x < kUnitCounts) ucount[kUnitsPlain + threadIdx.x] = 0;  // P2G is done
     if (scn[q].live && S[q].active) {
-      ledger_reduce(led_part, scn_units[q].x, scn_units[q].y, &S[q]);
+      ledger_reduce(led_part + (size_t)scn[q].useg_off * 6, strip_n + scn[q].strip_off,
+                    scn[q].nstrips, scn[q].G.ncols + 1, &S[q]);
       if (threadIdx.x == 0) S[q].pending = 1;
     }
     return;
@@ -2253,7 +2190,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
       copy_moving(cur, perm[j], nxt, j);
       nkey = nxt.key[j];
     }
-    count_key(nkey, ok, count, nxt.slot + (ok ? j : 0));
+    count_key(nkey, ok, count, tile_sum, nxt.slot + (ok ? j : 0));
     key_range(ok ? nkey : 0x7fffffff, ok ? nkey : -1, kred, &S[s]);
     return;
   }
@@ -2269,7 +2206,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     g2p_particle(cur, perm[j], g2p_in(cur, perm[j]), skey[j], nxt, j, nd, Z + n_off, G, P,
                  sh, S[s].dt, 0, 0,
                  c_off, m0, m1, m2, bad, nkey);
-  count_key(nkey, ok, count, nxt.slot + (ok ? j : 0));
+  count_key(nkey, ok, count, tile_sum, nxt.slot + (ok ? j : 0));
   cfl_block_max(m0, m1, m2, red, &S[s]);
   key_range(ok ? nkey : 0x7fffffff, ok ? nkey : -1, kred, &S[s]);
   flag_non_finite(bad, &S[s]);
@@ -2307,18 +2244,6 @@ __global__ void k_b_move(ParticlesT<R> dst, ParticlesT<R> src, const int4* __res
   const int i = m.y + threadIdx.x, o = m.x + threadIdx.x;
   copy_moving(src, i, dst, o);
   dst.key[o] = src.key[i] + m.w;
-}
-
-// Slots and counts of the keys [0, n) (after an upload or a compaction).
-__global__ void k_count_n(const int* __restrict__ key, int* __restrict__ count,
-                          int* __restrict__ slot, int n) {
-  const int lane = threadIdx.x & 31;
-  const int stride = gridDim.x * blockDim.x;
-  for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
-    const int i = i0 + lane;
-    const bool ok = i < n;
-    count_key(ok ? key[i] : -1, ok, count, slot + (ok ? i : 0));
-  }
 }
 
 // nblk[b] = {destination first node, source first node, count <= 256, 0}
@@ -2383,10 +2308,9 @@ void launch_prep(int grid, int block, cudaStream_t st, ParticlesT<R> p, const do
 template <class R>
 void launch_b_p2g(int grid, cudaStream_t st, ParticlesT<R> p, const int* perm,
                   const int* cstart, V2<R>* vvL, double* led_part, const Scn* scn,
-                  Scalars* S, const int4* ulist, const int* uorder, const int* ucount,
-                  const Scalars* Sg) {
-  k_b_p2g<R><<<grid, kP2GThreads, sizeof(P2GSmemT<R>), st>>>(
-      p, perm, cstart, vvL, led_part, scn, S, ulist, uorder, ucount, Sg);
+                  Scalars* S, const UnitPlan& u, const Scalars* Sg) {
+  k_b_p2g<R><<<grid, kP2GThreads, sizeof(P2GSmemT<R>), st>>>(p, perm, cstart, vvL, led_part, scn,
+                                                             S, u, Sg);
 }
 
 template <class R>
@@ -2408,9 +2332,10 @@ template <class R>
 void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nxt,
                   const int* perm, const int* skey, const V2<R>* vvL, const double* Z,
                   const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count,
-                  const double* led_part, const int2* scn_units, int nscn) {
+                  int* tile_sum, const double* led_part, const UnitPlan& u, int nscn) {
   k_b_g2p<R><<<nblk + nscn, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, vvL, Z, scn, S, gblk,
-                                                  Sg, count, led_part, scn_units, nscn);
+                                                  Sg, count, tile_sum, led_part, u.strip_n, u.ucount,
+                                                  nscn);
 }
 
 template <class R>
@@ -2432,12 +2357,12 @@ void launch_b_move(int grid, cudaStream_t st, ParticlesT<R> dst, ParticlesT<R> s
                                Geom, Phys, const Scalars*, int);                      \
   template void launch_b_p2g<R>(int, cudaStream_t, ParticlesT<R>, const int*,         \
                                 const int*, V2<R>*, double*, const Scn*, Scalars*,    \
-                                const int4*, const int*, const int*, const Scalars*); \
+                                const UnitPlan&, const Scalars*);                     \
   template int setup_b_p2g<R>();                                                      \
   template void launch_b_g2p<R>(int, cudaStream_t, ParticlesT<R>, ParticlesT<R>,      \
                                 const int*, const int*, const V2<R>*, const double*,  \
                                 const Scn*, Scalars*, const int2*, Scalars*, int*,    \
-                                const double*, const int2*, int);                     \
+                                int*, const double*, const UnitPlan&, int);           \
   template void launch_b_unpack<R>(int, cudaStream_t, ParticlesT<R>, const double*, int); \
   template void launch_b_move<R>(int, cudaStream_t, ParticlesT<R>, ParticlesT<R>,     \
                                  const int4*);
