@@ -48,7 +48,7 @@ struct dampm_ctx {
   int* uslot = nullptr;   // their ledger slots
   int* cbig = nullptr;  // cells with more than 256 particles (capacity / 256)
   double* ledger_log = nullptr;  // kLedgerLog rows {t, err_mass, err_mom}
-  int p2g_grid = 0;
+  int p2g_grid = 0, p2g_ctas = 0;  // launched, resident at most
   Scalars* S = nullptr;
   Scalars* Sh = nullptr;  // pinned host mirror
   MsBuffers msb{};
@@ -254,8 +254,8 @@ bool small_grid(const dampm_ctx* ctx) { return ctx->nc <= kSmallCells; }
 int* tile_totals(const dampm_ctx* ctx) { return small_grid(ctx) ? nullptr : ctx->tile_sum; }
 
 UnitPlan unit_plan(const dampm_ctx* ctx) {
-  return UnitPlan{kUnitsPerCta * ctx->p2g_grid, ctx->n_led, ctx->ulist, ctx->uslot,
-                  ctx->strip_n, ctx->ucount};
+  return UnitPlan{kUnitsPerCta * ctx->p2g_grid, unit_min_weight(ctx->n_led, ctx->p2g_ctas),
+                  ctx->n_led, ctx->ulist, ctx->uslot, ctx->strip_n, ctx->ucount};
 }
 
 // Enqueues the binning of the current particles (SORT), whose slots and
@@ -726,6 +726,7 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (per_sm < 1) per_sm = 1;
+    ctx->p2g_ctas = nsm * per_sm;
     ctx->p2g_grid = std::max(1, std::min(nsm * per_sm, ctx->n_led));
   }
   if (rc != DAMPM_OK) {

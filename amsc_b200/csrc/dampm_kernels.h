@@ -21,6 +21,16 @@ constexpr int kTR = 30;
 #endif
 constexpr int kUnitsPerCta = DAMPM_UNITS_PER_CTA;
 constexpr int kUnitMinWeight = 1024;
+// The least weight of a unit, from the number of (strip, column) pairs of the
+// grids and P2G's resident CTAs.  Where the pairs that hold particles (a quarter
+// of the grid in most flows, at most all) about fit the CTAs, a unit is one
+// column: a step of the 4096-particle dam break (195 pairs) takes 28 us against
+// 32, of the slab of 10000 (102 pairs) 29 against 35.  Above that the leading
+// column that every unit stages again costs more than the shorter chain gives (a
+// 0.58M-particle flow: 3 % slower).
+inline int unit_min_weight(long long pairs, int ctas) {
+  return pairs <= 4LL * ctas ? 1 : kUnitMinWeight;
+}
 constexpr int kColWeight = DAMPM_COL_WEIGHT;
 constexpr int kOrderThreads = 1024;
 constexpr int kMaxStrips = 8192;  // strip offsets of the unit list in shared memory
@@ -190,7 +200,7 @@ constexpr int kUnitsPlain = 1, kUnitsHeavy = 2, kUnitCursor = 3, kUnitCounts = 3
 // P2G's unit list -- the plain units from 0, the heavy ones (which P2G takes
 // first) from cap -- with each unit's ledger slot.
 struct UnitPlan {
-  int target_units, cap;
+  int target_units, min_weight, cap;
   int4* ulist;
   int* uslot;
   int* strip_n;  // units of each strip

@@ -1275,6 +1275,7 @@ __device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const
   const int rlo = max(r0 - 1, 0), rhi = min(r0 + kTR - 1, nrows - 1);
   const int lane = threadIdx.x & 31;
   const unsigned T32 = unsigned(T);
+  const long long heavy_from = 2 * max(T, (long long)kUnitMinWeight);
   // floor(p / T): in 32 bits where p allows it (T always does)
   const auto part = [&](long long p) {
     return (unsigned long long)p >> 32 ? p / T : (long long)(unsigned(p) / T32);
@@ -1285,7 +1286,7 @@ __device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const
   int J = 0, n = 0, heavies = 0;  // units flushed, in the buffer, heavy ones among them
   const auto emit = [&](bool ends, int cA, int cB, long long p0, long long p1, int prev) {
     const long long np = p1 - p0 - (long long)col_weight * (min(cB, ncols) - cA) + prev;
-    const bool keep = ends && np > 0, heavy = np > 2 * T;
+    const bool keep = ends && np > 0, heavy = np > heavy_from;
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     if (keep) buf[n + __popc(m & ((1u << lane) - 1u))] = make_int4(cA, cB, heavy ? 1 : 0, 0);
     n += __popc(m);
@@ -1339,9 +1340,9 @@ __device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const
 }
 
 __device__ __forceinline__ long long unit_weight(const Scalars* S,
-                                                 int target_units) {
-  long long T = (long long)S->np / max(target_units, 1);
-  return T < kUnitMinWeight ? kUnitMinWeight : T;
+                                                 const UnitPlan& u) {
+  const long long T = (long long)S->np / max(u.target_units, 1);
+  return T < u.min_weight ? u.min_weight : T;
 }
 
 // The planning warps of the grid, spread over the blocks: warp 0 of each block,
@@ -1387,7 +1388,7 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
   const int w = plan_warp(), nw = (gridDim.x * blockDim.x) >> 5;
   for (int strip = w; strip < strips; strip += nw) {
     if (L <= K)
-      plan_strip(o.start, G, unit_weight(S, u.target_units), strip, unit_buf(sv), u, strip * seg,
+      plan_strip(o.start, G, unit_weight(S, u), strip, unit_buf(sv), u, strip * seg,
                  u.strip_n + strip, kColWeight, L / G.nrows, min(K / G.nrows + 1, G.ncols),
                  [&](int cA, int cB) { return make_int4(strip, cA, cB, 0); });
     else if ((threadIdx.x & 31) == 0)
@@ -2095,7 +2096,7 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
       c_hi = L > H ? -1 : min((H - scn[s].c_off) / G.nrows + 1, G.ncols);
     }
     if (S[s].active && c_hi >= 0)  // (else no particle)
-      plan_strip(o.start + scn[s].c_off, G, unit_weight(Sg, u.target_units), local, unit_buf(sv),
+      plan_strip(o.start + scn[s].c_off, G, unit_weight(Sg, u), local, unit_buf(sv),
                  u, slot0, u.strip_n + b, col_weight, c_lo, c_hi,
                  [&](int cA, int cB) { return make_int4(s, local, cA, cB); });
     else if ((threadIdx.x & 31) == 0)
