@@ -42,7 +42,7 @@ constexpr int kP2GThreads = 128;
 #define DAMPM_P2G_MIN_BLOCKS 4
 #endif
 #ifndef DAMPM_CHAIN_UNROLL
-#define DAMPM_CHAIN_UNROLL 2  // P2G chain steps unrolled per loop trip
+#define DAMPM_CHAIN_UNROLL 2  // single-scenario P2G: chain steps per loop trip
 #endif
 constexpr int kChainUnroll = DAMPM_CHAIN_UNROLL;
 constexpr int kCap = DAMPM_P2G_CAP;

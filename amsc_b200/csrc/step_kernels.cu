@@ -1035,31 +1035,31 @@ __device__ __forceinline__ void chain_step(Chains<R>& a, const P2GSmemT<R>& s, i
 // [a0, a1) and [a1, b1) of the sorted order, walked in order: the first
 // with the upper cell's shape factors, the second with the lower cell's
 // (whose particles the lane's own row counts into the particle ledger).
-template <class R, int kG, bool kFin>
+template <class R, int kG, bool kFin, int kUnroll>
 __device__ __forceinline__ void chain_range(Chains<R>& a, const P2GSmemT<R>& s, int a0,
                                             int a1, int b1, int bb, int be,
                                             const ShapeT<R>& sh, bool own,
                                             double& lp0, double& lp1, double& lp2) {
   const int u1 = min(a1, be);
   int j = max(a0, bb);
-#pragma unroll kChainUnroll
+#pragma unroll kUnroll
   for (; j < u1; ++j) chain_step<R, kG, kFin, true>(a, s, j - bb, sh, false, lp0, lp1, lp2);
   const int j1 = min(b1, be);
   const bool led = kG == 0 && own;
   j = max(a1, bb);
-#pragma unroll kChainUnroll
+#pragma unroll kUnroll
   for (; j < j1; ++j) chain_step<R, kG, kFin, false>(a, s, j - bb, sh, led, lp0, lp1, lp2);
 }
 
-template <class R, int kG>
+template <class R, int kG, int kUnroll>
 __device__ __forceinline__ void chain_group(Chains<R>& a, const P2GSmemT<R>& s, bool lead,
                                             int a0, int a1, int b1, int bb, int be,
                                             const ShapeT<R>& sh, bool own, double& lp0,
                                             double& lp1, double& lp2) {
   if (lead)
-    chain_range<R, kG, false>(a, s, a0, a1, b1, bb, be, sh, own, lp0, lp1, lp2);
+    chain_range<R, kG, false, kUnroll>(a, s, a0, a1, b1, bb, be, sh, own, lp0, lp1, lp2);
   else
-    chain_range<R, kG, true>(a, s, a0, a1, b1, bb, be, sh, own, lp0, lp1, lp2);
+    chain_range<R, kG, true, kUnroll>(a, s, a0, a1, b1, bb, be, sh, own, lp0, lp1, lp2);
 }
 
 // ---- a batch inside one crowded cell ---------------------------------------
@@ -1404,7 +1404,12 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
   }
 }
 
-template <class R>
+// kUnroll: chain steps per loop trip.  Two in the single-scenario kernel (4M
+// particles: 1 % faster than one).  One in a batch: its units are a few short
+// columns, so the four warps' loops keep leaving and entering the instruction
+// cache (at two, 1.9 cycles of every issue wait for an instruction; a pass of 96
+// scenarios takes 156 us at two, 127 at one, 290 at four; in FP32 156 and 100).
+template <class R, int kUnroll>
 __device__ __forceinline__ void p2g_unit(
     const ParticlesT<R>& p, const int* __restrict__ perm,
     const int* __restrict__ cstart, const NodesT<R>& nodes,
@@ -1489,10 +1494,18 @@ __device__ __forceinline__ void p2g_unit(
                     lp0, lp1, lp2);
     } else {
       switch (grp) {
-        case 0: chain_group<R, 0>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2); break;
-        case 1: chain_group<R, 1>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2); break;
-        case 2: chain_group<R, 2>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2); break;
-        default: chain_group<R, 3>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2); break;
+        case 0:
+          chain_group<R, 0, kUnroll>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2);
+          break;
+        case 1:
+          chain_group<R, 1, kUnroll>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2);
+          break;
+        case 2:
+          chain_group<R, 2, kUnroll>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2);
+          break;
+        default:
+          chain_group<R, 3, kUnroll>(a, s, lead, a0, a1, b1, cur.bb, cur.be, sh, own, lp0, lp1, lp2);
+          break;
       }
     }
     if (last_of_col) {
@@ -1574,7 +1587,8 @@ __global__ void __launch_bounds__(kP2GThreads, kP2GMinBlocks)
     __syncthreads();
     if (k >= nunits) break;
     const int f = k < nheavy ? u.cap + k : k - nheavy;
-    p2g_unit(p, perm, cstart, nodes, led_part, G, P, S, record, s, u.uslot[f], u.ulist[f]);
+    p2g_unit<double, kChainUnroll>(p, perm, cstart, nodes, led_part, G, P, S, record, s,
+                                   u.uslot[f], u.ulist[f]);
   }
 }
 
@@ -2134,7 +2148,7 @@ __global__ void __launch_bounds__(kP2GThreads, kP2GMinBlocks)
     const int n_off = scn[u.x].n_off, c_off = scn[u.x].c_off;
     NodesT<R> nd{};
     nd.vvL = vvL + n_off;
-    p2g_unit<R>(p, perm, cstart + c_off, nd, led_part, G, P, &S[u.x], 0, sm,
+    p2g_unit<R, 1>(p, perm, cstart + c_off, nd, led_part, G, P, &S[u.x], 0, sm,
                 up.uslot[f], make_int4(u.y, u.z, u.w, 0));
   }
 }
