@@ -18,7 +18,12 @@ struct Geom {
   double hx, hy;
   double Lx, Ly;  // Nex*hx, Ney*hy (main/optim_par.cpp:557-558)
   int hx_pow2, hy_pow2;  // h is a power of two: v/h == v*(1/h) exactly
-  double ihx, ihy;       // 1/hx, 1/hy (used where h is a power of two)
+  double ihx, ihy;       // 1/hx, 1/hy
+  // division of a cell key in [0, 2^31) by nrows: key * rmul >> rshift, with
+  // rshift = 31 + ceil(log2 nrows) and rmul = 2^rshift / nrows + 1 (T. Granlund,
+  // P. Montgomery, Division by invariant integers using multiplication, 1994)
+  unsigned rmul;
+  int rshift;
   // The part of the grid a slab owns (the whole grid outside slab mode):
   // particles of cell columns [pc_lo, pc_hi), node columns [nc_lo, nc_hi]
   // written by P2G.
@@ -96,22 +101,26 @@ __device__ __forceinline__ int node_of(int inode, int c, int r, int nrows) {
   }
 }
 
+__device__ __forceinline__ int column_of(int key, const Geom& G) {
+  return int(((unsigned long long)(unsigned)key * G.rmul) >> G.rshift);
+}
+
 // Cell (row, col) of a position: floor(y/hy), floor(x/hx), clamped.  Where
 // h is a power of two the quotient equals the product with 1/h exactly
 // (both are the correctly rounded value of the same real number), and the
 // division is skipped.
+// (floor as a conversion: NaN gives 0 or the lowest integer, values beyond the
+// integers the nearest one, so the clamp gives what it gives for the floor)
 __device__ __forceinline__ int cell_index(double f, int n) {
-  if (!(f >= 0.0)) return 0;
-  if (f > double(n - 1)) return n - 1;
-  return int(f);
+  return max(0, min(n - 1, __double2int_rd(f)));
 }
 __device__ __forceinline__ int cell_row(double y, const Geom& G) {
-  if (G.hy_pow2) return cell_index(floor(y * G.ihy), G.nrows);
-  return cell_index(floor(y / G.hy), G.nrows);
+  if (G.hy_pow2) return cell_index(y * G.ihy, G.nrows);
+  return cell_index(y / G.hy, G.nrows);
 }
 __device__ __forceinline__ int cell_col(double x, const Geom& G) {
-  if (G.hx_pow2) return cell_index(floor(x * G.ihx), G.ncols);
-  return cell_index(floor(x / G.hx), G.ncols);
+  if (G.hx_pow2) return cell_index(x * G.ihx, G.ncols);
+  return cell_index(x / G.hx, G.ncols);
 }
 
 // The functions below are templates on the real type R of the particle

@@ -22,6 +22,10 @@ inline Geom make_geom(const dampm_grid& g) {
   G.hy_pow2 = std::frexp(g.hy, &e) == 0.5 ? 1 : 0;
   G.ihx = 1.0 / g.hx;
   G.ihy = 1.0 / g.hy;
+  int L = 0;
+  while ((1LL << L) < g.Ney) ++L;
+  G.rshift = 31 + L;
+  G.rmul = unsigned((1ULL << G.rshift) / unsigned(g.Ney) + 1);
   G.pc_lo = 0;
   G.pc_hi = g.Nex;
   G.nc_lo = 0;

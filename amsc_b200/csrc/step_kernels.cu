@@ -205,6 +205,22 @@ __global__ void k_reduce_state(Particles p, Scalars* S) {
   }
 }
 
+template <class R>
+struct ShapeT {
+  R ihx, mihx, ihy, mihy;
+};
+// 1/h, -1/h: in FP64 the geometry's (the host's quotient is the same value)
+template <class R>
+__device__ __forceinline__ ShapeT<R> shape_of(const Geom& G) {
+  if constexpr (sizeof(R) == 8) {
+    return ShapeT<R>{G.ihx, -G.ihx, G.ihy, -G.ihy};
+  } else {
+    const R ihx = R(1) / R(G.hx), ihy = R(1) / R(G.hy);
+    return ShapeT<R>{ihx, -ihx, ihy, -ihy};
+  }
+}
+using Shape = ShapeT<double>;
+
 // Record of the next P2G for every particle (see Particles): from the stored
 // Ap/Fb/mom (derive == 0: after an upload or a merge/split) or from the state
 // alone (derive != 0), exactly as the reference computes these values
@@ -219,11 +235,11 @@ __device__ __forceinline__ void next_record(const Geom& G, const Phys& P,
                                             R& gx, R& gy) {
   const int r = cell_row(double(y), G);
   const int c = cell_col(double(x), G);
-  const R ihx = R(1) / R(G.hx), ihy = R(1) / R(G.hy);
-  local_xy_g(x, y, c, r, G, ihx, ihy, xi, eta);
+  const ShapeT<R> sh = shape_of<R>(G);
+  local_xy_g(x, y, c, r, G, sh.ihx, sh.ihy, xi, eta);
   // g2pd Z -> dZxp, dZyp (main/optim_par.cpp:387)
-  const double dihx = 1.0 / G.hx, dmihx = -1.0 / G.hx;
-  const double dihy = 1.0 / G.hy, dmihy = -1.0 / G.hy;
+  const double dihx = G.ihx, dmihx = -G.ihx;
+  const double dihy = G.ihy, dmihy = -G.ihy;
   const double dxi = xi, deta = eta;
   double dzx = 0.0, dzy = 0.0;
 #pragma unroll
@@ -928,12 +944,6 @@ __device__ __forceinline__ void nodal_update(
   }
 }
 
-template <class R>
-struct ShapeT {
-  R ihx, mihx, ihy, mihy;
-};
-using Shape = ShapeT<double>;
-
 // s += v.  The FP32 chains are compensated (Kahan): c carries the part of
 // the running sum that the last rounding lost, so a chain of thousands of
 // contributions keeps FP32 precision.  The FP64 chains are the reference's
@@ -1432,7 +1442,7 @@ __device__ __forceinline__ void p2g_unit(
   const bool lane_ok = row < kTR;  // lanes kTR..31 idle
   const bool row_ok = lane_ok && (r <= nrows);
   const double dt = S->dt;
-  const ShapeT<R> sh{R(1) / R(G.hx), -R(1) / R(G.hx), R(1) / R(G.hy), -R(1) / R(G.hy)};
+  const ShapeT<R> sh = shape_of<R>(G);
   // exchange slots of each group's quantities: g0 0-2, g1 3-6, g2 7, g3 8
   const int slot0 = grp == 0 ? 0 : grp == 1 ? 3 : grp == 2 ? 7 : 8;
   const int nq = grp == 0 ? 3 : grp == 1 ? 4 : 1;
@@ -1710,15 +1720,14 @@ __device__ __forceinline__ void g2p_particle(
     const ParticlesT<R>& dst, int j,
     const NodesT<R>& nodes, const double* __restrict__ Z, const Geom& G, const Phys& P,
     const ShapeT<R>& sh, double dtd, int record, int want_grad, int key_off,
-    unsigned long long& m0, unsigned long long& m1, unsigned long long& m2, int& bad,
-    int& nkey) {
+    unsigned long long& m0, unsigned long long& m1, unsigned long long& m2, int& nkey) {
   const int nrows = G.nrows;
   const R ihx = sh.ihx, mihx = sh.mihx;
   const R ihy = sh.ihy, mihy = sh.mihy;
   const R eps = R(1e-10);
   const R dt = R(dtd);
   const int key = key_in - key_off;
-  const int r = key % nrows, c = key / nrows;
+  const int c = column_of(key, G), r = key - c * nrows;
   int nd[4];
   R vxn[4], vyn[4];
 #pragma unroll
@@ -1835,13 +1844,11 @@ __device__ __forceinline__ void g2p_particle(
     dst.Zp[j] = R(zp);
     dst.hpZ[j] = R(double(hp) + zp);
   }
-  m0 = max(m0, ordered_key(double(fabs(vpx))));
-  m1 = max(m1, ordered_key(double(fabs(vpy))));
-  m2 = max(m2, ordered_key(double(hp)));
-  // a diverged particle (NaN/inf anywhere in the state a step carries, or a
-  // negative depth) stops its scenario through the status word
-  bad |= !(isfinite(x) && isfinite(y) && isfinite(vpx) && isfinite(vpy) &&
-           isfinite(hp) && hp >= R(0));
+  // bits of non-negative values: ordered as they are; a value that is not
+  // finite is above all others
+  m0 = max(m0, (unsigned long long)__double_as_longlong(fabs(double(vpx))));
+  m1 = max(m1, (unsigned long long)__double_as_longlong(fabs(double(vpy))));
+  m2 = max(m2, (unsigned long long)__double_as_longlong(double(hp)));
 }
 
 // Copies the moving fields of slot s of src to slot j of dst (a particle
@@ -1884,10 +1891,8 @@ __device__ __forceinline__ void flag_non_finite(int bad, Scalars* S) {
 // Block min/max of the new keys into knext (the scan range of the next
 // sort); all threads of the block call it.
 __device__ __forceinline__ void key_range(int kmin, int kmax, int* sred, Scalars* S) {
-  for (int o = 16; o > 0; o >>= 1) {
-    kmin = min(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
-    kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-  }
+  kmin = __reduce_min_sync(0xffffffffu, kmin);
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
   if ((threadIdx.x & 31) == 0) {
     atomicMin(&sred[0], kmin);
     atomicMax(&sred[1], kmax);
@@ -1899,17 +1904,35 @@ __device__ __forceinline__ void key_range(int kmin, int kmax, int* sred, Scalars
   }
 }
 
+// The maximum over a warp, half by half with the warp's integer reduction (six
+// of them for the three maxima; 64-bit shuffles took about a hundred
+// instructions, a tenth of what a particle takes).
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k) {
+  const unsigned hi = unsigned(k >> 32);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? unsigned(k) : 0u);
+  return ((unsigned long long)mh << 32) | ml;
+}
+
+// A thread's maxima (bits of |vpx|, |vpy|, hp) tell whether one of its particles
+// diverged: a velocity or a depth that is not finite is the maximum, a depth is
+// at least 1e-2 or no number, and a position is not finite only where the
+// velocity is not either (it is clamped to the domain).
+__device__ __forceinline__ bool diverged(unsigned long long m0, unsigned long long m1,
+                                         unsigned long long m2) {
+  return max(m0, max(m1, m2)) >= 0x7ff0000000000000ull;
+}
+constexpr unsigned long long kKeySign = 0x8000000000000000ull;  // ordered_key of a value >= 0
+
 // Block reduction of the CFL maxima into one scenario's next-step slots.
 __device__ __forceinline__ void cfl_block_max(unsigned long long m0,
                                               unsigned long long m1,
                                               unsigned long long m2,
                                               unsigned long long* red,
                                               Scalars* S) {
-  for (int o = 16; o > 0; o >>= 1) {
-    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-    m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-    m2 = max(m2, __shfl_xor_sync(0xffffffffu, m2, o));
-  }
+  m0 = warp_max(m0);
+  m1 = warp_max(m1);
+  m2 = warp_max(m2);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(&red[0], m0);
     atomicMax(&red[1], m1);
@@ -1917,12 +1940,21 @@ __device__ __forceinline__ void cfl_block_max(unsigned long long m0,
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    atomicMax(&S->red_next[0], red[0]);
-    atomicMax(&S->red_next[1], red[1]);
-    atomicMax(&S->red_next[2], red[2]);
+    atomicMax(&S->red_next[0], red[0] | kKeySign);
+    atomicMax(&S->red_next[1], red[1] | kKeySign);
+    atomicMax(&S->red_next[2], red[2] | kKeySign);
   }
 }
 
+// Bound by latency and issue together (32 warps per SM at 64 registers): what
+// takes instructions or registers out of a particle's 900 counts, more loads in
+// flight at the price of either do not (the count's atomic sent early and the next
+// particle's position read ahead: 5 % slower; three blocks per SM without spills:
+// 5 %; five: 3 %).  The maxima kept as bits, which also tell a diverged particle,
+// their reduction by halves, 1/h from the constant bank, the cell's column by a
+// product and the cell by a conversion: 210 -> 196 us at 4M particles (4.6 TB/s
+// on its 900 MB), 22.4 -> 18 at 0.25M.
+//
 // kRecord / kGrad: the output fields and the velocity gradients are
 // written (compiled out of the plain step).  Thread t takes the particle
 // at position ng + t of this step's sorted order: slot perm[ng + t] of
@@ -1957,6 +1989,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     if (threadIdx.x == 0) S->pending = 1;
     return;
   }
+  if (blk * int(blockDim.x) >= n) return;  // (the grid is for the capacity)
   __shared__ unsigned long long red[3];
   __shared__ int kred[2];
   if (threadIdx.x < 3) red[threadIdx.x] = 0ull;
@@ -1966,9 +1999,9 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
   }
   __syncthreads();
   const double dt = S->dt;
-  const Shape sh{1.0 / G.hx, -1.0 / G.hx, 1.0 / G.hy, -1.0 / G.hy};
+  const Shape sh = shape_of<double>(G);
   unsigned long long m0 = 0, m1 = 0, m2 = 0;
-  int bad = 0, kmin = 0x7fffffff, kmax = -1;
+  int kmin = 0x7fffffff, kmax = -1;
   const int lane = threadIdx.x & 31;
   for (int t0 = blk * blockDim.x + (threadIdx.x & ~31); t0 < n; t0 += stride) {
     const int t = t0 + lane;
@@ -1979,7 +2012,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
       const int j = ng + t;
       const int s = perm[j];
       g2p_particle(cur, s, g2p_in(cur, s), skey[j], nxt, t, nodes, Z, G, P, sh, dt,
-                   kRecord ? 1 : 0, kGrad ? 1 : 0, 0, m0, m1, m2, bad, nkey);
+                   kRecord ? 1 : 0, kGrad ? 1 : 0, 0, m0, m1, m2, nkey);
       kmin = min(kmin, nkey);
       kmax = max(kmax, nkey);
       if (leave) {
@@ -1992,6 +2025,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     }
     count_key(nkey, stay, count, tile_sum, nxt.slot + (ok ? t : 0));
   }
+  const bool bad = diverged(m0, m1, m2);
   cfl_block_max(m0, m1, m2, red, S);
   key_range(kmin, kmax, kred, S);
   flag_non_finite(bad, S);
@@ -2214,14 +2248,16 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
   const int n_off = scn[s].n_off, c_off = scn[s].c_off;
   NodesT<R> nd{};
   nd.vvL = const_cast<V2<R>*>(vvL) + n_off;
+  // (by division: as values read with the scenario they would stay in registers
+  // from here on, 136 bytes of spills in place of 32 and 2 % of an ensemble's pass)
   const ShapeT<R> sh{R(1) / R(G.hx), -R(1) / R(G.hx), R(1) / R(G.hy), -R(1) / R(G.hy)};
   unsigned long long m0 = 0, m1 = 0, m2 = 0;
-  int bad = 0;
   if (ok)
     g2p_particle(cur, perm[j], g2p_in(cur, perm[j]), skey[j], nxt, j, nd, Z + n_off, G, P,
                  sh, S[s].dt, 0, 0,
-                 c_off, m0, m1, m2, bad, nkey);
+                 c_off, m0, m1, m2, nkey);
   count_key(nkey, ok, count, tile_sum, nxt.slot + (ok ? j : 0));
+  const bool bad = diverged(m0, m1, m2);
   cfl_block_max(m0, m1, m2, red, &S[s]);
   key_range(ok ? nkey : 0x7fffffff, ok ? nkey : -1, kred, &S[s]);
   flag_non_finite(bad, &S[s]);
