@@ -499,13 +499,34 @@ __device__ __forceinline__ void roll_keys(Scalars* S) {
 // Sorted position start[key] + slot takes the storage slot, the reference index
 // and the key (the cell of each sorted position, which G2P reads without waiting
 // for perm); inside a cell they lie as the count's atomics came.
+// kScatterPer particles per thread and trip: their loads, and then those of
+// their starts, are on the way together (4M particles: 21 us, one at a time 27; 24 B
+// a particle and the starts, which take 16).
+constexpr int kScatterPer = 4;
 __device__ __forceinline__ void scatter(const Binning& n, const int* start, int np) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const int k = n.key[i];
-    const int pos = start[k] + n.slot[i];
-    n.sslot[pos] = i;
-    n.sidx[pos] = n.idx[i];
-    n.skey[pos] = k;
+  const int stride = gridDim.x * blockDim.x;
+  for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < np; i0 += kScatterPer * stride) {
+    int key[kScatterPer], slot[kScatterPer], idx[kScatterPer];
+#pragma unroll
+    for (int u = 0; u < kScatterPer; ++u) {
+      const long long i = i0 + (long long)u * stride;
+      key[u] = -1;
+      if (i < np) {
+        key[u] = n.key[i];
+        slot[u] = n.slot[i];
+        idx[u] = n.idx[i];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kScatterPer; ++u)
+      if (key[u] >= 0) slot[u] += start[key[u]];
+#pragma unroll
+    for (int u = 0; u < kScatterPer; ++u)
+      if (key[u] >= 0) {
+        n.sslot[slot[u]] = i0 + u * stride;
+        n.sidx[slot[u]] = idx[u];
+        n.skey[slot[u]] = key[u];
+      }
   }
 }
 
