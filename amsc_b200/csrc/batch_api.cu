@@ -92,7 +92,7 @@ struct dampm_batch {
   int p2g_grid = 1;
   long long launches = 0;
   // tuning: P2G units per CTA and the weight of a column in the unit plan
-  int units_per_cta = kUnitsPerCta, col_weight = kColWeight;
+  int units_per_cta = kBatchUnitsPerCta, col_weight = kColWeight;
   // kBatchGraphPasses passes captured in a CUDA graph, replayed while the
   // layout holds; one graph per half the passes start from
   int use_graphs = 1;

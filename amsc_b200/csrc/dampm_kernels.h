@@ -20,6 +20,10 @@ constexpr int kTR = 30;
 #define DAMPM_COL_WEIGHT 192
 #endif
 constexpr int kUnitsPerCta = DAMPM_UNITS_PER_CTA;
+// A batch's columns are short (120 particles in 30 rows at 4 per cell), so the
+// leading column that each unit stages again weighs more than an even load: a pass
+// of 96 scenarios takes 229 us at one unit per CTA, 237 at two (FP32 201 and 209).
+constexpr int kBatchUnitsPerCta = 1;
 constexpr int kUnitMinWeight = 1024;
 // The least weight of a unit, from the number of (strip, column) pairs of the
 // grids and P2G's resident CTAs.  Where the pairs that hold particles (a quarter
