@@ -41,7 +41,7 @@ class Batch:
             raise DampmError(f"dampm_batch_create failed ({rc})")
         self.h = h
         self.np: Dict[int, int] = {}
-        self._tuning = (1, 192)  # the library's defaults
+        self._tuning = (2, 192)  # what autotune starts from: the even load of a large batch
 
     def _check(self, rc: int):
         if rc != 0:
