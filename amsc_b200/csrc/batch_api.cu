@@ -465,7 +465,7 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   // cells of all scenarios: fewer than their nodes
   rc = rc ? rc : balloc(b, &b->count, nn + 4);
   rc = rc ? rc : balloc(b, &b->start, nn + 1);
-  rc = rc ? rc : balloc(b, &b->tile_sum, nn / kScanTile + 2);
+  rc = rc ? rc : balloc(b, &b->tile_sum, (nn / kScanTile + 2) * kTileStride);
   rc = rc ? rc : balloc(b, &b->tflag, nn / kScanTile + 2);
   rc = rc ? rc : balloc(b, &b->perm, pc);
   rc = rc ? rc : balloc(b, &b->skey, pc);
@@ -519,7 +519,7 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   }
   if (rc == DAMPM_OK) {
     cudaMemsetAsync(b->count, 0, sizeof(int) * (nn + 4), b->stream);
-    cudaMemsetAsync(b->tile_sum, 0, sizeof(int) * (nn / kScanTile + 2), b->stream);
+    cudaMemsetAsync(b->tile_sum, 0, sizeof(int) * kTileStride * (nn / kScanTile + 2), b->stream);
     cudaMemsetAsync(b->vvL, 0, 2 * rsz * nn, b->stream);
     cudaMemsetAsync(b->S, 0, sizeof(Scalars) * size_t(scenario_cap), b->stream);
     cudaMemsetAsync(b->Sg, 0, sizeof(Scalars), b->stream);
@@ -686,7 +686,8 @@ int dampm_batch_compact(dampm_batch* b) {
   // beyond the new total may hold counts of removed scenarios, which a later
   // scenario's cells would otherwise inherit)
   BCK(cudaMemsetAsync(b->count, 0, sizeof(int) * size_t(b->N_cap + 4), b->stream));
-  BCK(cudaMemsetAsync(b->tile_sum, 0, sizeof(int) * size_t(b->N_cap / kScanTile + 2), b->stream));
+  BCK(cudaMemsetAsync(b->tile_sum, 0, sizeof(int) * kTileStride * size_t(b->N_cap / kScanTile + 2),
+                      b->stream));
   if (!mv.empty()) {
     BCK(cudaMemcpyAsync(b->mblk, mv.data(), sizeof(int4) * mv.size(),
                         cudaMemcpyHostToDevice, b->stream));

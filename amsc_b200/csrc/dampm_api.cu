@@ -698,7 +698,7 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   ctx->ntiles = (ctx->nc + kScanTile - 1) / kScanTile;
   rc = rc ? rc : dalloc(ctx, &ctx->count, size_t(ctx->nc) + 4);
   rc = rc ? rc : dalloc(ctx, &ctx->start, size_t(ctx->nc) + 1);
-  rc = rc ? rc : dalloc(ctx, &ctx->tile_sum, size_t(ctx->ntiles) + 1);
+  rc = rc ? rc : dalloc(ctx, &ctx->tile_sum, (size_t(ctx->ntiles) + 1) * kTileStride);
   ctx->strips = (grid->Ney + 1 + kTR - 1) / kTR;
   ctx->useg = grid->Nex + 1;
   ctx->n_led = ctx->strips * ctx->useg;  // most units a step can list
@@ -716,7 +716,8 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   }
   if (rc == DAMPM_OK) {
     cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream);
-    cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * size_t(ctx->ntiles), ctx->stream);
+    cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * kTileStride * size_t(ctx->ntiles),
+                     ctx->stream);
     cudaMemsetAsync(ctx->ucount, 0, sizeof(int) * 8, ctx->stream);
     cudaMemsetAsync(ctx->nodes.vvL, 0, sizeof(double2) * nn, ctx->stream);
     cudaMemsetAsync(ctx->S, 0, sizeof(Scalars), ctx->stream);
@@ -807,7 +808,8 @@ int dampm_upload_particles(dampm_ctx* ctx, long long np, const double* x,
   CK(cudaMemcpyAsync(ctx->S, ctx->Sh, sizeof(Scalars), cudaMemcpyHostToDevice,
                      ctx->stream));
   CK(cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream));
-  CK(cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * size_t(ctx->ntiles), ctx->stream));
+  CK(cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * kTileStride * size_t(ctx->ntiles),
+                     ctx->stream));
   if (np > 0) {
     // the slots hold the particles in DATA order (idx = slot)
     launch_init_particles<double>(grid_for(np, 256), 256, ctx->stream, p, ctx->Z,
@@ -1112,7 +1114,8 @@ int dampm_set_state(dampm_ctx* ctx, long long np, const double* const* fields,
                      ctx->stream));
   // the slots now hold the particles in reference order
   CK(cudaMemsetAsync(ctx->count, 0, sizeof(int) * ctx->nc, ctx->stream));
-  CK(cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * size_t(ctx->ntiles), ctx->stream));
+  CK(cudaMemsetAsync(ctx->tile_sum, 0, sizeof(int) * kTileStride * size_t(ctx->ntiles),
+                     ctx->stream));
   k_keys<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p, ctx->G, ctx->S, 1);
   k_count_n<<<grid_for(np, 256), 256, 0, ctx->stream>>>(p.key, ctx->count, tile_totals(ctx),
                                                            p.slot, int(np));

@@ -57,6 +57,10 @@ constexpr int kG2PThreads = 256;
 #endif
 constexpr int kG2PMinBlocks = DAMPM_G2P_MIN_BLOCKS;
 constexpr int kScanTile = 4096;
+// Tile totals lie apart: the atomics that count a flow's few dozen tiles would
+// queue at one or two lines of L2 (the count of 1M uploaded particles: 16 us side by
+// side, 10 a sector apart).
+constexpr int kTileStride = 8;
 constexpr int kScanThreads = 1024;
 constexpr int kSmallCells = 4 * kScanTile;  // grids that k_scan_scatter takes
 

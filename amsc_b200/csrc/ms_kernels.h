@@ -43,7 +43,7 @@ int ms_alloc(MsBuffers& m, long long cap, int /*ncells*/, Alloc alloc) {
     int rc = alloc((void**)q, sizeof(int) * size_t(cap + 1));
     if (rc) return rc;
   }
-  int rc = alloc((void**)&m.tile_sum, sizeof(int) * size_t(m.ntiles + 1));
+  int rc = alloc((void**)&m.tile_sum, sizeof(int) * size_t(m.ntiles + 1) * kTileStride);
   if (rc) return rc;
   rc = alloc((void**)&m.stage, sizeof(double) * size_t(cap));
   if (rc) return rc;

@@ -309,9 +309,9 @@ __device__ __forceinline__ void count_key(int k, bool ok, int* __restrict__ coun
     const int first = __ffs(who) - 1, t = kk / kScanTile;
     const int t0 = __shfl_sync(0xffffffffu, t, first & 31);
     if (__all_sync(0xffffffffu, !ok || t == t0)) {
-      if (lane == first) atomicAdd(&tile_sum[t], __popc(who));
+      if (lane == first) atomicAdd(&tile_sum[t * kTileStride], __popc(who));
     } else if (ok && lane == leader) {
-      atomicAdd(&tile_sum[t], __popc(peers));
+      atomicAdd(&tile_sum[t * kTileStride], __popc(peers));
     }
   }
   base = __shfl_sync(0xffffffffu, base, leader);
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kScanThreads)
   __shared__ int wsum[32];
   const int4 c = load_count4(count, t * kScanTile + threadIdx.x * 4, n);
   const int tot = block_sum(c.x + c.y + c.z + c.w, wsum);
-  if (threadIdx.x == 0) tile_sum[t] = tot;
+  if (threadIdx.x == 0) tile_sum[t * kTileStride] = tot;
 }
 
 // Appends a thread's crowded cells among i0 .. i0+3 (of cv particles) to `big`.
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kScanThreads)
   __shared__ int wsum[32];
   // particles in the range's tiles before this one
   int pre = 0;
-  for (int q = t0 + threadIdx.x; q < t; q += blockDim.x) pre += tile_sum[q];
+  for (int q = t0 + threadIdx.x; q < t; q += blockDim.x) pre += tile_sum[q * kTileStride];
   pre = block_sum(pre, wsum);
   const int i0 = t * kScanTile + threadIdx.x * 4;
   const int4 c = load_count4(count, i0, n);
@@ -537,7 +537,7 @@ __global__ void k_scatter(Binning n, const int* __restrict__ start, int* __restr
   if (!gate_open(S, gate)) return;
   scatter(n, start, S->np);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
-    tile_sum[t] = 0;
+    tile_sum[t * kTileStride] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) roll_keys(S);
 }
 
@@ -1301,6 +1301,7 @@ __device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const
                                            long long T, int strip, int4* buf, const UnitPlan& u,
                                            int slot0, int* strip_n, int col_weight, int c_lo,
                                            int c_hi, Make make) {
+  col_weight = min(col_weight, 1 << 25);
   const int nrows = G.nrows, ncols = G.ncols;
   const int r0 = strip * kTR;
   const int rlo = max(r0 - 1, 0), rhi = min(r0 + kTR - 1, nrows - 1);
@@ -1332,24 +1333,32 @@ __device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const
   int oA = c_lo, oV = c_lo > 0 ? column_count(cstart, rlo, rhi, c_lo - 1, nrows) : 0;
   long long oP = 0, carry = 0;
   int last = oV;  // particles of the column before the tile
-  int next = column(c_lo + lane), next2 = column(c_lo + 32 + lane);
+  // counts of the tiles to come, on the way
+  int n0 = column(c_lo + lane), n1 = column(c_lo + 32 + lane), n2 = column(c_lo + 64 + lane);
+  long long last_id = 0;  // part() of the column before the tile
   for (int base = c_lo; base <= c_hi; base += 32) {
     const int nc = base + lane;
-    const int cnt = next;
-    next = next2;
-    next2 = column(nc + 64);
-    const long long w = nc <= c_hi && nc < ncols ? (long long)cnt + col_weight : 0;
-    long long incl = w;
+    const int cnt = n0;
+    n0 = n1;
+    n1 = n2;
+    n2 = column(nc + 96);
+    // (32 bits hold a tile: fewer than 2^31 particles and 32 bounded weights)
+    const unsigned w = nc <= c_hi && nc < ncols ? unsigned(cnt) + col_weight : 0;
+    unsigned incl = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const long long t = __shfl_up_sync(0xffffffffu, incl, o);
+      const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
     const long long pex = carry + incl - w;
     int prev = __shfl_up_sync(0xffffffffu, cnt, 1);
-    if (lane == 0) prev = last;
-    const bool starts = nc > c_lo && nc <= c_hi && nc < ncols &&
-                        part(pex) != part(pex - prev - col_weight);
+    const long long id = part(pex);
+    long long id_prev = __shfl_up_sync(0xffffffffu, id, 1);
+    if (lane == 0) {
+      prev = last;
+      id_prev = last_id;
+    }
+    const bool starts = nc > c_lo && nc <= c_hi && nc < ncols && id != id_prev;
     const unsigned m = __ballot_sync(0xffffffffu, starts);
     if (m) {
       const unsigned below = m & ((1u << lane) - 1u);
@@ -1364,6 +1373,7 @@ __device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const
     }
     carry += __shfl_sync(0xffffffffu, incl, 31);
     last = __shfl_sync(0xffffffffu, cnt, 31);
+    last_id = __shfl_sync(0xffffffffu, id, 31);
   }
   emit(lane == 0, oA, c_hi + 1, oP, carry, oV);
   if (n > 0) flush_units(u, buf, n, heavies, slot0 + J, make);
