@@ -264,7 +264,7 @@ int enqueue_pass(dampm_batch* b) {
   k_b_step_begin<<<1 + grid_blocks(ntiles, 256), 256, 0, st>>>(b->scn, b->S, nscn, b->Sg,
                                                                 b->tflag, ntiles);
   const Gate gate = kGateBegun;
-  k_scan_apply<<<ntiles, kScanThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->start, b->cbig,
+  k_scan_apply<<<ntiles, kApplyThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->start, b->cbig,
                                                 b->ucount, b->Sg, gate, 0, b->tflag);
   const Binning n{key, slot, idx, b->sslot, b->sidx, b->skey};
   k_scatter<<<gp, 256, 0, st>>>(n, b->start, b->tile_sum, ntiles, b->Sg, gate);

@@ -273,7 +273,7 @@ void enqueue_sort(dampm_ctx* ctx, int begun, bool units) {
                      ctx->stream>>>(ctx->count, ctx->nc, ctx->start, ctx->cbig, ctx->ucount, n,
                                     ctx->S, gate);
   } else {
-    k_scan_apply<<<ctx->ntiles, kScanThreads, 0, ctx->stream>>>(
+    k_scan_apply<<<ctx->ntiles, kApplyThreads, 0, ctx->stream>>>(
         ctx->count, ctx->nc, ctx->tile_sum, ctx->start, ctx->cbig, ctx->ucount, ctx->S, gate, 1,
         nullptr);
     k_scatter<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(n, ctx->start, ctx->tile_sum,

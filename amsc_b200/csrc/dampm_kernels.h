@@ -62,6 +62,7 @@ constexpr int kScanTile = 4096;
 // side, 10 a sector apart).
 constexpr int kTileStride = 8;
 constexpr int kScanThreads = 1024;
+constexpr int kApplyThreads = 256, kApplyRows = kScanTile / (4 * kApplyThreads);
 constexpr int kSmallCells = 4 * kScanTile;  // grids that k_scan_scatter takes
 
 // Two values of R side by side (one 16-byte load in FP64, 8 in FP32).

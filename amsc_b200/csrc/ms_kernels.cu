@@ -791,7 +791,7 @@ int grid_for(long long n, int threads) {
 int scan_enqueue(int* a, int* out, int n, int* tile_sum, int ntiles,
                  const Scalars* S, cudaStream_t st) {
   k_scan_sums<<<ntiles, kScanThreads, 0, st>>>(a, n, tile_sum, S);
-  k_scan_apply<<<ntiles, kScanThreads, 0, st>>>(a, n, tile_sum, out, nullptr, nullptr, S,
+  k_scan_apply<<<ntiles, kApplyThreads, 0, st>>>(a, n, tile_sum, out, nullptr, nullptr, S,
                                                 kGateBegun, 0, nullptr);
   return 2;
 }
