@@ -1300,6 +1300,7 @@ __device__ __forceinline__ int column_count(const int* __restrict__ cstart,
 // the block and a flat list by the last block, this took 8 us at 4096 particles,
 // 12 at 4M and 30 for the 800 strips of a batch of 96 scenarios, all of it on the
 // way to P2G; by warps it runs beside the ordering (below).
+constexpr int kPlanShare = 8;  // at most one block in so many plans
 constexpr int kUnitBuf = int(2 * sizeof(unsigned long long) * kBigRun / sizeof(int4)) /
                          (kOrderThreads / 32);
 
@@ -1420,19 +1421,28 @@ __device__ __forceinline__ long long unit_weight(const Scalars* S,
   return T < u.min_weight ? u.min_weight : T;
 }
 
-// The planning warps of the grid, spread over the blocks: warp 0 of each block,
-// then warp 1 ...
-__device__ __forceinline__ int plan_warp() {
-  return int(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+// Who plans and who orders: the first plan_blocks() blocks plan, four warps each
+// where that is enough, and the others order -- beside the ordering's busy warps a
+// planning warp got an eighth of its scheduler's issue slots and was the last to
+// finish (a step of the 4096-particle dam break 0.6 us longer, of 4M particles 4).
+// In a grid of few blocks the first one does both.
+__device__ __forceinline__ int plan_blocks(int strips) {
+  return min(int(gridDim.x) / kPlanShare, (strips + 3) / 4);
 }
-// The order inside the cells is the other warps' (everyone's where that leaves
-// fewer than half).
-__device__ __forceinline__ void order_share(const CellOrder& o, int np, int w, int strips, int nw,
+// this warp's first strip and the step to its next one
+__device__ __forceinline__ int2 plan_share(int strips) {
+  const int nb = plan_blocks(strips), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (nb == 0) return make_int2(blockIdx.x == 0 ? w : strips, nw);
+  return make_int2(int(blockIdx.x) < nb ? w * nb + int(blockIdx.x) : strips, nb * nw);
+}
+__device__ __forceinline__ void order_share(const CellOrder& o, int np, int strips,
                                             unsigned long long* sv) {
   static_assert(kOrderWin * sizeof(int) <= kUnitBuf * sizeof(int4), "");
   int* win = reinterpret_cast<int*>(reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf);
-  const int planners = 2 * strips <= nw ? strips : 0;
-  if (w >= planners) order_cells(o, np, w - planners, nw - planners, win);
+  const int nb = plan_blocks(strips), nw = blockDim.x >> 5;
+  const int b = int(blockIdx.x) - nb;
+  if (b >= 0)
+    order_cells(o, np, b * nw + int(threadIdx.x >> 5), (int(gridDim.x) - nb) * nw, win);
 }
 __device__ __forceinline__ int4* unit_buf(unsigned long long* sv) {
   return reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf;
@@ -1460,8 +1470,8 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
   // node columns of the cells the particles are binned to (the key range the
   // scatter just rolled over), plus the column right of them
   const int L = S->krange[0], K = S->krange[1];
-  const int w = plan_warp(), nw = (gridDim.x * blockDim.x) >> 5;
-  for (int strip = w; strip < strips; strip += nw) {
+  const int2 share = plan_share(strips);
+  for (int strip = share.x; strip < strips; strip += share.y) {
     if (L <= K)
       plan_strip(o.start, G, unit_weight(S, u), strip, unit_buf(sv), u, strip * seg,
                  u.strip_n + strip, kColWeight, L / G.nrows, min(K / G.nrows + 1, G.ncols),
@@ -1469,7 +1479,7 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
     else if ((threadIdx.x & 31) == 0)
       u.strip_n[strip] = 0;
   }
-  order_share(o, S->np, w, strips, nw, sv);
+  order_share(o, S->np, strips, sv);
   __syncthreads();  // the shared memory is free again
   order_crowded(o, sv);
   if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;
@@ -2193,8 +2203,8 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
                     int col_weight) {
   if (!Sg->active) return;
   extern __shared__ unsigned long long sv[];
-  const int w = plan_warp(), nw = (gridDim.x * blockDim.x) >> 5;
-  for (int b = w; b < strips; b += nw) {
+  const int2 share = plan_share(strips);
+  for (int b = share.x; b < strips; b += share.y) {
     const int s = strip_scn[b];
     const Geom G = scn[s].G;
     const int local = b - scn[s].strip_off;
@@ -2215,7 +2225,7 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
     else if ((threadIdx.x & 31) == 0)
       u.strip_n[b] = 0;
   }
-  order_share(o, Sg->np, w, strips, nw, sv);
+  order_share(o, Sg->np, strips, sv);
   __syncthreads();  // the shared memory is free again
   order_crowded(o, sv);
   if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;
