@@ -1300,7 +1300,6 @@ __device__ __forceinline__ int column_count(const int* __restrict__ cstart,
 // the block and a flat list by the last block, this took 8 us at 4096 particles,
 // 12 at 4M and 30 for the 800 strips of a batch of 96 scenarios, all of it on the
 // way to P2G; by warps it runs beside the ordering (below).
-constexpr int kPlanShare = 8;  // at most one block in so many plans
 constexpr int kUnitBuf = int(2 * sizeof(unsigned long long) * kBigRun / sizeof(int4)) /
                          (kOrderThreads / 32);
 
@@ -1421,28 +1420,41 @@ __device__ __forceinline__ long long unit_weight(const Scalars* S,
   return T < u.min_weight ? u.min_weight : T;
 }
 
-// Who plans and who orders: the first plan_blocks() blocks plan, four warps each
-// where that is enough, and the others order -- beside the ordering's busy warps a
-// planning warp got an eighth of its scheduler's issue slots and was the last to
-// finish (a step of the 4096-particle dam break 0.6 us longer, of 4M particles 4).
-// In a grid of few blocks the first one does both.
+// Who plans and who orders: the first plan_blocks() blocks plan, four warps each,
+// and the others order -- beside the ordering's busy warps a planning warp got an
+// eighth of its scheduler's issue slots and was the last to finish (a step of the
+// 4096-particle dam break 0.6 us longer, of 4M particles 4).  Where that would take
+// more than one block in kPlanShare (a batch of many scenarios, or a grid of few
+// blocks) the strips are spread over the blocks, warp 0 of each, then warp 1 ...,
+// and the other warps order (everyone where that leaves fewer than half): 11 us
+// against 15 with the 800 strips of 96 scenarios.
+constexpr int kPlanShare = 4;
 __device__ __forceinline__ int plan_blocks(int strips) {
-  return min(int(gridDim.x) / kPlanShare, (strips + 3) / 4);
+  const int nb = (strips + 3) / 4;
+  return nb <= int(gridDim.x) / kPlanShare ? nb : 0;
 }
 // this warp's first strip and the step to its next one
 __device__ __forceinline__ int2 plan_share(int strips) {
   const int nb = plan_blocks(strips), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (nb == 0) return make_int2(blockIdx.x == 0 ? w : strips, nw);
-  return make_int2(int(blockIdx.x) < nb ? w * nb + int(blockIdx.x) : strips, nb * nw);
+  const int over = nb ? nb : gridDim.x;
+  return make_int2(int(blockIdx.x) < over ? w * over + int(blockIdx.x) : strips, over * nw);
 }
 __device__ __forceinline__ void order_share(const CellOrder& o, int np, int strips,
                                             unsigned long long* sv) {
   static_assert(kOrderWin * sizeof(int) <= kUnitBuf * sizeof(int4), "");
   int* win = reinterpret_cast<int*>(reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf);
-  const int nb = plan_blocks(strips), nw = blockDim.x >> 5;
-  const int b = int(blockIdx.x) - nb;
-  if (b >= 0)
-    order_cells(o, np, b * nw + int(threadIdx.x >> 5), (int(gridDim.x) - nb) * nw, win);
+  const int nb = plan_blocks(strips), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int first, all;  // this warp's place among those that order
+  if (nb > 0) {
+    first = (int(blockIdx.x) - nb) * nw + w;
+    all = (int(gridDim.x) - nb) * nw;
+  } else {
+    all = int(gridDim.x) * nw;
+    const int planners = 2 * strips <= all ? strips : 0;
+    first = w * int(gridDim.x) + int(blockIdx.x) - planners;
+    all -= planners;
+  }
+  if (first >= 0) order_cells(o, np, first, all, win);
 }
 __device__ __forceinline__ int4* unit_buf(unsigned long long* sv) {
   return reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf;
