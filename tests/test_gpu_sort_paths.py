@@ -24,9 +24,14 @@ def _scenario(ney, nex, h=0.5):
     rng = np.random.default_rng(ney * 7919 + nex)
     n = min(4 * len(SIZES), ney * nex)
     cells = np.unique(np.concatenate([[0, ney * nex - 1], rng.integers(0, ney * nex, n)]))
+    return _data(ney, nex, h, rng, [(c, SIZES[k % len(SIZES)])
+                                    for k, c in enumerate(rng.permutation(cells))])
+
+
+def _data(ney, nex, h, rng, cells):
+    """m particles in each cell c of (c, m), in random order."""
     x, y, ap = [], [], []
-    for k, c in enumerate(rng.permutation(cells)):
-        m = SIZES[k % len(SIZES)]
+    for c, m in cells:
         x.append((c // ney + rng.uniform(0.02, 0.98, m)) * h)
         y.append((c % ney + rng.uniform(0.02, 0.98, m)) * h)
         ap.append(np.full(m, h * h / m))
@@ -46,7 +51,20 @@ def _scenario(ney, nex, h=0.5):
 @pytest.mark.parametrize("ney,nex", [(1, 1), (1, 40), (61, 5), (64, 64), (128, 128), (127, 130),
                                      (16384, 1), (16400, 1), (2, 8300)])
 def test_sort_and_units_on_every_path(cuda_lib, ney, nex):
-    d = _scenario(ney, nex)
+    _check(_scenario(ney, nex))
+
+
+@pytest.mark.parametrize("ney,nex", [(8, 600), (100, 300)])
+def test_units_beyond_the_planner_s_buffer(cuda_lib, ney, nex):
+    """Every column holds particles and is a unit of its own: a strip's units are
+    appended to the list in several pieces, a crowded column among the heavy ones."""
+    rng = np.random.default_rng(nex)
+    cells = [(c, 1) for c in range(ney * nex)]
+    cells[ney * (nex // 2)] = (ney * (nex // 2), 2500)
+    _check(_data(ney, nex, 0.5, rng, cells))
+
+
+def _check(d):
     steps = 6
     o = Oracle(d, threads=2)
     o.run(steps)
