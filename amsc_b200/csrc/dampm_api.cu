@@ -279,10 +279,10 @@ void enqueue_sort(dampm_ctx* ctx, int begun, bool units) {
     k_scatter<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(n, ctx->start, ctx->tile_sum,
                                                                 ctx->ntiles, ctx->S, gate);
   }
-  k_order_units<<<order_blocks(ctx->cap), kOrderThreads, order_smem_bytes(), ctx->stream>>>(
-      CellOrder{n, ctx->start, ctx->cbig, ctx->ucount, ctx->perm, ctx->sortbuf, ctx->cap,
-                ctx->count, small ? ctx->nc : 0},
-      unit_plan(ctx), ctx->G, ctx->P, ctx->S, strips, ctx->useg, gate);
+  launch_order_units(order_blocks(ctx->cap), ctx->stream,
+                     CellOrder{n, ctx->start, ctx->cbig, ctx->ucount, ctx->perm, ctx->sortbuf,
+                               ctx->cap, ctx->count, small ? ctx->nc : 0},
+                     unit_plan(ctx), ctx->G, ctx->P, ctx->S, strips, ctx->useg, gate, ctx->slab);
   ctx->launches += small ? 2 : 3;
 }
 

@@ -219,8 +219,9 @@ struct UnitPlan {
 // list (seg: unit slots per strip) and ends the step before and begins this
 // one unless it has begun.  order_smem_bytes(): its dynamic shared memory;
 // setup_sort sets the sort kernels' limits (0 on failure)
-__global__ void k_order_units(CellOrder o, UnitPlan u, Geom G, Phys P, Scalars* S, int strips,
-                              int seg, Gate gate);
+// repeats: reference indices may repeat inside a cell
+void launch_order_units(int grid, cudaStream_t st, const CellOrder& o, const UnitPlan& u, Geom G,
+                        Phys P, Scalars* S, int strips, int seg, Gate gate, bool repeats);
 size_t order_smem_bytes();
 int setup_sort();
 // blocks of 1024 threads for np particles, one per SM at most

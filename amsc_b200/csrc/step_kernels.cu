@@ -619,12 +619,16 @@ __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
-// The order inside the cells, by the particles' reference index (unique; the
-// atomics of the count hand out a cell's places in arbitrary order): a
-// position's particle goes to the place its index has among those of its cell,
-// counted over the cell's indices.  A warp takes tiles of kOrderPer positions per
-// lane, with the indices of all their cells in its part `win` of the shared
-// memory (no more than kCrowded before and behind the tile): the lanes lie in a
+// The order inside the cells, by the particles' reference index (the atomics of
+// the count hand out a cell's places in arbitrary order): a position's particle
+// goes to the place its index has among those of its cell, counted over the
+// cell's indices.  The indices are unique -- two particles with the same one
+// would take the same place, and the place behind it none -- except in a slab,
+// whose caller numbers the particles: there (kRepeats) equal indices follow in
+// the order of their storage slots, as in order_crowded.
+// A warp takes tiles of kOrderPer positions per lane, with the indices of all
+// their cells in its part `win` of the shared memory (no more than kCrowded
+// before and behind the tile): the lanes lie in a
 // few cells and mostly read the same word, and no warp waits for another.
 // Warp w of nw takes every nw-th tile.
 // Before, a lane sorted a cell of up to 16 particles in registers and a warp a
@@ -635,6 +639,7 @@ __global__ void __launch_bounds__(kScanThreads)
 // particles, this way 42; 24 B a particle, which take 15 us).
 constexpr int kOrderPer = 4;
 constexpr int kOrderWin = 32 * kOrderPer + 2 * kCrowded;
+template <bool kRepeats>
 __device__ __forceinline__ void order_cells(const CellOrder& o, int np, int w, int nw, int* win) {
   const int lane = threadIdx.x & 31;
   const int per = max(1, min(kOrderPer, np / (32 * nw)));
@@ -684,8 +689,14 @@ __device__ __forceinline__ void order_cells(const CellOrder& o, int np, int w, i
       const int mine = win[p0 + u * 32 - lo];
       const int* v = win + (b[u] - lo);
       int rank = 0;
+      if constexpr (kRepeats) {  // by index, then by storage slot
+        const int* s = o.n.sslot + b[u];
+        for (int i = 0; i < n; ++i)
+          rank += v[i] < mine || (v[i] == mine && s[i] < slot[u]) ? 1 : 0;
+      } else {
 #pragma unroll 4
-      for (int i = 0; i < n; ++i) rank += v[i] < mine ? 1 : 0;
+        for (int i = 0; i < n; ++i) rank += v[i] < mine ? 1 : 0;
+      }
       o.perm[b[u] + rank] = slot[u];
     }
     __syncwarp();  // the window is free
@@ -1439,6 +1450,7 @@ __device__ __forceinline__ int2 plan_share(int strips) {
   const int over = nb ? nb : gridDim.x;
   return make_int2(int(blockIdx.x) < over ? w * over + int(blockIdx.x) : strips, over * nw);
 }
+template <bool kRepeats>
 __device__ __forceinline__ void order_share(const CellOrder& o, int np, int strips,
                                             unsigned long long* sv) {
   static_assert(kOrderWin * sizeof(int) <= kUnitBuf * sizeof(int4), "");
@@ -1454,7 +1466,7 @@ __device__ __forceinline__ void order_share(const CellOrder& o, int np, int stri
     first = w * int(gridDim.x) + int(blockIdx.x) - planners;
     all -= planners;
   }
-  if (first >= 0) order_cells(o, np, first, all, win);
+  if (first >= 0) order_cells<kRepeats>(o, np, first, all, win);
 }
 __device__ __forceinline__ int4* unit_buf(unsigned long long* sv) {
   return reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf;
@@ -1471,6 +1483,7 @@ __device__ __forceinline__ int4* unit_buf(unsigned long long* sv) {
 // to wait for its stores before it counts itself done (7 us at 0.25M and 4M
 // particles).
 // strips = 0: the sort alone (before a merge/split); seg: unit slots per strip
+template <bool kRepeats>
 __global__ void __launch_bounds__(kOrderThreads, 1)
     k_order_units(CellOrder o, UnitPlan u, Geom G, Phys P, Scalars* S, int strips, int seg,
                   Gate gate) {
@@ -1491,7 +1504,7 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
     else if ((threadIdx.x & 31) == 0)
       u.strip_n[strip] = 0;
   }
-  order_share(o, S->np, strips, sv);
+  order_share<kRepeats>(o, S->np, strips, sv);
   __syncthreads();  // the shared memory is free again
   order_crowded(o, sv);
   if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;
@@ -1692,12 +1705,19 @@ __global__ void __launch_bounds__(kP2GThreads, kP2GMinBlocks)
 size_t order_smem_bytes() { return 2 * sizeof(unsigned long long) * kBigRun; }
 
 int setup_sort() {
-  for (const void* f : {(const void*)k_order_units, (const void*)k_b_order_units})
+  for (const void* f : {(const void*)k_order_units<false>, (const void*)k_order_units<true>,
+                        (const void*)k_b_order_units})
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              int(order_smem_bytes())) != cudaSuccess)
       return 0;
   return cudaFuncSetAttribute(k_scan_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               int(sizeof(int)) * kSmallCells) == cudaSuccess;
+}
+
+void launch_order_units(int grid, cudaStream_t st, const CellOrder& o, const UnitPlan& u, Geom G,
+                        Phys P, Scalars* S, int strips, int seg, Gate gate, bool repeats) {
+  auto* kernel = repeats ? k_order_units<true> : k_order_units<false>;
+  kernel<<<grid, kOrderThreads, order_smem_bytes(), st>>>(o, u, G, P, S, strips, seg, gate);
 }
 
 int setup_p2g() {
@@ -2237,7 +2257,7 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
     else if ((threadIdx.x & 31) == 0)
       u.strip_n[b] = 0;
   }
-  order_share(o, Sg->np, strips, sv);
+  order_share<false>(o, Sg->np, strips, sv);
   __syncthreads();  // the shared memory is free again
   order_crowded(o, sv);
   if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;

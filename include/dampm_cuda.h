@@ -318,7 +318,10 @@ int dampm_cfl_dt_noalloc(const double* vpx, const double* vpy,
 int dampm_slab_record_doubles(void);
 /* After dampm_upload_particles of the slab's own particles (any order). */
 int dampm_slab_set(dampm_ctx* ctx, int col_lo, int col_hi);
-/* The reference index of each uploaded particle (np host ints). */
+/* The reference index of each uploaded particle (np host ints); without the
+ * call an upload's particles are numbered from 0.  A cell's sums run over its
+ * particles by index; particles of the same index in one cell follow in the
+ * order they lie in storage. */
 int dampm_slab_set_index(dampm_ctx* ctx, const int* idx);
 int dampm_slab_ghosts(dampm_ctx* ctx, double* buf, long long cap, long long* n);
 int dampm_slab_import(dampm_ctx* ctx, const double* buf, long long n, int ghosts);
