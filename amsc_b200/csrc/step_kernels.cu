@@ -640,7 +640,8 @@ __global__ void __launch_bounds__(kScanThreads)
 constexpr int kOrderPer = 4;
 constexpr int kOrderWin = 32 * kOrderPer + 2 * kCrowded;
 template <bool kRepeats>
-__device__ __forceinline__ void order_cells(const CellOrder& o, int np, int w, int nw, int* win) {
+__device__ __forceinline__ void order_cells(const CellOrder& o, int np, int w, int nw,
+                                            unsigned* win) {
   const int lane = threadIdx.x & 31;
   const int per = max(1, min(kOrderPer, np / (32 * nw)));
   const int tile = 32 * per;
@@ -679,15 +680,17 @@ __device__ __forceinline__ void order_cells(const CellOrder& o, int np, int w, i
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
     if (lo < hi)  // (else crowded cells only: lo + lane would overflow)
-      for (int i = lo + lane; i < hi; i += 32) win[i - lo] = o.n.sidx[i];
+      for (int i = lo + lane; i < hi; i += 32) win[i - lo] = unsigned(o.n.sidx[i]);
     load_keys(t + nw < tiles ? t + nw : tiles);
     __syncwarp();  // the window is filled
 #pragma unroll
     for (int u = 0; u < kOrderPer; ++u) {
       const int n = e[u] - b[u];
       if (n == 0) continue;
-      const int mine = win[p0 + u * 32 - lo];
-      const int* v = win + (b[u] - lo);
+      // (unsigned, as the entries of order_crowded compare: a slab's indices may
+      // have the top bit set)
+      const unsigned mine = win[p0 + u * 32 - lo];
+      const unsigned* v = win + (b[u] - lo);
       int rank = 0;
       if constexpr (kRepeats) {  // by index, then by storage slot
         const int* s = o.n.sslot + b[u];
@@ -1453,8 +1456,9 @@ __device__ __forceinline__ int2 plan_share(int strips) {
 template <bool kRepeats>
 __device__ __forceinline__ void order_share(const CellOrder& o, int np, int strips,
                                             unsigned long long* sv) {
-  static_assert(kOrderWin * sizeof(int) <= kUnitBuf * sizeof(int4), "");
-  int* win = reinterpret_cast<int*>(reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf);
+  static_assert(kOrderWin * sizeof(unsigned) <= kUnitBuf * sizeof(int4), "");
+  unsigned* win =
+      reinterpret_cast<unsigned*>(reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf);
   const int nb = plan_blocks(strips), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   int first, all;  // this warp's place among those that order
   if (nb > 0) {

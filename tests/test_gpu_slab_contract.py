@@ -1,5 +1,6 @@
 """What the slab calls accept: reference indices that repeat (each slab's
-particles numbered from 0, or all alike)."""
+particles numbered from 0, or all alike) or have the top bit set (they count as
+unsigned)."""
 import ctypes as C
 
 import numpy as np
@@ -79,3 +80,34 @@ def test_equal_indices_follow_in_storage_order(cuda_lib):
     finally:
         plain.close()
         alike.close()
+
+
+def test_indices_with_the_top_bit_set_come_last(cuda_lib):
+    """Indices count as unsigned numbers, in plain cells as in crowded ones: the
+    run is that of the particles listed in that order."""
+    d = scenarios.bench_slab(10000, nsteps=30)
+    rng = np.random.default_rng(3)
+    x, y, h = d.arrays["x"].copy(), d.arrays["y"].copy(), float(d.scalars["hx"])
+    pick = rng.permutation(x.size)[:600]  # a crowded cell too
+    x[pick] = 40.3 * h + 0.2 * h * rng.random(600)
+    y[pick] = 5.3 * h + 0.2 * h * rng.random(600)
+    d.arrays["x"], d.arrays["y"] = x, y
+    idx = (rng.permutation(d.np) - d.np // 2).astype(np.int32)
+    order = np.argsort(idx.view(np.uint32))
+    listed = d.copy()
+    for k in ("x", "y", "Mp", "Ap", "vpx", "vpy", "hp", "mom_px", "mom_py", "Vp"):
+        listed.arrays[k] = np.ascontiguousarray(d.arrays[k][order])
+    with Solver(listed) as s:
+        s.step(30)
+        ref = {k: s.download(k) for k in FIELDS}
+    run = local_run(d, 1)
+    try:
+        e = run.E[0]
+        _set_index(e, idx)
+        run.step(30)
+        for k in FIELDS:
+            v, ix = e.download(k)
+            v = v[np.argsort(ix.astype(np.int32).view(np.uint32))]
+            np.testing.assert_array_equal(v, ref[k], err_msg=k)
+    finally:
+        run.close()
