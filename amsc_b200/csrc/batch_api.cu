@@ -267,7 +267,7 @@ int enqueue_pass(dampm_batch* b) {
   k_scan_apply<<<ntiles, kApplyThreads, 0, st>>>(b->count, ncell, b->tile_sum, b->start, b->cbig,
                                                 b->ucount, b->Sg, gate, 0, b->tflag);
   const Binning n{key, slot, idx, b->sslot, b->sidx, b->skey};
-  k_scatter<<<gp, 256, 0, st>>>(n, b->start, b->tile_sum, ntiles, b->Sg, gate);
+  k_scatter<<<gp, 256, 0, st>>>(n, b->start, b->tile_sum, ntiles, b->ucount, b->Sg, gate);
   const UnitPlan u{b->units_per_cta * b->p2g_grid, unit_min_weight(b->useg_tot, b->p2g_grid),
                    int(b->USEG_cap), b->ulist, b->uslot, b->strip_n, b->ucount};
   k_b_order_units<<<order_blocks(b->P_tot), kOrderThreads, order_smem_bytes(), st>>>(

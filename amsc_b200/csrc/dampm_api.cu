@@ -277,7 +277,8 @@ void enqueue_sort(dampm_ctx* ctx, int begun, bool units) {
         ctx->count, ctx->nc, ctx->tile_sum, ctx->start, ctx->cbig, ctx->ucount, ctx->S, gate, 1,
         nullptr);
     k_scatter<<<grid_for(ctx->cap, 256), 256, 0, ctx->stream>>>(n, ctx->start, ctx->tile_sum,
-                                                                ctx->ntiles, ctx->S, gate);
+                                                                ctx->ntiles, ctx->ucount, ctx->S,
+                                                                gate);
   }
   launch_order_units(order_blocks(ctx->cap), ctx->stream,
                      CellOrder{n, ctx->start, ctx->cbig, ctx->ucount, ctx->perm, ctx->sortbuf,

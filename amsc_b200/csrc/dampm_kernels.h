@@ -186,11 +186,12 @@ struct Binning {
   const int *key, *slot, *idx;
   int *sslot, *sidx, *skey;
 };
-__global__ void k_scatter(Binning n, const int* start, int* tile_sum, int ntiles, Scalars* S,
-                          Gate gate);
+// (both scatters empty P2G's unit list, counters ucount)
+__global__ void k_scatter(Binning n, const int* start, int* tile_sum, int ntiles, int* ucount,
+                          Scalars* S, Gate gate);
 // scan and scatter in one, for up to kSmallCells cells (dynamic shared memory:
 // ncell ints); leaves the counts to be zeroed by the ordering
-__global__ void k_scan_scatter(const int* count, int ncell, int* start, int* big, int* list_n,
+__global__ void k_scan_scatter(const int* count, int ncell, int* start, int* big, int* ucount,
                                Binning n, Scalars* S, Gate gate);
 // What it takes to order the particles inside the cells.
 struct CellOrder {
@@ -204,7 +205,7 @@ struct CellOrder {
 };
 // The counters of a pass: the crowded cells (k_order_units, which uses them,
 // empties the list), P2G's units (plain, heavy) and its work cursor (set to zero
-// by G2P), the blocks of k_order_units that are done.
+// by the scatter), the blocks of k_order_units that are done.
 constexpr int kUnitsPlain = 1, kUnitsHeavy = 2, kUnitCursor = 3, kUnitCounts = 3, kOrderDone = 4;
 // P2G's unit list -- the plain units from 0, the heavy ones (which P2G takes
 // first) from cap -- with each unit's ledger slot.

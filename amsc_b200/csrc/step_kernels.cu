@@ -564,14 +564,21 @@ __device__ __forceinline__ void scatter(const Binning& n, const int* start, int 
   }
 }
 
+// Empties P2G's unit list for the planner that comes after (whether or not a G2P
+// followed the last one: half a step, then another upload).
+__device__ __forceinline__ void empty_units(int* ucount) {
+  if (blockIdx.x == 0 && threadIdx.x < kUnitCounts) ucount[kUnitsPlain + threadIdx.x] = 0;
+}
+
 // Also zeroes the tile totals (the scan has used them); block 0 rolls the key
 // ranges over.
 __global__ void k_scatter(Binning n, const int* __restrict__ start, int* __restrict__ tile_sum,
-                          int ntiles, Scalars* S, Gate gate) {
+                          int ntiles, int* __restrict__ ucount, Scalars* S, Gate gate) {
   if (!gate_open(S, gate)) return;
   scatter(n, start, S->np);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
     tile_sum[t * kTileStride] = 0;
+  empty_units(ucount);
   if (blockIdx.x == 0 && threadIdx.x == 0) roll_keys(S);
 }
 
@@ -585,7 +592,7 @@ __global__ void k_scatter(Binning n, const int* __restrict__ start, int* __restr
 // work, 64 KB of counts from L2, costs what the launches did.
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_scatter(const int* __restrict__ count, int ncell, int* __restrict__ start,
-                   int* __restrict__ big, int* __restrict__ list_n, Binning n, Scalars* S,
+                   int* __restrict__ big, int* __restrict__ ucount, Binning n, Scalars* S,
                    Gate gate) {
   if (!gate_open(S, gate)) return;
   extern __shared__ int sstart[];  // ncell
@@ -608,11 +615,12 @@ __global__ void __launch_bounds__(kScanThreads)
       }
       e += cv[k];
     }
-    if (writes) list_crowded(cv, i0, big, list_n);
+    if (writes) list_crowded(cv, i0, big, ucount);
     carry += total;
     __syncthreads();  // wsum is free again; the starts are in place
   }
   scatter(n, sstart, S->np);
+  empty_units(ucount);
   if (writes && threadIdx.x == 0) {
     start[ncell] = carry;
     roll_keys(S);
@@ -2083,7 +2091,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
             Phys P, Scalars* S, int* __restrict__ count, int* __restrict__ tile_sum,
             int* __restrict__ leave,
             const double* __restrict__ led_part, const int* __restrict__ strip_n, int strips,
-            int seg, int* __restrict__ ucount, double* __restrict__ log) {
+            int seg, double* __restrict__ log) {
   const int ng = S->nghost;
   const int n = S->np - ng;  // the slab's own particles
   const int blk = blockIdx.x - 1;  // the first block sums the ledger
@@ -2096,7 +2104,6 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
   }
   if (blk < 0) {
     ledger_final(led_part, strip_n, strips, seg, S, log);
-    if (threadIdx.x < kUnitCounts) ucount[kUnitsPlain + threadIdx.x] = 0;  // P2G is done
     if (threadIdx.x == 0) S->pending = 1;
     return;
   }
@@ -2149,8 +2156,7 @@ void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const i
   auto* kernel = record ? k_g2p_t<true, true>
                         : want_grad ? k_g2p_t<false, true> : k_g2p_t<false, false>;
   kernel<<<grid + 1, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G, P, S, count,
-                                           tile_sum, leave, led_part, u.strip_n, strips, seg,
-                                           u.ucount, log);
+                                           tile_sum, leave, led_part, u.strip_n, strips, seg, log);
 }
 
 size_t p2g_smem_bytes() { return sizeof(P2GSmemT<double>); }
@@ -2313,12 +2319,10 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
             const double* __restrict__ Z,
             const Scn* __restrict__ scn, Scalars* S, const int2* __restrict__ gblk,
             const Scalars* Sg, int* __restrict__ count, int* __restrict__ tile_sum,
-            const double* __restrict__ led_part, const int* __restrict__ strip_n,
-            int* __restrict__ ucount, int nscn) {
+            const double* __restrict__ led_part, const int* __restrict__ strip_n, int nscn) {
   if (blockIdx.x < nscn) {
     const int q = blockIdx.x;
     if (!Sg->active) return;
-    if (q == 0 && threadIdx.x < kUnitCounts) ucount[kUnitsPlain + threadIdx.x] = 0;  // P2G is done
     if (scn[q].live && S[q].active) {
       ledger_reduce(led_part + (size_t)scn[q].useg_off * 6, strip_n + scn[q].strip_off,
                     scn[q].nstrips, scn[q].G.ncols + 1, &S[q]);
@@ -2496,8 +2500,7 @@ void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nx
                   const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count,
                   int* tile_sum, const double* led_part, const UnitPlan& u, int nscn) {
   k_b_g2p<R><<<nblk + nscn, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, vvL, Z, scn, S, gblk,
-                                                  Sg, count, tile_sum, led_part, u.strip_n, u.ucount,
-                                                  nscn);
+                                                  Sg, count, tile_sum, led_part, u.strip_n, nscn);
 }
 
 template <class R>

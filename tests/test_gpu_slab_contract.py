@@ -1,13 +1,13 @@
 """What the slab calls accept: reference indices that repeat (each slab's
 particles numbered from 0, or all alike) or have the top bit set (they count as
-unsigned)."""
+unsigned), and a first half of a step that no second half follows."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
 from amsc_b200 import scenarios
-from amsc_b200.dampm import Solver
+from amsc_b200.dampm import Solver, _ptr
 from amsc_b200.slabs import local_run
 
 pytestmark = pytest.mark.gpu
@@ -109,5 +109,31 @@ def test_indices_with_the_top_bit_set_come_last(cuda_lib):
             v, ix = e.download(k)
             v = v[np.argsort(ix.astype(np.int32).view(np.uint32))]
             np.testing.assert_array_equal(v, ref[k], err_msg=k)
+    finally:
+        run.close()
+
+
+@pytest.mark.parametrize("cells", [64, 256])  # one launch for scan and scatter, two
+def test_upload_after_half_a_step(cuda_lib, cells):
+    """A caller that gives a step up after its first half and uploads again gets
+    the run of a fresh context: P2G's work list does not keep the units of the
+    half that was given up."""
+    d = scenarios.dam_break_flat(nsteps=100) if cells == 64 else scenarios.mudflow(N=cells)
+    with Solver(d) as s:
+        s.step(10)
+        ref = {k: s.download(k) for k in FIELDS}
+        led = s.ledgers()
+    run = local_run(d, 1)
+    try:
+        e = run.E[0]
+        arrs = [_ptr(d.arrays[k]) for k in ("x", "y", "Mp", "Ap", "vpx", "vpy", "hp", "mom_px",
+                                            "mom_py", "Vp")]
+        for _ in range(3):
+            e.pass_(0)
+            e.s._check(e.lib.dampm_upload_particles(e.h, d.np, *arrs))
+        run.step(10)
+        for k in FIELDS:
+            np.testing.assert_array_equal(run.gather(k), ref[k], err_msg=k)
+        np.testing.assert_allclose(run.ledgers()[:6], led[:6], rtol=1e-12, atol=1e-9)
     finally:
         run.close()
