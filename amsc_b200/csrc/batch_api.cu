@@ -568,6 +568,12 @@ int dampm_batch_add(dampm_batch* b, const dampm_grid* grid, const dampm_params* 
     return DAMPM_ERR_ARG;
   if (grid->Nex < 1 || grid->Ney < 1 || !(grid->hx > 0) || !(grid->hy > 0))
     return bfail(b, DAMPM_ERR_ARG, "bad grid");
+  // An addition runs when it is called: captured, its copies would read staging
+  // buffers that have moved on by the time the graph is launched.
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  BCK(cudaStreamIsCapturing(b->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone)
+    return bfail(b, DAMPM_ERR_CUDA, "a scenario cannot be added while its stream is captured");
   HostScn h;
   h.grid = *grid;
   h.params = *params;

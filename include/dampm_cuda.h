@@ -360,7 +360,9 @@ int dampm_batch_destroy(dampm_batch* b);
 
 /* Appends one scenario (DATA arrays in DATA order, terrain Z in quadgrid node
  * order; the gradients dZdx/dZdy only feed recorded outputs and are not
- * taken).  Returns DAMPM_ERR_CAPACITY when the batch is full.  *handle
+ * taken).  Returns DAMPM_ERR_CAPACITY when the batch is full, DAMPM_ERR_CUDA
+ * while the caller captures the batch's stream.  The arrays are the caller's
+ * again when the call returns; the stream is not waited for.  *handle
  * identifies the scenario in later calls. */
 int dampm_batch_add(dampm_batch* b, const dampm_grid* grid,
                     const dampm_params* params, const double* Z, long long np,
