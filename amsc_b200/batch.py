@@ -41,7 +41,7 @@ class Batch:
             raise DampmError(f"dampm_batch_create failed ({rc})")
         self.h = h
         self.np: Dict[int, int] = {}
-        self._tuning = (2, 192)  # what autotune starts from: the even load of a large batch
+        self._tuning = (1, 192)  # units per CTA and column weight in force (the library's)
 
     def _check(self, rc: int):
         if rc != 0:
@@ -118,6 +118,7 @@ class Batch:
         replay of multi-pass steps (0 / None keeps a setting)."""
         g = -1 if graphs is None else (1 if graphs else 0)
         self._check(self.lib.dampm_batch_tune(self.h, int(units_per_cta), int(col_weight), g))
+        self._tuning = (int(units_per_cta) or self._tuning[0], int(col_weight) or self._tuning[1])
 
     def autotune(self, passes: int = 16, units=(1, 2, 4, 8), weights=(64, 192, 512),
                  margin: float = 0.03) -> Dict:
@@ -154,7 +155,6 @@ class Batch:
                 if t < cur * (1.0 - margin):
                     cw, cur = w, t
         self.tune(cu, cw)
-        self._tuning = (cu, cw)
         return {"units_per_cta": cu, "col_weight": cw, "ms_per_pass": 1e3 * cur,
                 "passes": 3 * passes * len(trials), "trials": trials}
 
