@@ -46,7 +46,7 @@ struct dampm_batch {
   long long USEG_cap = 0;
   // packed totals (live and dead scenarios)
   long long P_tot = 0, N_tot = 0, C_tot = 0, useg_tot = 0;
-  int strips_tot = 0, nblk = 0;
+  int strips_tot = 0, pieces_tot = 0, nblk = 0;
   std::vector<HostScn> scns;  // packed order = device table order
   int next_handle = 0;
   // device
@@ -70,7 +70,7 @@ struct dampm_batch {
   unsigned char* tflag = nullptr;  // the scan tiles of a pass (k_b_step_begin)
   int4* ulist = nullptr;  // plain units, then heavy ones (USEG_cap each)
   int* uslot = nullptr;   // their ledger slots
-  int *strip_n = nullptr, *ucount = nullptr, *strip_scn = nullptr;
+  int *piece_n = nullptr, *ucount = nullptr, *piece_scn = nullptr;
   double* led_part = nullptr;
   int2* gblk = nullptr;
   int4 *mblk = nullptr, *nmove = nullptr;
@@ -81,7 +81,7 @@ struct dampm_batch {
   // pinned mirrors of the tables: an addition appends its entries and copies
   // them without waiting (only a compaction, which waits, rewrites them)
   Scn* scn_h = nullptr;
-  int* strip_scn_h = nullptr;
+  int* piece_scn_h = nullptr;
   int2* gblk_h = nullptr;
   // staging of an addition's arrays, pinned and on the device, two of each:
   // one is filled while the other travels
@@ -199,28 +199,29 @@ ParticlesT<R> shifted(const ParticlesT<R>& p, long long off) {
 }
 
 int strips_of(const dampm_grid& g) { return (g.Ney + 1 + kTR - 1) / kTR; }
+int pieces_of(const Scn& d) { return d.nstrips * d.G.pieces; }
 
-// Appends scenario `pos` to the table mirrors; the entries' ranges in *strip
+// Appends scenario `pos` to the table mirrors; the entries' ranges in *piece
 // and *blk.
-void append_tables(dampm_batch* b, size_t pos, int2* strip, int2* blk) {
+void append_tables(dampm_batch* b, size_t pos, int2* piece, int2* blk) {
   const Scn& d = b->scns[pos].d;
   b->scn_h[pos] = d;
-  *strip = make_int2(d.strip_off, d.nstrips);
-  for (int k = 0; k < d.nstrips; ++k) b->strip_scn_h[d.strip_off + k] = int(pos);
+  *piece = make_int2(d.piece_off, pieces_of(d));
+  for (int k = 0; k < piece->y; ++k) b->piece_scn_h[d.piece_off + k] = int(pos);
   blk->x = b->nblk;
   for (int f = 0; f < d.np; f += kG2PThreads) b->gblk_h[b->nblk++] = make_int2(int(pos), f);
   blk->y = b->nblk - blk->x;
 }
 
-// Uploads entries of the tables (scenarios, strips, G2P blocks) with the
+// Uploads entries of the tables (scenarios, pieces, G2P blocks) with the
 // batch totals, without waiting.
-int upload_tables(dampm_batch* b, int2 scn, int2 strip, int2 blk) {
+int upload_tables(dampm_batch* b, int2 scn, int2 piece, int2 blk) {
   if (scn.y > 0)
     BCK(cudaMemcpyAsync(b->scn + scn.x, b->scn_h + scn.x, sizeof(Scn) * size_t(scn.y),
                         cudaMemcpyHostToDevice, b->stream));
-  if (strip.y > 0)
-    BCK(cudaMemcpyAsync(b->strip_scn + strip.x, b->strip_scn_h + strip.x,
-                        sizeof(int) * size_t(strip.y), cudaMemcpyHostToDevice, b->stream));
+  if (piece.y > 0)
+    BCK(cudaMemcpyAsync(b->piece_scn + piece.x, b->piece_scn_h + piece.x,
+                        sizeof(int) * size_t(piece.y), cudaMemcpyHostToDevice, b->stream));
   if (blk.y > 0)
     BCK(cudaMemcpyAsync(b->gblk + blk.x, b->gblk_h + blk.x, sizeof(int2) * size_t(blk.y),
                         cudaMemcpyHostToDevice, b->stream));
@@ -269,10 +270,10 @@ int enqueue_pass(dampm_batch* b) {
   const Binning n{key, slot, idx, b->sslot, b->sidx, b->skey};
   k_scatter<<<gp, 256, 0, st>>>(n, b->start, b->tile_sum, ntiles, b->ucount, b->Sg, gate);
   const UnitPlan u{b->units_per_cta * b->p2g_grid, unit_min_weight(b->useg_tot, b->p2g_grid),
-                   int(b->USEG_cap), b->ulist, b->uslot, b->strip_n, b->ucount};
-  k_b_order_units<<<order_blocks(b->P_tot), kOrderThreads, order_smem_bytes(), st>>>(
+                   int(b->USEG_cap), b->ulist, b->uslot, b->piece_n, b->ucount};
+  k_b_order_units<<<order_blocks(b->P_tot, b->pieces_tot), kOrderThreads, order_smem_bytes(), st>>>(
       CellOrder{n, b->start, b->cbig, b->ucount, b->perm, b->sortbuf, b->P_cap, b->count, 0},
-      u, b->scn, b->S, nscn, b->strip_scn, b->strips_tot, b->Sg, b->col_weight);
+      u, b->scn, b->S, nscn, b->piece_scn, b->pieces_tot, b->Sg, b->col_weight);
   if (b->precision == DAMPM_FP32)
     launch_b_p2g<float>(b->p2g_grid, st, b->p32[b->cur], b->perm, b->start,
                         static_cast<float2*>(b->vvL),
@@ -476,8 +477,10 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   rc = rc ? rc : balloc(b, &b->ulist, 2 * us);
   rc = rc ? rc : balloc(b, &b->uslot, 2 * us);
   rc = rc ? rc : balloc(b, &b->led_part, us * 6);
-  rc = rc ? rc : balloc(b, &b->strip_n, size_t(b->STRIP_cap));
-  rc = rc ? rc : balloc(b, &b->strip_scn, size_t(b->STRIP_cap));
+  // a strip of n columns has at most n / kPlanCols + 1 pieces
+  const size_t pieces = size_t(b->STRIP_cap) + us / kPlanCols;
+  rc = rc ? rc : balloc(b, &b->piece_n, pieces);
+  rc = rc ? rc : balloc(b, &b->piece_scn, pieces);
   rc = rc ? rc : balloc(b, &b->ucount, 8);
   if (rc == DAMPM_OK && cudaMemsetAsync(b->ucount, 0, sizeof(int) * 8, b->stream) != cudaSuccess)
     rc = bfail(b, DAMPM_ERR_CUDA, "cudaMemsetAsync failed");
@@ -502,7 +505,7 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
     };
     const size_t at_S = place(sizeof(Scalars) * size_t(scenario_cap));
     const size_t at_scn = place(sizeof(Scn) * size_t(scenario_cap));
-    const size_t at_strip = place(sizeof(int) * size_t(b->STRIP_cap));
+    const size_t at_piece = place(sizeof(int) * pieces);
     const size_t at_blk = place(sizeof(int2) * size_t(b->B_cap));
     const size_t at_raw[2] = {place(sizeof(double) * kRawDoubles),
                               place(sizeof(double) * kRawDoubles)};
@@ -512,7 +515,7 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
       char* p = static_cast<char*>(b->pinned);
       b->Sh = reinterpret_cast<Scalars*>(p + at_S);
       b->scn_h = reinterpret_cast<Scn*>(p + at_scn);
-      b->strip_scn_h = reinterpret_cast<int*>(p + at_strip);
+      b->piece_scn_h = reinterpret_cast<int*>(p + at_piece);
       b->gblk_h = reinterpret_cast<int2*>(p + at_blk);
       for (int k = 0; k < 2; ++k) b->raw_h[k] = reinterpret_cast<double*>(p + at_raw[k]);
     }
@@ -589,13 +592,14 @@ int dampm_batch_add(dampm_batch* b, const dampm_grid* grid, const dampm_params* 
                  "batch full: remove finished scenarios and compact, or create a larger batch");
   Scn& d = h.d;
   d.G = make_geom(*grid);
+  set_pieces(d.G, np);
   d.P = make_phys(*params);
   d.p_off = int(b->P_tot);
   d.np = int(np);
   d.n_off = int(b->N_tot);
   d.c_off = int(b->C_tot);
-  d.strip_off = b->strips_tot;
   d.nstrips = nstrips;
+  d.piece_off = b->pieces_tot;
   d.useg_off = int(b->useg_tot);
   d.live = 1;
   h.handle = b->next_handle++;
@@ -625,10 +629,11 @@ int dampm_batch_add(dampm_batch* b, const dampm_grid* grid, const dampm_params* 
   b->N_tot += h.nn;
   b->C_tot += h.nc;
   b->strips_tot += nstrips;
+  b->pieces_tot += pieces_of(d);
   b->useg_tot += useg;
-  int2 strip, blk;
-  append_tables(b, size_t(pos), &strip, &blk);
-  int rc = upload_tables(b, make_int2(pos, 1), strip, blk);
+  int2 piece, blk;
+  append_tables(b, size_t(pos), &piece, &blk);
+  int rc = upload_tables(b, make_int2(pos, 1), piece, blk);
   if (rc) return rc;
   *handle = h.handle;
   return DAMPM_OK;
@@ -658,7 +663,7 @@ int dampm_batch_compact(dampm_batch* b) {
   std::vector<Scalars> S;
   std::vector<int4> mv, nm;
   long long P = 0, N = 0, C = 0, U = 0;
-  int strips = 0;
+  int strips = 0, pieces = 0;
   for (size_t s = 0; s < b->scns.size(); ++s) {
     HostScn h = b->scns[s];
     if (!h.d.live) continue;
@@ -666,7 +671,7 @@ int dampm_batch_compact(dampm_batch* b) {
     h.d.p_off = int(P);
     h.d.n_off = int(N);
     h.d.c_off = int(C);
-    h.d.strip_off = strips;
+    h.d.piece_off = pieces;
     h.d.useg_off = int(U);
     for (int f = 0; f < old.np; f += kG2PThreads)
       mv.push_back(make_int4(h.d.p_off + f, old.p_off + f,
@@ -678,6 +683,7 @@ int dampm_batch_compact(dampm_batch* b) {
     N += h.nn;
     C += h.nc;
     strips += old.nstrips;
+    pieces += pieces_of(old);
     U += (long long)old.nstrips * (h.grid.Nex + 1);
     S.push_back(b->Sh[s]);
     // its cells move: the first plan after the move covers all of them
@@ -724,13 +730,14 @@ int dampm_batch_compact(dampm_batch* b) {
   b->N_tot = N;
   b->C_tot = C;
   b->strips_tot = strips;
+  b->pieces_tot = pieces;
   b->useg_tot = U;
   // every table entry anew, once the copies of the old ones have been made
   BCK(cudaStreamSynchronize(b->stream));
   b->nblk = 0;
-  int2 strip, blk;
-  for (size_t s = 0; s < keep.size(); ++s) append_tables(b, s, &strip, &blk);
-  return upload_tables(b, make_int2(0, int(keep.size())), make_int2(0, strips),
+  int2 piece, blk;
+  for (size_t s = 0; s < keep.size(); ++s) append_tables(b, s, &piece, &blk);
+  return upload_tables(b, make_int2(0, int(keep.size())), make_int2(0, pieces),
                        make_int2(0, b->nblk));
 }
 

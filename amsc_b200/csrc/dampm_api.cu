@@ -43,7 +43,7 @@ struct dampm_ctx {
   double* led_part = nullptr;
   int n_led = 0;
   int strips = 0, useg = 0;  // strips; unit slots per strip (ncols + 1)
-  int *strip_n = nullptr, *ucount = nullptr;
+  int *piece_n = nullptr, *ucount = nullptr;
   int4* ulist = nullptr;  // plain units, then heavy ones (n_led each)
   int* uslot = nullptr;   // their ledger slots
   int* cbig = nullptr;  // cells with more than 256 particles (capacity / 256)
@@ -255,7 +255,7 @@ int* tile_totals(const dampm_ctx* ctx) { return small_grid(ctx) ? nullptr : ctx-
 
 UnitPlan unit_plan(const dampm_ctx* ctx) {
   return UnitPlan{kUnitsPerCta * ctx->p2g_grid, unit_min_weight(ctx->n_led, ctx->p2g_ctas),
-                  ctx->n_led, ctx->ulist, ctx->uslot, ctx->strip_n, ctx->ucount};
+                  ctx->n_led, ctx->ulist, ctx->uslot, ctx->piece_n, ctx->ucount};
 }
 
 // Enqueues the binning of the current particles (SORT), whose slots and
@@ -265,11 +265,11 @@ UnitPlan unit_plan(const dampm_ctx* ctx) {
 // the step before and the begin of this one.
 void enqueue_sort(dampm_ctx* ctx, int begun, bool units) {
   const Gate gate = make_gate(ctx->P, begun);
-  const int strips = units ? ctx->strips : 0;
+  const int pieces = units ? ctx->strips * ctx->G.pieces : 0;
   const bool small = small_grid(ctx);
   const Binning n{ctx->p.key, ctx->p.slot, ctx->p.idx, ctx->sslot, ctx->sidx, ctx->skey};
   if (small) {
-    k_scan_scatter<<<order_blocks(ctx->cap), kScanThreads, sizeof(int) * size_t(ctx->nc),
+    k_scan_scatter<<<order_blocks(ctx->cap, 0), kScanThreads, sizeof(int) * size_t(ctx->nc),
                      ctx->stream>>>(ctx->count, ctx->nc, ctx->start, ctx->cbig, ctx->ucount, n,
                                     ctx->S, gate);
   } else {
@@ -280,10 +280,10 @@ void enqueue_sort(dampm_ctx* ctx, int begun, bool units) {
                                                                 ctx->ntiles, ctx->ucount, ctx->S,
                                                                 gate);
   }
-  launch_order_units(order_blocks(ctx->cap), ctx->stream,
+  launch_order_units(order_blocks(ctx->cap, pieces), ctx->stream,
                      CellOrder{n, ctx->start, ctx->cbig, ctx->ucount, ctx->perm, ctx->sortbuf,
                                ctx->cap, ctx->count, small ? ctx->nc : 0},
-                     unit_plan(ctx), ctx->G, ctx->P, ctx->S, strips, ctx->useg, gate, ctx->slab);
+                     unit_plan(ctx), ctx->G, ctx->P, ctx->S, pieces, ctx->useg, gate, ctx->slab);
   ctx->launches += small ? 2 : 3;
 }
 
@@ -338,7 +338,7 @@ int enqueue_back(dampm_ctx* ctx) {
   ev_mark(ctx, 2);
   launch_g2p(grid_for(ctx->cap, kG2PThreads), ctx->stream, ctx->p, ctx->q, ctx->perm,
              ctx->skey, ctx->nodes, ctx->Z, ctx->G, ctx->P, ctx->S, ctx->count,
-             tile_totals(ctx), ctx->leave, ctx->led_part, unit_plan(ctx), ctx->strips, ctx->useg,
+             tile_totals(ctx), ctx->leave, ctx->led_part, unit_plan(ctx), ctx->strips * ctx->G.pieces, ctx->useg,
              ctx->ledger_log,
              ctx->record ? 1 : 0,
              (grad_next || ctx->record) ? 1 : 0);
@@ -708,7 +708,7 @@ int dampm_ctx_create(const dampm_grid* grid, const dampm_params* params,
   rc = rc ? rc : dalloc(ctx, &ctx->led_part, size_t(ctx->n_led) * 6);
   rc = rc ? rc : dalloc(ctx, &ctx->ulist, size_t(ctx->n_led) * 2);
   rc = rc ? rc : dalloc(ctx, &ctx->uslot, size_t(ctx->n_led) * 2);
-  rc = rc ? rc : dalloc(ctx, &ctx->strip_n, size_t(ctx->strips));
+  rc = rc ? rc : dalloc(ctx, &ctx->piece_n, size_t(ctx->strips) * size_t(ctx->G.pieces));  // at most
   rc = rc ? rc : dalloc(ctx, &ctx->ucount, 8);
   rc = rc ? rc : dalloc(ctx, &ctx->ledger_log, size_t(kLedgerLog) * 3);
   rc = rc ? rc : dalloc(ctx, &ctx->S, 1);
@@ -801,6 +801,7 @@ int dampm_upload_particles(dampm_ctx* ctx, long long np, const double* x,
     CK(upload_pair(p.mp, mom_px, mom_py, np, ctx->msb.mx, ctx->msb.my, ctx->stream));
     CK(cudaMemcpyAsync(p.Vp, Vp, b, cudaMemcpyHostToDevice, ctx->stream));
   }
+  set_pieces(ctx->G, np);
   Scalars s0{};
   s0.fresh = 1;
   s0.np = int(np);
@@ -1106,6 +1107,7 @@ int dampm_set_state(dampm_ctx* ctx, long long np, const double* const* fields,
   }
   int rc = sync_status(ctx, false);
   if (rc) return rc;
+  set_pieces(ctx->G, np);
   ctx->Sh->np = int(np);
   ctx->Sh->fresh = fresh ? 1 : 0;
   ctx->Sh->status = 0;  // a new state: an earlier divergence no longer applies

@@ -24,6 +24,8 @@ struct Geom {
   // P. Montgomery, Division by invariant integers using multiplication, 1994)
   unsigned rmul;
   int rshift;
+  // the pieces of a strip that the unit planner takes one by one, their columns
+  int pieces, plan_cols;
   // The part of the grid a slab owns (the whole grid outside slab mode):
   // particles of cell columns [pc_lo, pc_hi), node columns [nc_lo, nc_hi]
   // written by P2G.

@@ -1,5 +1,6 @@
 // dampm_kernels.h -- device buffers and kernel entry points of the step.
 #pragma once
+#include <algorithm>
 #include <cstddef>
 #include <utility>
 
@@ -37,6 +38,18 @@ inline int unit_min_weight(long long pairs, int ctas) {
 }
 constexpr int kColWeight = DAMPM_COL_WEIGHT;
 constexpr int kOrderThreads = 1024;
+// A strip is planned in pieces of kPlanCols columns or a multiple of them, a warp
+// each: one warp takes 9 us for 512 columns, 35 for the 2048 of a strip, which a flow
+// of few particles waits for, and 4 ms for those of a strip of 200000.  The
+// particles are ordered beside it, a million in 9 us: a piece has 512 columns for
+// every million, and strips of up to 2048 columns with 4M particles stay whole.
+// (Each cut between two pieces adds at most one unit to the 50 or more that the
+// columns of a piece make by their weight alone.)
+constexpr int kPlanCols = 512;
+inline void set_pieces(Geom& G, long long np) {
+  G.plan_cols = kPlanCols * int((np >> 20) + 1);
+  G.pieces = (G.ncols + G.plan_cols - 1) / G.plan_cols;
+}
 constexpr int kMaxStrips = 8192;  // strip offsets of the unit list in shared memory
 constexpr int kP2GThreads = 128;
 #ifndef DAMPM_P2G_CAP
@@ -213,21 +226,22 @@ struct UnitPlan {
   int target_units, min_weight, cap;
   int4* ulist;
   int* uslot;
-  int* strip_n;  // units of each strip
+  int* piece_n;  // units of each piece of each strip
   int* ucount;   // the counters
 };
-// orders the particles inside the cells and, with strips > 0, makes the unit
-// list (seg: unit slots per strip) and ends the step before and begins this
+// orders the particles inside the cells and, with pieces > 0 (all strips'), makes
+// the unit list (seg: unit slots per strip) and ends the step before and begins this
 // one unless it has begun.  order_smem_bytes(): its dynamic shared memory;
 // setup_sort sets the sort kernels' limits (0 on failure)
 // repeats: reference indices may repeat inside a cell
 void launch_order_units(int grid, cudaStream_t st, const CellOrder& o, const UnitPlan& u, Geom G,
-                        Phys P, Scalars* S, int strips, int seg, Gate gate, bool repeats);
+                        Phys P, Scalars* S, int pieces, int seg, Gate gate, bool repeats);
 size_t order_smem_bytes();
 int setup_sort();
-// blocks of 1024 threads for np particles, one per SM at most
-inline int order_blocks(long long np) {
-  const long long b = (np + kOrderThreads - 1) / kOrderThreads;
+// blocks of 1024 threads for np particles and (k_order_units) `pieces` to plan,
+// four to a block, one per SM at most
+inline int order_blocks(long long np, long long pieces) {
+  const long long b = std::max((np + kOrderThreads - 1) / kOrderThreads, (pieces + 3) / 4);
   return int(b < 1 ? 1 : b > 148 ? 148 : b);
 }
 // P2G of the single-scenario step (k_p2g specialised for recorded outputs);
@@ -244,7 +258,7 @@ constexpr int kLedgerLog = 1024;  // rows of the per-step ledger log
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
                 int* count, int* tile_sum, int* leave, const double* led_part, const UnitPlan& u,
-                int strips, int seg, double* log, int record, int want_grad);
+                int pieces, int seg, double* log, int record, int want_grad);
 
 // ---- batches of independent scenarios --------------------------------------
 // One scenario of a batch: its geometry, physics and place in the packed
@@ -255,13 +269,14 @@ struct Scn {
   int p_off, np;           // particles [p_off, p_off + np)
   int n_off;               // first node
   int c_off;               // first cell (cell keys are c_off + r + c*nrows)
-  int strip_off, nstrips;  // its strips in the batch's strip order
+  int nstrips;
+  int piece_off;           // its pieces in the batch's order
   int useg_off;            // first unit-plan slot of its first strip
   int live;                // 0 once removed
 };
 
 __global__ void k_b_order_units(CellOrder o, UnitPlan u, const Scn* scn, Scalars* S, int nscn,
-                                const int* strip_scn, int strips, const Scalars* Sg,
+                                const int* piece_scn, int pieces, const Scalars* Sg,
                                 int col_weight);
 __global__ void k_b_step_begin(const Scn* scn, Scalars* S, int nscn, Scalars* Sg,
                                unsigned char* tflag, int ntiles);

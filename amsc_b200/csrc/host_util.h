@@ -26,6 +26,7 @@ inline Geom make_geom(const dampm_grid& g) {
   while ((1LL << L) < g.Ney) ++L;
   G.rshift = 31 + L;
   G.rmul = unsigned((1ULL << G.rshift) / unsigned(g.Ney) + 1);
+  set_pieces(G, 0);
   G.pc_lo = 0;
   G.pc_hi = g.Nex;
   G.nc_lo = 0;

@@ -1294,9 +1294,9 @@ __device__ __forceinline__ void solo_batch(Chains<R>& a, P2GSmemT<R>& s, int rc,
 // carries about the same weight -- its particles plus kColWeight per column
 // -- whatever the local particle density: P2G takes them from a shared
 // cursor, so its time is the average load rather than the heaviest fixed
-// block.  The list is in no particular order; the ledger partial of a strip's
-// n-th unit sits in the strip's n-th slot, so the ledger reduction order is
-// fixed.
+// block.  The list is in no particular order; the ledger partials of the units
+// of a piece sit in order from the slot of its first column on, so the ledger
+// reduction order is fixed.
 namespace {
 
 __device__ __forceinline__ int column_count(const int* __restrict__ cstart,
@@ -1306,16 +1306,15 @@ __device__ __forceinline__ int column_count(const int* __restrict__ cstart,
 
 }  // namespace
 
-// Cuts strip `strip` of one grid (cstart of that grid's cells, node columns
-// [c_lo, c_hi]) into units of weight about T and appends those with particles
+// Cuts node columns [c_lo, c_hi] of strip `strip` of one grid (cstart of that
+// grid's cells) into units of weight about T and appends those with particles
 // (including the particles of the leading column cA-1, which feed node column
-// cA) to P2G's list as make(cA, cB), with the ledger slot slot0 + n of the
-// strip's n-th unit; units of more than twice the target weight (a crowded
-// column) go to the half of the list that P2G takes first.  *strip_n: the
-// number of units.  Node column nc (< ncols) weighs the particles of cell column
+// cA) to P2G's list as make(cA, cB), with the ledger slot slot0 + n of the n-th
+// of them; units of more than twice the target weight (a crowded column) go to
+// the half of the list that P2G takes first.  Returns the number of units.  Node column nc (< ncols) weighs the particles of cell column
 // nc in the strip's cell rows plus col_weight; nc starts a unit where
 // floor(exclusive prefix / T) changes.
-// One warp cuts a strip, 32 columns at a time, and needs no barrier: a lane
+// One warp cuts a strip (or a piece of one), 32 columns at a time, and needs no barrier: a lane
 // whose column starts a unit emits the one that ends there.  The units wait in
 // `buf` (kUnitBuf entries of shared memory) and are appended together, so that
 // nothing has to wait for all the strips.  With one block per strip, scans over
@@ -1353,10 +1352,10 @@ __device__ __forceinline__ void flush_units(const UnitPlan& u, const int4* buf, 
 }
 
 template <class Make>
-__device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const Geom& G,
-                                           long long T, int strip, int4* buf, const UnitPlan& u,
-                                           int slot0, int* strip_n, int col_weight, int c_lo,
-                                           int c_hi, Make make) {
+__device__ __forceinline__ int plan_columns(const int* __restrict__ cstart, const Geom& G,
+                                            long long T, int strip, int4* buf, const UnitPlan& u,
+                                            int slot0, int col_weight, int c_lo, int c_hi,
+                                            Make make) {
   col_weight = min(col_weight, 1 << 25);
   const int nrows = G.nrows, ncols = G.ncols;
   const int r0 = strip * kTR;
@@ -1433,7 +1432,7 @@ __device__ __forceinline__ void plan_strip(const int* __restrict__ cstart, const
   }
   emit(lane == 0, oA, c_hi + 1, oP, carry, oV);
   if (n > 0) flush_units(u, buf, n, heavies, slot0 + J, make);
-  if (lane == 0) *strip_n = J + n;
+  return J + n;
 }
 
 __device__ __forceinline__ long long unit_weight(const Scalars* S,
@@ -1442,39 +1441,55 @@ __device__ __forceinline__ long long unit_weight(const Scalars* S,
   return T < u.min_weight ? u.min_weight : T;
 }
 
+// Plans piece k of a strip (G.plan_cols columns; node columns [c_lo, c_hi] of
+// them): slot0 and piece_n are the first ledger slot and the unit count of the
+// strip's first piece.
+template <class Make>
+__device__ __forceinline__ void plan_piece(const int* __restrict__ cstart, const Geom& G,
+                                           long long T, int strip, int k, int4* buf,
+                                           const UnitPlan& u, int slot0, int* piece_n,
+                                           int col_weight, int c_lo, int c_hi, Make make) {
+  const int first = k * G.plan_cols;
+  const int lo = max(c_lo, first), hi = k + 1 < G.pieces ? min(c_hi, first + G.plan_cols - 1) : c_hi;
+  int n = 0;
+  if (lo <= hi)
+    n = plan_columns(cstart, G, T, strip, buf, u, slot0 + first, col_weight, lo, hi, make);
+  if ((threadIdx.x & 31) == 0) piece_n[k] = n;
+}
+
 // Who plans and who orders: the first plan_blocks() blocks plan, four warps each,
 // and the others order -- beside the ordering's busy warps a planning warp got an
 // eighth of its scheduler's issue slots and was the last to finish (a step of the
 // 4096-particle dam break 0.6 us longer, of 4M particles 4).  Where that would take
 // more than one block in kPlanShare (a batch of many scenarios, or a grid of few
-// blocks) the strips are spread over the blocks, warp 0 of each, then warp 1 ...,
+// blocks) the pieces are spread over the blocks, warp 0 of each, then warp 1 ...,
 // and the other warps order (everyone where that leaves fewer than half): 11 us
 // against 15 with the 800 strips of 96 scenarios.
 constexpr int kPlanShare = 4;
-__device__ __forceinline__ int plan_blocks(int strips) {
-  const int nb = (strips + 3) / 4;
+__device__ __forceinline__ int plan_blocks(int pieces) {
+  const int nb = (pieces + 3) / 4;
   return nb <= int(gridDim.x) / kPlanShare ? nb : 0;
 }
-// this warp's first strip and the step to its next one
-__device__ __forceinline__ int2 plan_share(int strips) {
-  const int nb = plan_blocks(strips), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// this warp's first piece and the step to its next one
+__device__ __forceinline__ int2 plan_share(int pieces) {
+  const int nb = plan_blocks(pieces), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int over = nb ? nb : gridDim.x;
-  return make_int2(int(blockIdx.x) < over ? w * over + int(blockIdx.x) : strips, over * nw);
+  return make_int2(int(blockIdx.x) < over ? w * over + int(blockIdx.x) : pieces, over * nw);
 }
 template <bool kRepeats>
-__device__ __forceinline__ void order_share(const CellOrder& o, int np, int strips,
+__device__ __forceinline__ void order_share(const CellOrder& o, int np, int pieces,
                                             unsigned long long* sv) {
   static_assert(kOrderWin * sizeof(unsigned) <= kUnitBuf * sizeof(int4), "");
   unsigned* win =
       reinterpret_cast<unsigned*>(reinterpret_cast<int4*>(sv) + (threadIdx.x >> 5) * kUnitBuf);
-  const int nb = plan_blocks(strips), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nb = plan_blocks(pieces), w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   int first, all;  // this warp's place among those that order
   if (nb > 0) {
     first = (int(blockIdx.x) - nb) * nw + w;
     all = (int(gridDim.x) - nb) * nw;
   } else {
     all = int(gridDim.x) * nw;
-    const int planners = 2 * strips <= all ? strips : 0;
+    const int planners = 2 * pieces <= all ? pieces : 0;
     first = w * int(gridDim.x) + int(blockIdx.x) - planners;
     all -= planners;
   }
@@ -1494,10 +1509,11 @@ __device__ __forceinline__ int4* unit_buf(unsigned long long* sv) {
 // The begin sits here and not at the end of G2P, where every block would have
 // to wait for its stores before it counts itself done (7 us at 0.25M and 4M
 // particles).
-// strips = 0: the sort alone (before a merge/split); seg: unit slots per strip
+// pieces: of all strips; 0: the sort alone (before a merge/split); seg: unit slots
+// per strip
 template <bool kRepeats>
 __global__ void __launch_bounds__(kOrderThreads, 1)
-    k_order_units(CellOrder o, UnitPlan u, Geom G, Phys P, Scalars* S, int strips, int seg,
+    k_order_units(CellOrder o, UnitPlan u, Geom G, Phys P, Scalars* S, int pieces, int seg,
                   Gate gate) {
   if (!gate_open(S, gate)) {
     if (!gate.begun && blockIdx.x == 0 && threadIdx.x == 0) S->active = 0;
@@ -1507,16 +1523,15 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
   // node columns of the cells the particles are binned to (the key range the
   // scatter just rolled over), plus the column right of them
   const int L = S->krange[0], K = S->krange[1];
-  const int2 share = plan_share(strips);
-  for (int strip = share.x; strip < strips; strip += share.y) {
-    if (L <= K)
-      plan_strip(o.start, G, unit_weight(S, u), strip, unit_buf(sv), u, strip * seg,
-                 u.strip_n + strip, kColWeight, L / G.nrows, min(K / G.nrows + 1, G.ncols),
-                 [&](int cA, int cB) { return make_int4(strip, cA, cB, 0); });
-    else if ((threadIdx.x & 31) == 0)
-      u.strip_n[strip] = 0;
+  const int2 share = plan_share(pieces);
+  for (int q = share.x; q < pieces; q += share.y) {
+    const int strip = G.pieces == 1 ? q : q / G.pieces;
+    plan_piece(o.start, G, unit_weight(S, u), strip, q - strip * G.pieces, unit_buf(sv), u,
+               strip * seg, u.piece_n + strip * G.pieces, kColWeight, L <= K ? L / G.nrows : 1,
+               L <= K ? min(K / G.nrows + 1, G.ncols) : 0,
+               [&](int cA, int cB) { return make_int4(strip, cA, cB, 0); });
   }
-  order_share<kRepeats>(o, S->np, strips, sv);
+  order_share<kRepeats>(o, S->np, pieces, sv);
   __syncthreads();  // the shared memory is free again
   order_crowded(o, sv);
   if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;
@@ -1727,9 +1742,9 @@ int setup_sort() {
 }
 
 void launch_order_units(int grid, cudaStream_t st, const CellOrder& o, const UnitPlan& u, Geom G,
-                        Phys P, Scalars* S, int strips, int seg, Gate gate, bool repeats) {
+                        Phys P, Scalars* S, int pieces, int seg, Gate gate, bool repeats) {
   auto* kernel = repeats ? k_order_units<true> : k_order_units<false>;
-  kernel<<<grid, kOrderThreads, order_smem_bytes(), st>>>(o, u, G, P, S, strips, seg, gate);
+  kernel<<<grid, kOrderThreads, order_smem_bytes(), st>>>(o, u, G, P, S, pieces, seg, gate);
 }
 
 int setup_p2g() {
@@ -1758,16 +1773,21 @@ void launch_p2g(int grid, cudaStream_t st, Particles p, const int* perm, const i
 }
 
 // Block reduction, in a fixed order, of the ledger partials of a grid's units
-// -- strip_n[q] of them from slot q * seg on for strip q -- into S->ledger, and
-// the conservation errors.  One warp takes a strip, its lanes the units.
-__device__ __forceinline__ void ledger_reduce(const double* __restrict__ led_part,
-                                              const int* __restrict__ strip_n, int strips,
-                                              int seg, Scalars* S) {
+// -- piece_n[q] of them for piece q, `per` pieces of `cols` columns to a strip,
+// whose slots lie at its first column among its strip's seg -- into S->ledger, and
+// the conservation errors.  One warp takes a piece, its lanes the units.
+// (Not inlined: inside G2P its loops changed what the compiler spills there, 200
+// against 214 us at 4M particles.)
+__device__ __noinline__ void ledger_reduce(const double* __restrict__ led_part,
+                                           const int* __restrict__ piece_n, int pieces, int per,
+                                           int cols, int seg, Scalars* S) {
   __shared__ double sm[6][32];
   double v[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x >> 5; b < strips; b += blockDim.x >> 5) {
-    const double* part = led_part + (size_t)b * seg * 6;
-    const int n = strip_n[b];
+  for (int b = threadIdx.x >> 5; b < pieces; b += blockDim.x >> 5) {
+    const int strip = per == 1 ? b : b / per;
+    const int slot0 = strip * seg + (b - strip * per) * cols;
+    const double* part = led_part + (size_t)slot0 * 6;
+    const int n = piece_n[b];
     for (int f = threadIdx.x & 31; f < n; f += 32)
 #pragma unroll
       for (int q = 0; q < 6; ++q) v[q] += part[(size_t)f * 6 + q];
@@ -1801,9 +1821,10 @@ __device__ __forceinline__ void ledger_reduce(const double* __restrict__ led_par
 
 // log: a ring of kLedgerLog rows {t, err_mass, err_mom}, row (it-1) % kLedgerLog
 __device__ __forceinline__ void ledger_final(const double* __restrict__ led_part,
-                                             const int* __restrict__ strip_n, int strips, int seg,
-                                             Scalars* S, double* __restrict__ log) {
-  ledger_reduce(led_part, strip_n, strips, seg, S);
+                                             const int* __restrict__ piece_n, int pieces, int seg,
+                                             const Geom& G, Scalars* S,
+                                             double* __restrict__ log) {
+  ledger_reduce(led_part, piece_n, pieces, G.pieces, G.plan_cols, seg, S);
   if (threadIdx.x == 0 && log) {
     double* row = log + 3 * ((S->it - 1) % kLedgerLog);
     row[0] = S->ledger[8];
@@ -2090,7 +2111,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
             const int* __restrict__ skey, Nodes nodes, const double* __restrict__ Z, Geom G,
             Phys P, Scalars* S, int* __restrict__ count, int* __restrict__ tile_sum,
             int* __restrict__ leave,
-            const double* __restrict__ led_part, const int* __restrict__ strip_n, int strips,
+            const double* __restrict__ led_part, const int* __restrict__ piece_n, int pieces,
             int seg, double* __restrict__ log) {
   const int ng = S->nghost;
   const int n = S->np - ng;  // the slab's own particles
@@ -2103,7 +2124,7 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     return;
   }
   if (blk < 0) {
-    ledger_final(led_part, strip_n, strips, seg, S, log);
+    ledger_final(led_part, piece_n, pieces, seg, G, S, log);
     if (threadIdx.x == 0) S->pending = 1;
     return;
   }
@@ -2152,11 +2173,11 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
                 int* count, int* tile_sum, int* leave, const double* led_part, const UnitPlan& u,
-                int strips, int seg, double* log, int record, int want_grad) {
+                int pieces, int seg, double* log, int record, int want_grad) {
   auto* kernel = record ? k_g2p_t<true, true>
                         : want_grad ? k_g2p_t<false, true> : k_g2p_t<false, false>;
   kernel<<<grid + 1, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G, P, S, count,
-                                           tile_sum, leave, led_part, u.strip_n, strips, seg, log);
+                                           tile_sum, leave, led_part, u.piece_n, pieces, seg, log);
 }
 
 size_t p2g_smem_bytes() { return sizeof(P2GSmemT<double>); }
@@ -2241,16 +2262,16 @@ __global__ void k_b_step_end(const Scn* __restrict__ scn, Scalars* S, int nscn) 
 // block to finish rolls the scenarios' key ranges over.
 __global__ void __launch_bounds__(kOrderThreads, 1)
     k_b_order_units(CellOrder o, UnitPlan u, const Scn* __restrict__ scn, Scalars* S, int nscn,
-                    const int* __restrict__ strip_scn, int strips, const Scalars* Sg,
+                    const int* __restrict__ piece_scn, int pieces, const Scalars* Sg,
                     int col_weight) {
   if (!Sg->active) return;
   extern __shared__ unsigned long long sv[];
-  const int2 share = plan_share(strips);
-  for (int b = share.x; b < strips; b += share.y) {
-    const int s = strip_scn[b];
+  const int2 share = plan_share(pieces);
+  for (int b = share.x; b < pieces; b += share.y) {
+    const int s = piece_scn[b];
     const Geom G = scn[s].G;
-    const int local = b - scn[s].strip_off;
-    const int slot0 = scn[s].useg_off + local * (G.ncols + 1);
+    const int q = b - scn[s].piece_off, local = G.pieces == 1 ? q : q / G.pieces;
+    const int k = q - local * G.pieces;
     // node columns of the cells the scenario's particles are binned to (the
     // keys its last G2P made), plus the column right of them; every column
     // after a layout change
@@ -2260,14 +2281,12 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
       c_lo = (L - scn[s].c_off) / G.nrows;
       c_hi = L > H ? -1 : min((H - scn[s].c_off) / G.nrows + 1, G.ncols);
     }
-    if (S[s].active && c_hi >= 0)  // (else no particle)
-      plan_strip(o.start + scn[s].c_off, G, unit_weight(Sg, u), local, unit_buf(sv),
-                 u, slot0, u.strip_n + b, col_weight, c_lo, c_hi,
-                 [&](int cA, int cB) { return make_int4(s, local, cA, cB); });
-    else if ((threadIdx.x & 31) == 0)
-      u.strip_n[b] = 0;
+    if (!S[s].active) c_hi = -1;  // (no unit)
+    plan_piece(o.start + scn[s].c_off, G, unit_weight(Sg, u), local, k, unit_buf(sv), u,
+               scn[s].useg_off + local * (G.ncols + 1), u.piece_n + (b - k), col_weight, c_lo,
+               c_hi, [&](int cA, int cB) { return make_int4(s, local, cA, cB); });
   }
-  order_share<false>(o, Sg->np, strips, sv);
+  order_share<false>(o, Sg->np, pieces, sv);
   __syncthreads();  // the shared memory is free again
   order_crowded(o, sv);
   if (!last_block(u.ucount + kOrderDone, gridDim.x)) return;
@@ -2319,13 +2338,14 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
             const double* __restrict__ Z,
             const Scn* __restrict__ scn, Scalars* S, const int2* __restrict__ gblk,
             const Scalars* Sg, int* __restrict__ count, int* __restrict__ tile_sum,
-            const double* __restrict__ led_part, const int* __restrict__ strip_n, int nscn) {
+            const double* __restrict__ led_part, const int* __restrict__ piece_n, int nscn) {
   if (blockIdx.x < nscn) {
     const int q = blockIdx.x;
     if (!Sg->active) return;
     if (scn[q].live && S[q].active) {
-      ledger_reduce(led_part + (size_t)scn[q].useg_off * 6, strip_n + scn[q].strip_off,
-                    scn[q].nstrips, scn[q].G.ncols + 1, &S[q]);
+      ledger_reduce(led_part + (size_t)scn[q].useg_off * 6, piece_n + scn[q].piece_off,
+                    scn[q].nstrips * scn[q].G.pieces, scn[q].G.pieces, scn[q].G.plan_cols,
+                    scn[q].G.ncols + 1, &S[q]);
       if (threadIdx.x == 0) S[q].pending = 1;
     }
     return;
@@ -2500,7 +2520,7 @@ void launch_b_g2p(int nblk, cudaStream_t st, ParticlesT<R> cur, ParticlesT<R> nx
                   const Scn* scn, Scalars* S, const int2* gblk, Scalars* Sg, int* count,
                   int* tile_sum, const double* led_part, const UnitPlan& u, int nscn) {
   k_b_g2p<R><<<nblk + nscn, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, vvL, Z, scn, S, gblk,
-                                                  Sg, count, tile_sum, led_part, u.strip_n, nscn);
+                                                  Sg, count, tile_sum, led_part, u.piece_n, nscn);
 }
 
 template <class R>
