@@ -247,8 +247,14 @@ int read_scalars(dampm_batch* b) {
   return DAMPM_OK;
 }
 
-// One pass of every live scenario: kPassLaunches kernel launches.
-constexpr int kPassLaunches = 6;
+bool ledgers_apart(const dampm_batch* b) {
+  for (const HostScn& h : b->scns)
+    if (h.d.led_pieces == 0) return true;
+  return false;
+}
+
+// One pass of every live scenario: pass_launches() kernel launches.
+int pass_launches(const dampm_batch* b) { return ledgers_apart(b) ? 7 : 6; }
 int enqueue_pass(dampm_batch* b) {
   cudaStream_t st = b->stream;
   const int nscn = int(b->scns.size());
@@ -290,8 +296,10 @@ int enqueue_pass(dampm_batch* b) {
     launch_b_g2p<double>(b->nblk, st, b->p64[b->cur], b->p64[nxt], b->perm, b->skey,
                          static_cast<const double2*>(b->vvL), b->Z[b->zcur], b->scn, b->S,
                          b->gblk, b->Sg, b->count, b->tile_sum, b->led_part, u, nscn);
+  if (ledgers_apart(b))
+    k_b_ledger<<<nscn, kLedgerThreads, 0, st>>>(b->led_part, b->piece_n, b->scn, b->S, b->Sg);
   b->cur = nxt;
-  b->launches += kPassLaunches;
+  b->launches += pass_launches(b);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return bfail(b, DAMPM_ERR_CUDA, cudaGetErrorString(e));
   return DAMPM_OK;
@@ -600,6 +608,7 @@ int dampm_batch_add(dampm_batch* b, const dampm_grid* grid, const dampm_params* 
   d.c_off = int(b->C_tot);
   d.nstrips = nstrips;
   d.piece_off = b->pieces_tot;
+  d.led_pieces = ledger_apart(pieces_of(d), np, kBatchApartLeast) ? 0 : pieces_of(d);
   d.useg_off = int(b->useg_tot);
   d.live = 1;
   h.handle = b->next_handle++;
@@ -795,7 +804,7 @@ int dampm_batch_step(dampm_batch* b, int nsteps) {
     if (rc) return rc;
     for (; left >= kBatchGraphPasses; left -= kBatchGraphPasses) {
       BCK(cudaGraphLaunch(b->graph[h], b->stream));
-      b->launches += (long long)kPassLaunches * kBatchGraphPasses + 1;
+      b->launches += (long long)pass_launches(b) * kBatchGraphPasses + 1;
     }
   }
   const bool plain = left > 0;

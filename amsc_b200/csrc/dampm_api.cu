@@ -42,6 +42,7 @@ struct dampm_ctx {
   int ntiles = 0;
   double* led_part = nullptr;
   int n_led = 0;
+  bool led_apart = false;  // ledger_apart() of the last upload
   int strips = 0, useg = 0;  // strips; unit slots per strip (ncols + 1)
   int *piece_n = nullptr, *ucount = nullptr;
   int4* ulist = nullptr;  // plain units, then heavy ones (n_led each)
@@ -72,7 +73,7 @@ struct dampm_ctx {
   static constexpr int kKeyBytes = 2 * sizeof(Particles) + sizeof(Nodes) + sizeof(Geom) +
                                    sizeof(Phys) + sizeof(long long) + sizeof(int) +
                                    sizeof(dampm_ms_params) + sizeof(int) + sizeof(double) +
-                                   3 * sizeof(int);
+                                   4 * sizeof(int);
   struct GraphSlot {
     cudaGraphExec_t exec = nullptr;
     int passes = 0, phase = 0;
@@ -253,6 +254,12 @@ int alloc_particles(dampm_ctx* ctx, long long cap) {
 bool small_grid(const dampm_ctx* ctx) { return ctx->nc <= kSmallCells; }
 int* tile_totals(const dampm_ctx* ctx) { return small_grid(ctx) ? nullptr : ctx->tile_sum; }
 
+// What a new particle count decides: the planner's pieces, who sums the ledger.
+void set_plan(dampm_ctx* ctx, long long np) {
+  set_pieces(ctx->G, np);
+  ctx->led_apart = ledger_apart((long long)ctx->strips * ctx->G.pieces, np, kApartLeast);
+}
+
 UnitPlan unit_plan(const dampm_ctx* ctx) {
   return UnitPlan{kUnitsPerCta * ctx->p2g_grid, unit_min_weight(ctx->n_led, ctx->p2g_ctas),
                   ctx->n_led, ctx->ulist, ctx->uslot, ctx->piece_n, ctx->ucount};
@@ -341,7 +348,8 @@ int enqueue_back(dampm_ctx* ctx) {
              tile_totals(ctx), ctx->leave, ctx->led_part, unit_plan(ctx), ctx->strips * ctx->G.pieces, ctx->useg,
              ctx->ledger_log,
              ctx->record ? 1 : 0,
-             (grad_next || ctx->record) ? 1 : 0);
+             (grad_next || ctx->record) ? 1 : 0, ctx->led_apart);
+  if (ctx->led_apart) ctx->launches += 1;
   if (ctx->record) {
     k_hv<<<grid_for(ctx->nn, 256), 256, 0, ctx->stream>>>(ctx->q, ctx->start,
                                                            ctx->nodes.HV, ctx->G, ctx->S);
@@ -415,7 +423,7 @@ void graph_key_of(const dampm_ctx* ctx, int passes, int phase, unsigned char* k)
   put(&ctx->ms, sizeof(dampm_ms_params));
   put(&ctx->ms_variant, sizeof(int));
   put(&ctx->ms_stretch, sizeof(double));
-  const int cyc[3] = {ms_cadence(ctx) ? 1 : 0, passes, phase};
+  const int cyc[4] = {ms_cadence(ctx) ? 1 : 0, passes, phase, ctx->led_apart ? 1 : 0};
   put(cyc, sizeof(cyc));
 }
 
@@ -801,7 +809,7 @@ int dampm_upload_particles(dampm_ctx* ctx, long long np, const double* x,
     CK(upload_pair(p.mp, mom_px, mom_py, np, ctx->msb.mx, ctx->msb.my, ctx->stream));
     CK(cudaMemcpyAsync(p.Vp, Vp, b, cudaMemcpyHostToDevice, ctx->stream));
   }
-  set_pieces(ctx->G, np);
+  set_plan(ctx, np);
   Scalars s0{};
   s0.fresh = 1;
   s0.np = int(np);
@@ -1107,7 +1115,7 @@ int dampm_set_state(dampm_ctx* ctx, long long np, const double* const* fields,
   }
   int rc = sync_status(ctx, false);
   if (rc) return rc;
-  set_pieces(ctx->G, np);
+  set_plan(ctx, np);
   ctx->Sh->np = int(np);
   ctx->Sh->fresh = fresh ? 1 : 0;
   ctx->Sh->status = 0;  // a new state: an earlier divergence no longer applies

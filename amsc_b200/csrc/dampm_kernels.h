@@ -252,13 +252,23 @@ void launch_p2g(int grid, cudaStream_t st, Particles p, const int* perm, const i
                 const UnitPlan& u);
 int setup_p2g();
 constexpr int kLedgerLog = 1024;  // rows of the per-step ledger log
+constexpr int kLedgerThreads = 1024;
+// Whether the ledger is summed by a launch of its own (4 us, and in a batch one for
+// all) and not by a block of G2P, whose eight warps take 1.3 us a piece while the
+// others take 50 us a million particles: where that block would be the last for
+// long.
+inline bool ledger_apart(long long pieces, long long np, int least) {
+  return pieces > least && 4096 * pieces > np;
+}
+constexpr int kApartLeast = 64, kBatchApartLeast = 256;
 // G2P of the single-scenario step (k_g2p_t specialised for the two flags):
 // reads `cur` through perm, writes `nxt` in this step's sorted order, counts
-// the next binning's keys and sums the ledger; the step's end is left pending
+// the next binning's keys and sums the ledger (apart: by a launch of its own); the
+// step's end is left pending
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
                 int* count, int* tile_sum, int* leave, const double* led_part, const UnitPlan& u,
-                int pieces, int seg, double* log, int record, int want_grad);
+                int pieces, int seg, double* log, int record, int want_grad, bool apart);
 
 // ---- batches of independent scenarios --------------------------------------
 // One scenario of a batch: its geometry, physics and place in the packed
@@ -273,6 +283,7 @@ struct Scn {
   int piece_off;           // its pieces in the batch's order
   int useg_off;            // first unit-plan slot of its first strip
   int live;                // 0 once removed
+  int led_pieces;          // its pieces, or 0 where k_b_ledger sums its ledger
 };
 
 __global__ void k_b_order_units(CellOrder o, UnitPlan u, const Scn* scn, Scalars* S, int nscn,
@@ -281,6 +292,8 @@ __global__ void k_b_order_units(CellOrder o, UnitPlan u, const Scn* scn, Scalars
 __global__ void k_b_step_begin(const Scn* scn, Scalars* S, int nscn, Scalars* Sg,
                                unsigned char* tflag, int ntiles);
 __global__ void k_b_step_end(const Scn* scn, Scalars* S, int nscn);
+__global__ void k_b_ledger(const double* led_part, const int* piece_n, const Scn* scn, Scalars* S,
+                           const Scalars* Sg);
 template <class R>
 void launch_b_p2g(int grid, cudaStream_t st, ParticlesT<R> p, const int* perm,
                   const int* cstart, V2<R>* vvL, double* led_part, const Scn* scn,

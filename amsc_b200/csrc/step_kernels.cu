@@ -1441,20 +1441,19 @@ __device__ __forceinline__ long long unit_weight(const Scalars* S,
   return T < u.min_weight ? u.min_weight : T;
 }
 
-// Plans piece k of a strip (G.plan_cols columns; node columns [c_lo, c_hi] of
-// them): slot0 and piece_n are the first ledger slot and the unit count of the
-// strip's first piece.
-template <class Make>
-__device__ __forceinline__ void plan_piece(const int* __restrict__ cstart, const Geom& G,
-                                           long long T, int strip, int k, int4* buf,
-                                           const UnitPlan& u, int slot0, int* piece_n,
-                                           int col_weight, int c_lo, int c_hi, Make make) {
-  const int first = k * G.plan_cols;
-  const int lo = max(c_lo, first), hi = k + 1 < G.pieces ? min(c_hi, first + G.plan_cols - 1) : c_hi;
-  int n = 0;
-  if (lo <= hi)
-    n = plan_columns(cstart, G, T, strip, buf, u, slot0 + first, col_weight, lo, hi, make);
-  if ((threadIdx.x & 31) == 0) piece_n[k] = n;
+// Piece q of a grid: its strip, its first ledger slot (of the grid's; seg to a
+// strip), and its share of node columns [c_lo, c_hi].
+__device__ __forceinline__ void piece_of(const Geom& G, int q, int seg, int& strip, int& slot,
+                                         int& c_lo, int& c_hi) {
+  strip = q;
+  slot = q * seg;
+  if (G.pieces > 1) {
+    strip = q / G.pieces;
+    const int k = q - strip * G.pieces, first = k * G.plan_cols;
+    slot = strip * seg + first;
+    c_lo = max(c_lo, first);
+    if (k + 1 < G.pieces) c_hi = min(c_hi, first + G.plan_cols - 1);
+  }
 }
 
 // Who plans and who orders: the first plan_blocks() blocks plan, four warps each,
@@ -1525,11 +1524,16 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
   const int L = S->krange[0], K = S->krange[1];
   const int2 share = plan_share(pieces);
   for (int q = share.x; q < pieces; q += share.y) {
-    const int strip = G.pieces == 1 ? q : q / G.pieces;
-    plan_piece(o.start, G, unit_weight(S, u), strip, q - strip * G.pieces, unit_buf(sv), u,
-               strip * seg, u.piece_n + strip * G.pieces, kColWeight, L <= K ? L / G.nrows : 1,
-               L <= K ? min(K / G.nrows + 1, G.ncols) : 0,
-               [&](int cA, int cB) { return make_int4(strip, cA, cB, 0); });
+    int strip, slot, c_lo = L / G.nrows, c_hi = min(K / G.nrows + 1, G.ncols);
+    piece_of(G, q, seg, strip, slot, c_lo, c_hi);
+    if (L <= K && c_lo <= c_hi) {
+      const int n = plan_columns(o.start, G, unit_weight(S, u), strip, unit_buf(sv), u, slot,
+                                 kColWeight, c_lo, c_hi,
+                                 [&](int cA, int cB) { return make_int4(strip, cA, cB, 0); });
+      if ((threadIdx.x & 31) == 0) u.piece_n[q] = n;
+    } else if ((threadIdx.x & 31) == 0) {
+      u.piece_n[q] = 0;
+    }
   }
   order_share<kRepeats>(o, S->np, pieces, sv);
   __syncthreads();  // the shared memory is free again
@@ -1772,26 +1776,10 @@ void launch_p2g(int grid, cudaStream_t st, Particles p, const int* perm, const i
                                                               G, P, S, u);
 }
 
-// Block reduction, in a fixed order, of the ledger partials of a grid's units
-// -- piece_n[q] of them for piece q, `per` pieces of `cols` columns to a strip,
-// whose slots lie at its first column among its strip's seg -- into S->ledger, and
-// the conservation errors.  One warp takes a piece, its lanes the units.
-// (Not inlined: inside G2P its loops changed what the compiler spills there, 200
-// against 214 us at 4M particles.)
-__device__ __noinline__ void ledger_reduce(const double* __restrict__ led_part,
-                                           const int* __restrict__ piece_n, int pieces, int per,
-                                           int cols, int seg, Scalars* S) {
+// Block reduction, in a fixed order, of the threads' ledger sums into S->ledger,
+// and the conservation errors.
+__device__ __forceinline__ void ledger_close(const double (&v)[6], Scalars* S) {
   __shared__ double sm[6][32];
-  double v[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x >> 5; b < pieces; b += blockDim.x >> 5) {
-    const int strip = per == 1 ? b : b / per;
-    const int slot0 = strip * seg + (b - strip * per) * cols;
-    const double* part = led_part + (size_t)slot0 * 6;
-    const int n = piece_n[b];
-    for (int f = threadIdx.x & 31; f < n; f += 32)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) v[q] += part[(size_t)f * 6 + q];
-  }
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
     double x = v[q];
@@ -1819,18 +1807,87 @@ __device__ __noinline__ void ledger_reduce(const double* __restrict__ led_part,
   }
 }
 
+// The ledger of a grid from the partials of its units: piece_n[q] of them for
+// piece q, `per` pieces of `cols` columns to a strip, whose slots lie at its first
+// column among its strip's seg.  One warp takes a piece, its lanes the units.
+// (Not inlined: inside G2P its loops changed what the compiler spills there, 200
+// against 214 us at 4M particles.)
+__device__ __noinline__ void ledger_reduce(const double* __restrict__ led_part,
+                                           const int* __restrict__ piece_n, int pieces, int per,
+                                           int cols, int seg, Scalars* S) {
+  double v[6] = {0, 0, 0, 0, 0, 0};
+  for (int b = threadIdx.x >> 5; b < pieces; b += blockDim.x >> 5) {
+    const int strip = per == 1 ? b : b / per;
+    const int slot0 = strip * seg + (b - strip * per) * cols;
+    const double* part = led_part + (size_t)slot0 * 6;
+    const int n = piece_n[b];
+    for (int f = threadIdx.x & 31; f < n; f += 32)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) v[q] += part[(size_t)f * 6 + q];
+  }
+  ledger_close(v, S);
+}
+
+// The same for many pieces of few units: a warp takes 32 pieces at a time, lane by
+// lane, sums up their counts, and its lanes take the units of all of them side by
+// side.  (In place of ledger_reduce it costs G2P 1 % at 4M particles, in registers.)
+__device__ __forceinline__ void ledger_reduce_many(const double* __restrict__ led_part,
+                                                   const int* __restrict__ piece_n, int pieces,
+                                                   int per, int cols, int seg, Scalars* S) {
+  double v[6] = {0, 0, 0, 0, 0, 0};
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int b0 = threadIdx.x >> 5; b0 < pieces; b0 += 32 * nw) {
+    const int b = b0 + lane * nw, strip = per == 1 ? b : b / per;
+    const int n = b < pieces ? piece_n[b] : 0;
+    int upto = n;  // units of this piece and those before it
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    const int slot = strip * seg + (b - strip * per) * cols - (upto - n);
+    const int units = __shfl_sync(0xffffffffu, upto, 31);
+#pragma unroll 2
+    for (int f0 = 0; f0 < units; f0 += 32) {
+      const int f = min(f0 + lane, units - 1);
+      int q = 0;  // the unit's piece: as many end at f or before
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, upto, q + step - 1) <= f) q += step;
+      const int at = __shfl_sync(0xffffffffu, slot, q) + f;
+      if (f0 + lane < units) {
+        const double2* part = reinterpret_cast<const double2*>(led_part) + 3 * (size_t)at;
+        const double2 a = part[0], c = part[1], d = part[2];
+        v[0] += a.x;
+        v[1] += a.y;
+        v[2] += c.x;
+        v[3] += c.y;
+        v[4] += d.x;
+        v[5] += d.y;
+      }
+    }
+  }
+  ledger_close(v, S);
+}
+
 // log: a ring of kLedgerLog rows {t, err_mass, err_mom}, row (it-1) % kLedgerLog
-__device__ __forceinline__ void ledger_final(const double* __restrict__ led_part,
-                                             const int* __restrict__ piece_n, int pieces, int seg,
-                                             const Geom& G, Scalars* S,
-                                             double* __restrict__ log) {
-  ledger_reduce(led_part, piece_n, pieces, G.pieces, G.plan_cols, seg, S);
+__device__ __forceinline__ void ledger_log(const Scalars* S, double* __restrict__ log) {
   if (threadIdx.x == 0 && log) {
     double* row = log + 3 * ((S->it - 1) % kLedgerLog);
     row[0] = S->ledger[8];
     row[1] = S->ledger[6];
     row[2] = S->ledger[7];
   }
+}
+
+// The ledger as a launch of its own, after G2P (which was given no pieces): see
+// ledger_apart.
+__global__ void __launch_bounds__(kLedgerThreads)
+    k_ledger(const double* __restrict__ led_part, const int* __restrict__ piece_n, int pieces,
+             int seg, Geom G, Scalars* S, double* __restrict__ log) {
+  if (!S->active) return;
+  ledger_reduce_many(led_part, piece_n, pieces, G.pieces, G.plan_cols, seg, S);
+  ledger_log(S, log);
 }
 
 // ---------------------------------------------------------------------------
@@ -2124,7 +2181,8 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     return;
   }
   if (blk < 0) {
-    ledger_final(led_part, piece_n, pieces, seg, G, S, log);
+    ledger_reduce(led_part, piece_n, pieces, G.pieces, G.plan_cols, seg, S);
+    ledger_log(S, log);
     if (threadIdx.x == 0) S->pending = 1;
     return;
   }
@@ -2173,11 +2231,14 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
 void launch_g2p(int grid, cudaStream_t st, Particles cur, Particles nxt, const int* perm,
                 const int* skey, Nodes nodes, const double* Z, Geom G, Phys P, Scalars* S,
                 int* count, int* tile_sum, int* leave, const double* led_part, const UnitPlan& u,
-                int pieces, int seg, double* log, int record, int want_grad) {
+                int pieces, int seg, double* log, int record, int want_grad, bool apart) {
   auto* kernel = record ? k_g2p_t<true, true>
                         : want_grad ? k_g2p_t<false, true> : k_g2p_t<false, false>;
   kernel<<<grid + 1, kG2PThreads, 0, st>>>(cur, nxt, perm, skey, nodes, Z, G, P, S, count,
-                                           tile_sum, leave, led_part, u.piece_n, pieces, seg, log);
+                                           tile_sum, leave, led_part, u.piece_n,
+                                           apart ? 0 : pieces, seg, log);
+  if (apart)
+    k_ledger<<<1, kLedgerThreads, 0, st>>>(led_part, u.piece_n, pieces, seg, G, S, log);
 }
 
 size_t p2g_smem_bytes() { return sizeof(P2GSmemT<double>); }
@@ -2270,21 +2331,24 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
   for (int b = share.x; b < pieces; b += share.y) {
     const int s = piece_scn[b];
     const Geom G = scn[s].G;
-    const int q = b - scn[s].piece_off, local = G.pieces == 1 ? q : q / G.pieces;
-    const int k = q - local * G.pieces;
     // node columns of the cells the scenario's particles are binned to (the
     // keys its last G2P made), plus the column right of them; every column
     // after a layout change
-    int c_lo = 0, c_hi = G.ncols;
+    int strip, slot, c_lo = 0, c_hi = G.ncols;
     if (!(Sg->krange[0] <= Sg->krange[1])) {
       const int L = S[s].knext[0], H = S[s].knext[1];
       c_lo = (L - scn[s].c_off) / G.nrows;
       c_hi = L > H ? -1 : min((H - scn[s].c_off) / G.nrows + 1, G.ncols);
     }
-    if (!S[s].active) c_hi = -1;  // (no unit)
-    plan_piece(o.start + scn[s].c_off, G, unit_weight(Sg, u), local, k, unit_buf(sv), u,
-               scn[s].useg_off + local * (G.ncols + 1), u.piece_n + (b - k), col_weight, c_lo,
-               c_hi, [&](int cA, int cB) { return make_int4(s, local, cA, cB); });
+    piece_of(G, b - scn[s].piece_off, G.ncols + 1, strip, slot, c_lo, c_hi);
+    if (S[s].active && c_lo <= c_hi) {  // (else no particle)
+      const int n = plan_columns(o.start + scn[s].c_off, G, unit_weight(Sg, u), strip,
+                                 unit_buf(sv), u, scn[s].useg_off + slot, col_weight, c_lo, c_hi,
+                                 [&](int cA, int cB) { return make_int4(s, strip, cA, cB); });
+      if ((threadIdx.x & 31) == 0) u.piece_n[b] = n;
+    } else if ((threadIdx.x & 31) == 0) {
+      u.piece_n[b] = 0;
+    }
   }
   order_share<false>(o, Sg->np, pieces, sv);
   __syncthreads();  // the shared memory is free again
@@ -2344,8 +2408,8 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
     if (!Sg->active) return;
     if (scn[q].live && S[q].active) {
       ledger_reduce(led_part + (size_t)scn[q].useg_off * 6, piece_n + scn[q].piece_off,
-                    scn[q].nstrips * scn[q].G.pieces, scn[q].G.pieces, scn[q].G.plan_cols,
-                    scn[q].G.ncols + 1, &S[q]);
+                    scn[q].led_pieces, scn[q].G.pieces, scn[q].G.plan_cols, scn[q].G.ncols + 1,
+                    &S[q]);
       if (threadIdx.x == 0) S[q].pending = 1;
     }
     return;
@@ -2396,6 +2460,17 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
   cfl_block_max(m0, m1, m2, red, &S[s]);
   key_range(ok ? nkey : 0x7fffffff, ok ? nkey : -1, kred, &S[s]);
   flag_non_finite(bad, &S[s]);
+}
+
+// k_ledger of a batch, a block per scenario.
+__global__ void __launch_bounds__(kLedgerThreads)
+    k_b_ledger(const double* __restrict__ led_part, const int* __restrict__ piece_n,
+               const Scn* __restrict__ scn, Scalars* S, const Scalars* Sg) {
+  const int q = blockIdx.x;
+  if (!Sg->active || !scn[q].live || !S[q].active || scn[q].led_pieces > 0) return;
+  ledger_reduce_many(led_part + (size_t)scn[q].useg_off * 6, piece_n + scn[q].piece_off,
+                     scn[q].nstrips * scn[q].G.pieces, scn[q].G.pieces, scn[q].G.plan_cols,
+                     scn[q].G.ncols + 1, &S[q]);
 }
 
 template <class R>

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from amsc_b200.batch import Batch
+from amsc_b200.dampm import Solver
 from test_gpu_sort_paths import FIELDS, _check, _data
 from oracle.oracle import Oracle
 
@@ -47,3 +48,30 @@ def test_several_pieces_at_a_time(cuda_lib, col_weight):
             for k in FIELDS:
                 np.testing.assert_array_equal(b.download(h, k), o.get(k), err_msg=k)
             np.testing.assert_allclose(b.ledgers(h)[:6], o.ledger()[:6], rtol=1e-11, atol=1e-9)
+
+
+@pytest.mark.parametrize("case", [CASES[0], CASES[8]])  # 2 and 301 pieces
+def test_ledger_of_every_step(cuda_lib, case):
+    """A block of G2P sums the ledger, or a launch of its own where the pieces are
+    many: the log holds every step's row, replayed from a graph or not."""
+    d = _columns(*case)
+    o = Oracle(d, threads=2)
+    with Solver(d) as s:
+        s.step(19)
+        log = s.ledger_history(1, 19)
+        for it in range(1, 20):
+            o.run(1)
+            led = o.ledger()
+            assert log[it - 1][0] == pytest.approx(it * 1e-4 - 1e-4, abs=1e-12)
+            np.testing.assert_allclose(log[it - 1][1:], led[6:8], rtol=0, atol=1e-12)
+        np.testing.assert_allclose(s.ledgers()[:6], o.ledger()[:6], rtol=1e-11, atol=1e-9)
+        assert tuple(s.ledgers()[[8, 6, 7]]) == tuple(log[18])
+    # in a batch, beside one of the other kind (which a graph's passes take along)
+    e = _columns(*CASES[3])
+    with Batch(d.np + e.np, d.nnodes + e.nnodes, 2) as b:
+        hd, he = b.add(d), b.add(e)
+        b.step(19)
+        np.testing.assert_allclose(b.ledgers(hd)[:6], o.ledger()[:6], rtol=1e-11, atol=1e-9)
+        o = Oracle(e, threads=2)
+        o.run(19)
+        np.testing.assert_allclose(b.ledgers(he)[:6], o.ledger()[:6], rtol=1e-11, atol=1e-9)
