@@ -64,7 +64,8 @@ struct dampm_batch {
   unsigned long long* sortbuf = nullptr;  // 2 x capacity: crowded cells' order
   int *count = nullptr, *start = nullptr, *perm = nullptr;
   // of each sorted position: cell, storage slot and reference index before the
-  // order inside the cells
+  // order inside the cells (the last two in `stage`: a pass uses them, a download
+  // comes between passes)
   int *skey = nullptr, *sslot = nullptr, *sidx = nullptr;
   int *tile_sum = nullptr, *cbig = nullptr;
   unsigned char* tflag = nullptr;  // the scan tiles of a pass (k_b_step_begin)
@@ -478,8 +479,8 @@ int dampm_batch_create(long long particle_cap, long long node_cap, int scenario_
   rc = rc ? rc : balloc(b, &b->tflag, nn / kScanTile + 2);
   rc = rc ? rc : balloc(b, &b->perm, pc);
   rc = rc ? rc : balloc(b, &b->skey, pc);
-  rc = rc ? rc : balloc(b, &b->sslot, pc);
-  rc = rc ? rc : balloc(b, &b->sidx, pc);
+  b->sslot = reinterpret_cast<int*>(b->stage);
+  b->sidx = b->sslot + pc;
   rc = rc ? rc : balloc(b, &b->cbig, pc / 256 + 4);
   const size_t us = size_t(b->USEG_cap);
   rc = rc ? rc : balloc(b, &b->ulist, 2 * us);

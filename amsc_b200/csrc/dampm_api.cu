@@ -36,7 +36,8 @@ struct dampm_ctx {
   double *Z = nullptr, *dZdx = nullptr, *dZdy = nullptr;
   int *count = nullptr, *start = nullptr, *perm = nullptr, *tile_sum = nullptr;
   // of each sorted position: cell, storage slot and reference index before the
-  // order inside the cells
+  // order inside the cells (the last two in msb.stage: a sort uses them, a download
+  // comes between steps)
   int *skey = nullptr, *sslot = nullptr, *sidx = nullptr;
   unsigned long long* sortbuf = nullptr;  // 2 x capacity: crowded cells' order
   int ntiles = 0;
@@ -229,7 +230,7 @@ int alloc_particles(dampm_ctx* ctx, long long cap) {
     if (rc) return rc;
     CK(cudaMemsetAsync(*q, 0, cap * sizeof(double), ctx->stream));
   }
-  int** fi[] = {&p.label, &p.level, &ctx->perm, &ctx->skey, &ctx->sslot, &ctx->sidx};
+  int** fi[] = {&p.label, &p.level, &ctx->perm, &ctx->skey};
   for (int** q : fi) {
     int rc = dalloc(ctx, q, cap);
     if (rc) return rc;
@@ -245,6 +246,8 @@ int alloc_particles(dampm_ctx* ctx, long long cap) {
     return dalloc(ctx, reinterpret_cast<unsigned char**>(q), bytes);
   });
   if (rc) return rc;
+  ctx->sslot = reinterpret_cast<int*>(ctx->msb.stage);
+  ctx->sidx = ctx->sslot + cap;
   if (ctx->record) return alloc_record(ctx);
   return DAMPM_OK;
 }
