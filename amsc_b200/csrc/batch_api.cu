@@ -276,8 +276,9 @@ int enqueue_pass(dampm_batch* b) {
                                                 b->ucount, b->Sg, gate, 0, b->tflag);
   const Binning n{key, slot, idx, b->sslot, b->sidx, b->skey};
   k_scatter<<<gp, 256, 0, st>>>(n, b->start, b->tile_sum, ntiles, b->ucount, b->Sg, gate);
-  const UnitPlan u{b->units_per_cta * b->p2g_grid, unit_min_weight(b->useg_tot, b->p2g_grid),
-                   int(b->USEG_cap), b->ulist, b->uslot, b->piece_n, b->ucount};
+  const UnitPlan u{batch_units(b->units_per_cta, b->p2g_grid, b->P_tot),
+                   unit_min_weight(b->useg_tot, b->p2g_grid), int(b->USEG_cap), b->ulist,
+                   b->uslot, b->piece_n, b->ucount};
   k_b_order_units<<<order_blocks(b->P_tot, b->pieces_tot), kOrderThreads, order_smem_bytes(), st>>>(
       CellOrder{n, b->start, b->cbig, b->ucount, b->perm, b->sortbuf, b->P_cap, b->count, 0},
       u, b->scn, b->S, nscn, b->piece_scn, b->pieces_tot, b->Sg, b->col_weight);

@@ -22,9 +22,20 @@ constexpr int kTR = 30;
 #endif
 constexpr int kUnitsPerCta = DAMPM_UNITS_PER_CTA;
 // A batch's columns are short (120 particles in 30 rows at 4 per cell), so the
-// leading column that each unit stages again weighs more than an even load: a pass
-// of 96 scenarios takes 229 us at one unit per CTA, 237 at two (FP32 201 and 209).
+// leading column that each unit stages again weighs more than an even load, as long
+// as the units are not long.  Microseconds a pass at one unit per CTA and at two: 96
+// scenarios of 64 to 128 cells a side 85.8 and 96.5 (FP32 77.3 and 88.0), 40 of 200
+// to 500 183 and 199, 24 requests 196 and 209, four 512 x 512 flows 166 and 177, one
+// of 1536 x 1536 292 and 301.  From a weight of 4096 on the load counts: 512
+// scenarios (14600 a CTA) take 1640 at one unit per CTA, 1340 at 8192 a unit, 1330
+// at 4096, and 2650, 2060 and 2050 when crowded columns have formed (P2G takes units
+// of more than twice the weight first); 16 dense flows (7000 a CTA) 557 either way.
 constexpr int kBatchUnitsPerCta = 1;
+constexpr int kBatchUnitMaxWeight = 4096;
+inline int batch_units(int units_per_cta, int ctas, long long np) {
+  return int(std::max((long long)units_per_cta * ctas,
+                      (np + kBatchUnitMaxWeight - 1) / kBatchUnitMaxWeight));
+}
 constexpr int kUnitMinWeight = 1024;
 // The least weight of a unit, from the number of (strip, column) pairs of the
 // grids and P2G's resident CTAs.  Where the pairs that hold particles (a quarter

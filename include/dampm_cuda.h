@@ -386,8 +386,8 @@ int dampm_batch_compact(dampm_batch* b);
 int dampm_batch_step(dampm_batch* b, int nsteps);
 int dampm_batch_sync(dampm_batch* b);
 
-/* Tuning, for an autotuner: P2G units per CTA of the unit plan and the
- * weight (in particles) of a column in it, and whether dampm_batch_step
+/* Tuning, for an autotuner: P2G units per CTA of the unit plan (at least: a
+ * unit weighs 4096 at most) and the weight (in particles) of a column in it, and whether dampm_batch_step
  * replays its passes as a CUDA graph (captured after each change of layout;
  * 1 by default).  0 (or -1 for use_graphs) keeps a setting.  None of these
  * changes any result. */

@@ -5,6 +5,7 @@ the oracle, alone and in a batch, ledger to the round-off of its order."""
 import numpy as np
 import pytest
 
+from amsc_b200 import scenarios
 from amsc_b200.batch import Batch
 from amsc_b200.dampm import Solver
 from test_gpu_sort_paths import FIELDS, _check, _data
@@ -75,3 +76,16 @@ def test_ledger_of_every_step(cuda_lib, case):
         o = Oracle(e, threads=2)
         o.run(19)
         np.testing.assert_allclose(b.ledgers(he)[:6], o.ledger()[:6], rtol=1e-11, atol=1e-9)
+
+
+def test_units_of_a_large_batch(cuda_lib):
+    """More than 4096 particles per CTA: the units stay at that weight, the state is
+    that of the scenario alone."""
+    d = scenarios.mudflow(N=2048)
+    with Solver(d, capacity=d.np) as s, Batch(d.np, d.nnodes, 1) as b:
+        h = b.add(d)
+        s.step(4)
+        b.step(4)
+        for k in FIELDS:
+            np.testing.assert_array_equal(b.download(h, k), s.download(k), err_msg=k)
+        np.testing.assert_allclose(b.ledgers(h)[:6], s.ledgers()[:6], rtol=1e-12, atol=1e-6)
