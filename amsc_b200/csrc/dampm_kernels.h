@@ -61,7 +61,9 @@ inline void set_pieces(Geom& G, long long np) {
   G.plan_cols = kPlanCols * int((np >> 20) + 1);
   G.pieces = (G.ncols + G.plan_cols - 1) / G.plan_cols;
 }
-constexpr int kMaxStrips = 8192;  // strip offsets of the unit list in shared memory
+// Strips of a batch (the size of its planner's tables, whatever its capacity), and
+// of a single grid, which keeps to the same limit.
+constexpr int kMaxStrips = 8192;
 constexpr int kP2GThreads = 128;
 #ifndef DAMPM_P2G_CAP
 #define DAMPM_P2G_CAP 512

@@ -644,7 +644,8 @@ __global__ void __launch_bounds__(kScanThreads)
 // particles per cell half of the cells in the warps' share.  Counting over the
 // indices in global memory is bound by L1's tag lookups, with a block's tile in
 // shared memory by the block's barriers (k_order_units 66 and 60 us at 4M
-// particles, this way 42; 24 B a particle, which take 15 us).
+// particles, this way 42, and 36 with the planning warps in blocks of their own,
+// below; 16 B a particle, which take 10 us).
 constexpr int kOrderPer = 4;
 constexpr int kOrderWin = 32 * kOrderPer + 2 * kCrowded;
 template <bool kRepeats>
@@ -1462,7 +1463,7 @@ __device__ __forceinline__ void piece_of(const Geom& G, int q, int seg, int& str
 // 4096-particle dam break 0.6 us longer, of 4M particles 4).  Where that would take
 // more than one block in kPlanShare (a batch of many scenarios, or a grid of few
 // blocks) the pieces are spread over the blocks, warp 0 of each, then warp 1 ...,
-// and the other warps order (everyone where that leaves fewer than half): 11 us
+// and the other warps order (everyone where that leaves fewer than half): 12.5 us
 // against 15 with the 800 strips of 96 scenarios.
 constexpr int kPlanShare = 4;
 __device__ __forceinline__ int plan_blocks(int pieces) {
@@ -1504,7 +1505,7 @@ __device__ __forceinline__ int4* unit_buf(unsigned long long* sv) {
 // no block still reads the loop condition then.
 // The planner and the order of the smaller and of the larger cells were launches
 // of their own: 46 us in all at 4M particles, 20 at 0.25M, 13 at 4096 and 53 in a
-// batch of 96 scenarios; together 42, 13, 6 and 13.
+// batch of 96 scenarios; together 36, 11.5, 6 and 12.5.
 // The begin sits here and not at the end of G2P, where every block would have
 // to wait for its stores before it counts itself done (7 us at 0.25M and 4M
 // particles).
@@ -1548,8 +1549,9 @@ __global__ void __launch_bounds__(kOrderThreads, 1)
 // kUnroll: chain steps per loop trip.  Two in the single-scenario kernel (4M
 // particles: 1 % faster than one).  One in a batch: its units are a few short
 // columns, so the four warps' loops keep leaving and entering the instruction
-// cache (at two, 1.9 cycles of every issue wait for an instruction; a pass of 96
-// scenarios takes 156 us at two, 127 at one, 290 at four; in FP32 156 and 100).
+// cache (at two, 1.9 cycles of every issue wait for an instruction; this kernel
+// takes 138 us with 96 scenarios at two, 118 at one, 234 at four; in FP32 129, 97
+// and 269).
 template <class R, int kUnroll>
 __device__ __forceinline__ void p2g_unit(
     const ParticlesT<R>& p, const int* __restrict__ perm,

@@ -235,7 +235,8 @@ long long dampm_last_launch_count(dampm_ctx* ctx);
 
 /* Wall time of the kernels of the last dampm_step call, measured with CUDA
  * events on the context stream (ms, synchronises); per kernel class:
- * out[0] sort, out[1] p2g, out[2] g2p, out[3] other, out[4] total. */
+ * out[0] sort (with P2G's unit plan), out[1] p2g, out[2] g2p (with the ledger),
+ * out[3] other, out[4] total. */
 int dampm_last_timings(dampm_ctx* ctx, int enable_events, double out[5]);
 
 const char* dampm_last_error(dampm_ctx* ctx);

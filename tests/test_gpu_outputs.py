@@ -84,7 +84,7 @@ def test_edge_pileup_and_walls(cuda_lib):
 @pytest.mark.gpu
 def test_cell_with_twenty_thousand_particles(cuda_lib):
     """One cell holding 20,000 particles: its index order comes from sorted
-    runs of 8192 merged pairwise (k_segment_order_big)."""
+    runs of 8192 merged pairwise (order_crowded)."""
     d = scenarios.bench_slab(30000, nsteps=3)
     x, y = d.arrays["x"].copy(), d.arrays["y"].copy()
     rng = np.random.default_rng(7)

@@ -1,9 +1,9 @@
 """The paths of a pass's sort and planner: grids up to 16384 cells are scanned
-and scattered in one launch, larger ones in tiles; a block cuts several strips
-where there are more than blocks; the cuts of a strip of more than 8192 columns
-leave the shared memory.  Cells of every size class of the ordering (1, 2..16 a
-lane, 17..256 a warp, more a block).  State bitwise equal to the oracle, alone
-and in a batch."""
+and scattered in one launch, larger ones in tiles; warps cut the strips, several
+each where there are more strips than warps, in pieces where a strip is long.
+Cells on both sides of 256 particles, up to which a warp counts over the indices
+of a particle's cell and above which a block orders the cell.  State bitwise equal
+to the oracle, alone and in a batch."""
 import numpy as np
 import pytest
 
